@@ -103,37 +103,129 @@ __global__ void k_flip_scatter(G3 g, long long n, const float *__restrict__ pos,
     }
 }
 
-// buildFinalize (:532-550)
+// buildFinalize (:532-550).  Validity leaves as the extension's layer bytes
+// (0 valid, LAYER_OPEN not).
 __global__ void k_flip_finalize(long long n, const int *__restrict__ num, const int *__restrict__ den, float scale,
-                                float eps, float *__restrict__ data, int *__restrict__ valid) {
+                                float eps, float *__restrict__ data, uint8_t *__restrict__ valid) {
     for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < n; f += (long long)gridDim.x * blockDim.x) {
         const float numer = (float)num[f] / scale;
         const float denom = (float)den[f] / scale;
         if (denom > eps) {
             data[f] = numer / denom;
-            valid[f] = 1;
+            valid[f] = 0;
         } else {
             data[f] = 0.0f;
-            valid[f] = 0;
+            valid[f] = LAYER_OPEN;
         }
     }
 }
 
-// computeU/V/WFluidAdjacent (:586-618)
-__global__ void k_flip_adjacent(G3 g, int a, const float *__restrict__ mask, int *__restrict__ adj) {
-    int s[3];
-    comp_shape(g, a, s[0], s[1], s[2]);
-    const long long n = (long long)s[0] * s[1] * s[2];
+// up to three components' layer bytes for one launch
+struct Layers3 {
+    uint8_t *b[3];
+};
+
+// computeU/V/WFluidAdjacent (:586-618), as layer bytes, four faces a thread
+__global__ void __launch_bounds__(256) k_flip_adjacent(G3 g, Comps3 C, const float *__restrict__ mask, Layers3 adj) {
+    const int a = blockIdx.z;
+    const CompDims &c = C.c[a];
     const int nn = a == 0 ? g.nx : (a == 1 ? g.ny : g.nz);
-    for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < n; f += (long long)gridDim.x * blockDim.x) {
-        int idx[3];
-        unflatten(f, s[0], s[1], idx[0], idx[1], idx[2]);
-        int lo[3] = {idx[0], idx[1], idx[2]}, hi[3] = {idx[0], idx[1], idx[2]};
-        lo[a] = iclamp(idx[a] - 1, 0, nn - 1);
-        hi[a] = iclamp(idx[a], 0, nn - 1);
-        const float ml = mask[lo[0] + (long long)g.nx * (lo[1] + (long long)g.ny * lo[2])];
-        const float mh = mask[hi[0] + (long long)g.nx * (hi[1] + (long long)g.ny * hi[2])];
-        adj[f] = (ml > 0.5f || mh > 0.5f) ? 1 : 0;
+    const int step = a == 0 ? 1 : (a == 1 ? g.nx : g.nx * g.ny);
+    const unsigned nq = (c.n + 3) / 4;
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
+        int i, j, k;
+        c.at(4 * q, i, j, k);
+        unsigned bytes = 0;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            if (4 * q + m < c.n) {
+                const int idx = a == 0 ? i : (a == 1 ? j : k);
+                // the cell above the face, clamped, and the one below it
+                const int hi = (i - (a == 0 && i == nn)) + g.nx * ((j - (a == 1 && j == nn)) + g.ny * (k - (a == 2 && k == nn)));
+                const int lo = (idx > 0 && idx < nn) ? hi - step : hi;
+                if (!(mask[lo] > 0.5f || mask[hi] > 0.5f)) bytes |= LAYER_OPEN << (8 * m);
+            }
+            if (++i == c.sx) {
+                i = 0;
+                if (++j == c.sy) j = 0, ++k;
+            }
+        }
+        reinterpret_cast<unsigned *>(adj.b[a])[q] = bytes;
+    }
+}
+
+// extension step t over a whole component: the air around the liquid, where
+// most faces are not valid.  Four faces a thread: the words of bytes beside,
+// above and below them (unaligned ones from two words by a funnel shift)
+// tell in a few SIMD-in-a-word compares whether any of the four can have a
+// valid neighbour (the words ignore row and plane ends, so they may say yes
+// too often, never too seldom).  Those faces queue in shared memory and the
+// block takes the exact per-face step on the queue with all its threads: spray
+// leaves one or two such faces a warp in most of the air, and a warp that
+// stepped four faces a thread in place would run the whole step four times
+// for them.  Step 1 reads the validity `src` and writes every byte of `lay`;
+// later ones work on `lay` in place (src == lay).  Bound by issue, not by its
+// bytes (3 MB a component).  256 x 128 x 128, 40% liquid with 2% spray, three
+// components: 30 us a step (45 us with four faces a thread in place; 110 us
+// for three double-buffered passes over int32 markers).
+__global__ void __launch_bounds__(256) k_extend(Comps3 C, Layers3 src, Layers3 lay, int t) {
+    __shared__ unsigned queue[1024];
+    __shared__ unsigned queued;
+    const int a = blockIdx.z;
+    const CompDims &c = C.c[a];
+    const uint8_t *s = src.b[a];
+    const unsigned *sw = reinterpret_cast<const unsigned *>(s);
+    float *d = C.d[a];
+    const int nq = (int)((c.n + 3) / 4);
+    const int off[4] = {-c.sx, c.sx, -c.sx * c.sy, c.sx * c.sy};
+    const unsigned tt = (unsigned)t * 0x01010101u;
+    const bool copy = src.b[a] != lay.b[a];
+    auto word_at = [&](int wi) { return (unsigned)wi < (unsigned)nq ? sw[wi] : 0xffffffffu; };
+    if (threadIdx.x == 0) queued = 0;
+    for (int q0 = blockIdx.x * blockDim.x; q0 < nq; q0 += gridDim.x * blockDim.x) {
+        const int q = q0 + (int)threadIdx.x;
+        unsigned near = 0;
+        if (q < nq) {
+            const unsigned word = sw[q], open = __vcmpeq4(word, 0xffffffffu);
+            if (copy) reinterpret_cast<unsigned *>(lay.b[a])[q] = word;
+            if (open) {
+                const unsigned prev = word_at(q - 1), next = word_at(q + 1);
+                near = __vcmpltu4(__funnelshift_r(word, next, 8), tt) | __vcmpltu4(__funnelshift_l(prev, word, 8), tt);
+#pragma unroll
+                for (int o = 0; o < 4; ++o) {
+                    const int wi = q + (off[o] >> 2);
+                    near |= __vcmpltu4(__funnelshift_r(word_at(wi), word_at(wi + 1), 8 * (off[o] & 3)), tt);
+                }
+                near &= open;
+            }
+        }
+        __syncthreads();   // the last round's queue is used up, its count cleared
+        if (near) {
+            unsigned at = atomicAdd(&queued, (unsigned)__popc(near) >> 3);
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+                if (near >> (8 * m) & 1u) queue[at++] = 4 * (unsigned)q + m;
+        }
+        __syncthreads();
+        const unsigned cnt = queued;
+        for (unsigned e = threadIdx.x; e < cnt; e += blockDim.x) {
+            const unsigned f = queue[e];
+            float v;
+            if (f < c.n && extend_face(c, d, s, f, t, v)) {
+                d[f] = v;
+                lay.b[a][f] = (uint8_t)t;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) queued = 0;
+    }
+}
+// valid bytes back to 0 (steps then count from 1 again)
+__global__ void __launch_bounds__(256) k_fold(Comps3 C, Layers3 lay) {
+    const unsigned nq = (C.c[blockIdx.z].n + 3) / 4;
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
+        unsigned &w = reinterpret_cast<unsigned *>(lay.b[blockIdx.z])[q];
+        w = __vcmpeq4(w, 0xffffffffu);
     }
 }
 
@@ -709,6 +801,41 @@ int post(const char *what) {
     return FF_OK;
 }
 
+Comps3 comps3(const G3 &g, float *const d[3], int ncomp) {
+    Comps3 C{};
+    for (int a = 0; a < ncomp; ++a) {
+        C.c[a] = comp_dims(g, a);
+        C.d[a] = d[a];
+    }
+    return C;
+}
+// a grid for four faces a thread over the largest component
+dim3 quad_grid(const Comps3 &C, int ncomp) {
+    unsigned n = 0;
+    for (int a = 0; a < ncomp; ++a) n = std::max(n, C.c[a].n);
+    return dim3((unsigned)blocks_for(((long long)n + 3) / 4), 1, (unsigned)ncomp);
+}
+
+// createExtrapolateToRegion3 from the faces whose `from` byte is 0, `depth` layers
+int extend(cudaStream_t s, const G3 &g, int ncomp, float *const data[3], uint8_t *const from[3],
+           uint8_t *const lay[3], int depth) {
+    const Comps3 C = comps3(g, data, ncomp);
+    const dim3 grid = quad_grid(C, ncomp);
+    Layers3 src{}, dst{};
+    for (int a = 0; a < ncomp; ++a) {
+        src.b[a] = from[a];
+        dst.b[a] = lay[a];
+    }
+    for (int it = 0, t = 1; it < depth; ++it, ++t) {
+        if (t > LAYER_STEPS) {
+            k_fold<<<grid, 256, 0, s>>>(C, dst);
+            t = 1;
+        }
+        k_extend<<<grid, 256, 0, s>>>(C, it == 0 ? src : dst, dst, t);
+    }
+    return post("extrapolate");
+}
+
 // mulberry32 (jitter_random.js:29-41)
 struct Mulberry32 {
     uint32_t state;
@@ -800,8 +927,8 @@ struct ff_flip_s {
     ff_field pos = nullptr, vel = nullptr, conc = nullptr, mask = nullptr, active = nullptr, target = nullptr;
     ff_field cell_conc = nullptr, cell_rho = nullptr, beta[3] = {};
     float *old[3] = {};
-    int *num[3] = {}, *den[3] = {}, *valid[3] = {}, *adj[3] = {}, *vtmp[2][3] = {};
-    float *scratch[3] = {};
+    int *num[3] = {}, *den[3] = {};
+    uint8_t *valid[3] = {}, *adj[3] = {}, *lay[3] = {};   // extension bytes: after P2G, by fluid adjacency, work
     int *ccnt = nullptr, *cacc = nullptr;
     // resampling: per-cell counts, the donor pool, block totals (particle
     // blocks then cell blocks) and the two totals
@@ -838,9 +965,7 @@ extern "C" int ff_flip3_destroy(ff_flip f) {
         ff_dev_free(f->den[a]);
         ff_dev_free(f->valid[a]);
         ff_dev_free(f->adj[a]);
-        ff_dev_free(f->vtmp[0][a]);
-        ff_dev_free(f->vtmp[1][a]);
-        ff_dev_free(f->scratch[a]);
+        ff_dev_free(f->lay[a]);
     }
     ff_dev_free(f->ccnt);
     ff_dev_free(f->cacc);
@@ -911,11 +1036,13 @@ extern "C" int ff_flip3_create(ff_ctx ctx, const ff_flip_desc *d, ff_field u, ff
         if ((st = ff_dev_alloc((void **)&f->old[a], b, s))) return bail(st);
         if ((st = ff_dev_alloc((void **)&f->num[a], b, s))) return bail(st);
         if ((st = ff_dev_alloc((void **)&f->den[a], b, s))) return bail(st);
-        if ((st = ff_dev_alloc((void **)&f->valid[a], b, s))) return bail(st);
-        if ((st = ff_dev_alloc((void **)&f->adj[a], b, s))) return bail(st);
-        if ((st = ff_dev_alloc((void **)&f->vtmp[0][a], b, s))) return bail(st);
-        if ((st = ff_dev_alloc((void **)&f->vtmp[1][a], b, s))) return bail(st);
-        if ((st = ff_dev_alloc((void **)&f->scratch[a], b, s))) return bail(st);
+        if ((st = ff_dev_alloc((void **)&f->valid[a], b / 4, s))) return bail(st);
+        if ((st = ff_dev_alloc((void **)&f->adj[a], b / 4, s))) return bail(st);
+        if ((st = ff_dev_alloc((void **)&f->lay[a], b / 4, s))) return bail(st);
+        // no P2G and no fluid mask yet: no face is valid
+        if (cudaMemsetAsync(f->valid[a], LAYER_OPEN, b / 4, s) != cudaSuccess ||
+            cudaMemsetAsync(f->adj[a], LAYER_OPEN, b / 4, s) != cudaSuccess)
+            return bail(ff_set_error(FF_E_CUDA, "flip create"));
         if (density) {
             const int fs3[3] = {f->g.nx + (a == 0), f->g.ny + (a == 1), f->g.nz + (a == 2)};
             if ((st = ff_field_create(ctx, FF_FLOAT, 3, fs3, &f->beta[a]))) return bail(st);
@@ -1012,23 +1139,6 @@ extern "C" int ff_flip3_grid_fields(ff_flip f, ff_field *cell_concentration, ff_
     return FF_OK;
 }
 
-static int extrapolate(ff_flip f, float *data, const int *marker, int a) {
-    cudaStream_t s = f->ctx->stream;
-    int sx, sy, sz;
-    comp_shape(f->g, a, sx, sy, sz);
-    const long long n = comp_n(f->g, a);
-    FF_CUDA(cudaMemcpyAsync(f->vtmp[0][a], marker, n * 4, cudaMemcpyDeviceToDevice, s));
-    float *src = data, *dst = f->scratch[a];
-    int *vs = f->vtmp[0][a], *vd = f->vtmp[1][a];
-    for (int it = 0; it < f->desc.extrapolation_depth; ++it) {
-        k_extrapolate<<<blocks_for(n), 256, 0, s>>>(sx, sy, sz, src, dst, vs, vd);
-        std::swap(src, dst);
-        std::swap(vs, vd);
-    }
-    if (src != data) FF_CUDA(cudaMemcpyAsync(data, src, n * 4, cudaMemcpyDeviceToDevice, s));
-    return post("extrapolate");
-}
-
 // One stage of onAdvanceTimeStep (:1110-1150).
 extern "C" int ff_flip3_stage(ff_flip f, int stage) {
     FF_CHECK(f, FF_E_ARG, "NULL FLIP solver");
@@ -1071,15 +1181,17 @@ extern "C" int ff_flip3_stage(ff_flip f, int stage) {
             FF_CUDA(cudaMemcpyAsync(f->old[a], uvw[a], comp_n(g, a) * 4, cudaMemcpyDeviceToDevice, s));
         return FF_OK;
     case FF_FLIP_EXTRAPOLATE_WEIGHT:
-        for (int a = 0; a < 3; ++a) FF_TRY(extrapolate(f, uvw[a], f->valid[a], a));
-        return FF_OK;
+        return extend(s, g, 3, uvw, f->valid, f->lay, d.extrapolation_depth);
     case FF_FLIP_CONSTRAIN:
         return ff_bc3_constrain(f->bc, f->u, f->v, f->w, d.extrapolation_depth);
     case FF_FLIP_MARK_FLUID:
         FF_CUDA(cudaMemsetAsync(f->mask->d, 0, comp_n(g, 3) * 4, s));
         if (n) k_flip_mark<<<blocks_for(n), 256, 0, s>>>(g, n, pos, (float *)f->mask->d);
-        for (int a = 0; a < 3; ++a)
-            k_flip_adjacent<<<blocks_for(comp_n(g, a)), 256, 0, s>>>(g, a, (const float *)f->mask->d, f->adj[a]);
+        {
+            const Comps3 C = comps3(g, uvw, 3);
+            k_flip_adjacent<<<quad_grid(C, 3), 256, 0, s>>>(g, C, (const float *)f->mask->d,
+                                                            Layers3{{f->adj[0], f->adj[1], f->adj[2]}});
+        }
         return post("markFluidCells");
     case FF_FLIP_CONCENTRATION_GRID: {
         if (!d.carry_concentration) return FF_OK;
@@ -1116,8 +1228,7 @@ extern "C" int ff_flip3_stage(ff_flip f, int stage) {
         return ff_pressure3_project(f->ps, f->u, f->v, f->w, f->u, f->v, f->w, &f->last);
     }
     case FF_FLIP_EXTRAPOLATE_PRESSURE:
-        for (int a = 0; a < 3; ++a) FF_TRY(extrapolate(f, uvw[a], f->adj[a], a));
-        return FF_OK;
+        return extend(s, g, 3, uvw, f->adj, f->lay, d.extrapolation_depth);
     case FF_FLIP_G2P:
         if (n) k_flip_g2p<<<blocks_for(n), 256, 0, s>>>(g, n, pos, vel, uvw[0], uvw[1], uvw[2], f->old[0], f->old[1],
                                                         f->old[2], (float)d.flip_ratio,
@@ -1243,8 +1354,8 @@ struct ff_twophase_s {
     ff_field pos = nullptr, vel = nullptr, phase = nullptr, frac = nullptr, rho = nullptr, beta[3] = {};
     ff_field active = nullptr, target = nullptr;
     float *old[3] = {};
-    int *num[3] = {}, *den[3] = {}, *valid[3] = {}, *vtmp[2][3] = {};
-    float *scratch[3] = {};
+    int *num[3] = {}, *den[3] = {};
+    uint8_t *valid[3] = {}, *lay[3] = {};   // extension bytes: after P2G, work
     int *ccnt = nullptr, *cacc = nullptr;
     int *rs_need = nullptr, *rs_pool = nullptr;
     long long *rs_bsum = nullptr, *rs_tot = nullptr;
@@ -1268,9 +1379,7 @@ extern "C" int ff_twophase2_destroy(ff_twophase t) {
         ff_dev_free(t->num[a]);
         ff_dev_free(t->den[a]);
         ff_dev_free(t->valid[a]);
-        ff_dev_free(t->vtmp[0][a]);
-        ff_dev_free(t->vtmp[1][a]);
-        ff_dev_free(t->scratch[a]);
+        ff_dev_free(t->lay[a]);
     }
     void *ps[] = {t->ccnt, t->cacc, t->rs_need, t->rs_pool, t->rs_bsum, t->rs_tot};
     for (void *p : ps) ff_dev_free(p);
@@ -1330,10 +1439,10 @@ static int tp_setup(ff_twophase t) {
         if ((st = ff_dev_alloc((void **)&t->old[a], b, s))) return st;
         if ((st = ff_dev_alloc((void **)&t->num[a], b, s))) return st;
         if ((st = ff_dev_alloc((void **)&t->den[a], b, s))) return st;
-        if ((st = ff_dev_alloc((void **)&t->valid[a], b, s))) return st;
-        if ((st = ff_dev_alloc((void **)&t->vtmp[0][a], b, s))) return st;
-        if ((st = ff_dev_alloc((void **)&t->vtmp[1][a], b, s))) return st;
-        if ((st = ff_dev_alloc((void **)&t->scratch[a], b, s))) return st;
+        if ((st = ff_dev_alloc((void **)&t->valid[a], b / 4, s))) return st;
+        if ((st = ff_dev_alloc((void **)&t->lay[a], b / 4, s))) return st;
+        // no P2G yet: no face is valid
+        if (cudaMemsetAsync(t->valid[a], LAYER_OPEN, b / 4, s) != cudaSuccess) return ff_set_error(FF_E_CUDA, "twophase");
     }
     if ((st = ff_dev_alloc((void **)&t->ccnt, (size_t)nc * 4, s))) return st;
     if ((st = ff_dev_alloc((void **)&t->cacc, (size_t)nc * 4, s))) return st;
@@ -1650,23 +1759,6 @@ extern "C" int ff_twophase3_cell_counts(ff_twophase t, int32_t *count, int32_t *
     return FF_OK;
 }
 
-static int tp_extrapolate(ff_twophase t, float *data, const int *marker, int a) {
-    cudaStream_t s = t->ctx->stream;
-    int sx, sy, sz;
-    comp_shape(t->g, a, sx, sy, sz);
-    const long long n = comp_n(t->g, a);
-    FF_CUDA(cudaMemcpyAsync(t->vtmp[0][a], marker, n * 4, cudaMemcpyDeviceToDevice, s));
-    float *src = data, *dst = t->scratch[a];
-    int *vs = t->vtmp[0][a], *vd = t->vtmp[1][a];
-    for (int it = 0; it < t->d.extrapolation_depth; ++it) {
-        k_extrapolate<<<blocks_for(n), 256, 0, s>>>(sx, sy, sz, src, dst, vs, vd);
-        std::swap(src, dst);
-        std::swap(vs, vd);
-    }
-    if (src != data) FF_CUDA(cudaMemcpyAsync(data, src, n * 4, cudaMemcpyDeviceToDevice, s));
-    return post("extrapolate");
-}
-
 // One stage of onAdvanceTimeStep (:1505-1592).  The 2D solver's grid is one
 // cell thick with an internal zero w; the 3D solver moves all three
 // components.
@@ -1728,8 +1820,7 @@ extern "C" int ff_twophase2_stage(ff_twophase t, int stage) {
             FF_CUDA(cudaMemcpyAsync(t->old[a], uvw[a], comp_n(g, a) * 4, cudaMemcpyDeviceToDevice, s));
         return FF_OK;
     case FF_TP_EXTRAPOLATE_WEIGHT:
-        for (int a = 0; a < na; ++a) FF_TRY(tp_extrapolate(t, uvw[a], t->valid[a], a));
-        return FF_OK;
+        return extend(s, g, na, uvw, t->valid, t->lay, d.extrapolation_depth);
     case FF_TP_CONSTRAIN:
         // in 2D the grid's u and v are the 3D arrays' k = 0 planes
         return ff_bc3_constrain(t->bc, t->u, t->v, t->w, d.extrapolation_depth);

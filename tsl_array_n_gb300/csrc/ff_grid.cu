@@ -19,34 +19,126 @@
 namespace {
 using namespace ffg;
 
+// The constraint's work outside the obstacle is one read of the weights and
+// one of the values: a 256^3 grid has 50M faces, of which the collider
+// closes 0.2M, and only those change before the clamp.  So the marking pass
+// lists them, the extension steps, the no-flux projection and its write-back
+// run over the list, and the last pass writes a face only when it changes.
+// Measured at 256^3 around a sphere of radius 24 cells, back to back: 0.18 ms
+// a call (mark 52 us, clamp 39 us and solid cells 17 us with cold caches, at
+// 4.8, 5.2 and 3.9 TB/s; the list kernels 2-10 us each), against 2.43 ms for
+// passes over every face with int32 markers (five extension passes of 88 us a
+// component, no-flux 118 us, copies).
+struct FaceLists {
+    uint8_t *layer[3];   // extension bytes (extend_face)
+    int *list[3];        // listed faces, in no fixed order
+    float *temp[3];      // the no-flux result, by list position
+    unsigned *count;     // entries per component
+    const float *cw[3];  // collider face weights, or null
+};
+
+// appends this lane's faces (`keep` bit m: face f0 + m) to the list; every
+// lane of the warp takes part
+__device__ __forceinline__ void list_append(unsigned keep, unsigned f0, int *__restrict__ list, unsigned *count) {
+    if (!__ballot_sync(0xffffffffu, keep != 0)) return;
+    const int lane = threadIdx.x & 31, mine = __popc(keep);
+    int s = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += t;
+    }
+    unsigned base = 0;
+    if (lane == 31) base = atomicAdd(count, (unsigned)s);
+    base = __shfl_sync(0xffffffffu, base, 31) + (unsigned)(s - mine);
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+        if (keep >> m & 1) list[base++] = (int)(f0 + m);
+}
+
 // makeMarkAndProject (grid_blocked_boundary_condition_solver3.js:196-249):
-// open faces are fluid (marker 1); closed faces take the collider's
-// velocity (a static collider: 0) and marker 0
-__global__ void __launch_bounds__(256, 6) k_mark(VelField F, int a, const float *__restrict__ cw, float *__restrict__ data,
-                       int *__restrict__ marker) {
-    int sx, sy, sz;
-    comp_shape(F.g, a, sx, sy, sz);
-    const long long n = (long long)sx * sy * sz;
+// open faces are valid; closed faces take the collider's velocity (a static
+// collider: 0) and are listed.  Four faces a thread (16-byte weights, one
+// word of layer bytes; every array is 256-byte aligned and padded).
+__global__ void __launch_bounds__(256) k_mark(Comps3 C, FaceLists L) {
+    const int a = blockIdx.z;
+    const CompDims &c = C.c[a];
+    const float *__restrict__ cw = L.cw[a];
+    const unsigned nq = (c.n + 3) / 4, step = gridDim.x * blockDim.x;
+    // whole warps step together (list_append shuffles), two quads' loads in flight a thread
+    for (unsigned q0 = blockIdx.x * blockDim.x + threadIdx.x; (q0 & ~31u) < nq; q0 += 2 * step) {
+        const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
+        const float4 w4[2] = {q0 < nq ? __ldg(reinterpret_cast<const float4 *>(cw) + q0) : one,
+                              q0 + step < nq ? __ldg(reinterpret_cast<const float4 *>(cw) + q0 + step) : one};
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const unsigned q = q0 + p * step, f0 = 4 * q;
+            const float wv[4] = {w4[p].x, w4[p].y, w4[p].z, w4[p].w};
+            unsigned keep = 0, bytes = 0;
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+                if (f0 + m < c.n && !(wv[m] > 0.0f)) {
+                    keep |= 1u << m;
+                    bytes |= LAYER_OPEN << (8 * m);
+                    C.d[a][f0 + m] = 0.0f;
+                }
+            if (q < nq) reinterpret_cast<unsigned *>(L.layer[a])[q] = bytes;
+            list_append(keep, f0, L.list[a], L.count + a);
+        }
+    }
+}
+
+// whether the no-flux projection replaces a face (makeNoFluxProjection, :251-286)
+__device__ __forceinline__ bool face_blocked(const VelField &F, const float *cw, unsigned f, F3 pt) {
+    return cw ? (cw[f] <= 0.0f) : (sample_phi(F, F.phi, pt) < 0.0f);
+}
+
+// k_mark without collider weights: the open fraction from the SDF on the
+// two sides of the face; listed when closed or blocked
+__global__ void __launch_bounds__(256, 6) k_mark_sdf(VelField F, Comps3 C, FaceLists L) {
+    const int a = blockIdx.z;
+    const CompDims &c = C.c[a];
     const F3 o = comp_origin(F.g, a);
-    for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < n; f += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        unflatten(f, sx, sy, i, j, k);
-        float open;
-        if (cw) {
-            open = cw[f];
-        } else {
+    const F3 off{a == 0 ? F.g.hx * 0.5f : 0.0f, a == 1 ? F.g.hy * 0.5f : 0.0f, a == 2 ? F.g.hz * 0.5f : 0.0f};
+    for (unsigned f0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); f0 < c.n; f0 += gridDim.x * blockDim.x) {
+        const unsigned f = f0 + (threadIdx.x & 31u);
+        unsigned keep = 0;
+        if (f < c.n) {
+            int i, j, k;
+            c.at(f, i, j, k);
             const F3 pt = index_pos(F.g, o, i, j, k);
-            const F3 off{a == 0 ? F.g.hx * 0.5f : 0.0f, a == 1 ? F.g.hy * 0.5f : 0.0f, a == 2 ? F.g.hz * 0.5f : 0.0f};
             const float fr = frac_inside_sdf(sample_phi(F, F.phi, F3{pt.x - off.x, pt.y - off.y, pt.z - off.z}),
                                              sample_phi(F, F.phi, F3{pt.x + off.x, pt.y + off.y, pt.z + off.z}));
-            open = 1.0f - fminf(fmaxf(fr, 0.0f), 1.0f);
+            const bool open = 1.0f - fminf(fmaxf(fr, 0.0f), 1.0f) > 0.0f;
+            if (!open) C.d[a][f] = 0.0f;
+            L.layer[a][f] = open ? 0 : LAYER_OPEN;
+            keep = (!open || face_blocked(F, nullptr, f, pt)) ? 1u : 0u;
         }
-        if (open > 0.0f) {
-            marker[f] = 1;
-        } else {
-            data[f] = 0.0f;
-            marker[f] = 0;
+        list_append(keep, f, L.list[a], L.count + a);
+    }
+}
+
+// extension step t over the listed faces
+__global__ void __launch_bounds__(256) k_extend_list(Comps3 C, FaceLists L, int t) {
+    const int a = blockIdx.z;
+    const unsigned n = L.count[a];
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+        const unsigned f = (unsigned)L.list[a][q];
+        float v;
+        if (L.layer[a][f] == LAYER_OPEN && extend_face(C.c[a], C.d[a], L.layer[a], f, t, v)) {
+            C.d[a][f] = v;
+            L.layer[a][f] = (uint8_t)t;
         }
+    }
+}
+
+// folds the bytes of the listed faces: valid ones to 0 (steps then count from 1 again)
+__global__ void __launch_bounds__(256) k_fold_list(FaceLists L) {
+    const int a = blockIdx.z;
+    const unsigned n = L.count[a];
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+        uint8_t &b = L.layer[a][L.list[a][q]];
+        if (b != LAYER_OPEN) b = 0;
     }
 }
 
@@ -116,90 +208,162 @@ __global__ void k_trace(VelField F, long long n, const float *__restrict__ pin, 
     }
 }
 
-// makeNoFluxProjection (:251-286) with projectAndApplyFriction (:30-44):
-// a closed face takes the tangential part of the sampled velocity,
-// reduced by Coulomb friction (coefficient 0.5, sdf_collider3.js:16)
-__global__ void __launch_bounds__(256, 6) k_noflux(VelField F, int a, const float *__restrict__ cw, const float *__restrict__ data,
-                         float *__restrict__ temp) {
-    int sx, sy, sz;
-    comp_shape(F.g, a, sx, sy, sz);
-    const long long n = (long long)sx * sy * sz;
+// makeNoFluxProjection (:251-286) with projectAndApplyFriction (:30-44)
+// over the listed faces: a blocked face takes the tangential part of the
+// sampled velocity, reduced by Coulomb friction (coefficient 0.5,
+// sdf_collider3.js:16).  The samples read the values of all components
+// before any face is replaced, so the results wait in temp.
+__global__ void __launch_bounds__(256) k_noflux(VelField F, Comps3 C, FaceLists L) {
+    const int a = blockIdx.z;
+    const CompDims &c = C.c[a];
+    const unsigned n = L.count[a];
     const F3 o = comp_origin(F.g, a), oc = comp_origin(F.g, 3);
-    for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < n; f += (long long)gridDim.x * blockDim.x) {
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+        const unsigned f = (unsigned)L.list[a][q];
         int i, j, k;
-        unflatten(f, sx, sy, i, j, k);
+        c.at(f, i, j, k);
         const F3 pt = index_pos(F.g, o, i, j, k);
-        const bool blocked = cw ? (cw[f] <= 0.0f) : (sample_phi(F, F.phi, pt) < 0.0f);
-        if (!blocked) {
-            temp[f] = data[f];
-            continue;
-        }
-        const F3 vel = sample_vel(F, pt);
-        const F3 gr = trilinear_gradient(F.phi, F.g, oc, pt);
-        const float gl = sqrtf(gr.x * gr.x + gr.y * gr.y + gr.z * gr.z);
-        if (gl > 0.0f) {
-            const F3 nn{gr.x / gl, gr.y / gl, gr.z / gl};
-            const float vn = vel.x * nn.x + vel.y * nn.y + vel.z * nn.z;
-            F3 vt{vel.x - nn.x * vn, vel.y - nn.y * vn, vel.z - nn.z * vn};
-            const float tl = sqrtf(vt.x * vt.x + vt.y * vt.y + vt.z * vt.z);
-            if (tl > 0.0f) {
-                const float veln = fmaxf(-vn, 0.0f);
-                const float scale = fmaxf(1.0f - veln * 0.5f / tl, 0.0f);
-                vt = F3{vt.x * scale, vt.y * scale, vt.z * scale};
+        float res = C.d[a][f];
+        if (face_blocked(F, L.cw[a], f, pt)) {
+            const F3 vel = sample_vel(F, pt);
+            const F3 gr = trilinear_gradient(F.phi, F.g, oc, pt);
+            const float gl = sqrtf(gr.x * gr.x + gr.y * gr.y + gr.z * gr.z);
+            res = 0.0f;
+            if (gl > 0.0f) {
+                const F3 nn{gr.x / gl, gr.y / gl, gr.z / gl};
+                const float vn = vel.x * nn.x + vel.y * nn.y + vel.z * nn.z;
+                F3 vt{vel.x - nn.x * vn, vel.y - nn.y * vn, vel.z - nn.z * vn};
+                const float tl = sqrtf(vt.x * vt.x + vt.y * vt.y + vt.z * vt.z);
+                if (tl > 0.0f) {
+                    const float veln = fmaxf(-vn, 0.0f);
+                    const float scale = fmaxf(1.0f - veln * 0.5f / tl, 0.0f);
+                    vt = F3{vt.x * scale, vt.y * scale, vt.z * scale};
+                }
+                res = a == 0 ? vt.x : (a == 1 ? vt.y : vt.z);
             }
-            temp[f] = a == 0 ? vt.x : (a == 1 ? vt.y : vt.z);
-        } else {
-            temp[f] = 0.0f;
         }
+        L.temp[a][q] = res;
     }
+}
+__global__ void __launch_bounds__(256) k_noflux_write(Comps3 C, FaceLists L) {
+    const int a = blockIdx.z;
+    const unsigned n = L.count[a];
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
+        C.d[a][L.list[a][q]] = L.temp[a][q];
 }
 
 // blockedBoundary (:288-330): a collider cell's faces toward fluid cells
-// take the collider velocity (0)
-__global__ void k_blocked(G3 g, const float *__restrict__ phi, float *u, float *v, float *w) {
-    const long long n = (long long)g.nx * g.ny * g.nz;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        unflatten(c, g.nx, g.ny, i, j, k);
-        auto solid = [&](int ii, int jj, int kk) { return phi[ii + (long long)g.nx * (jj + (long long)g.ny * kk)] < 0.0f; };
-        if (!solid(i, j, k)) continue;
-        const int nx = g.nx, ny = g.ny, nz = g.nz;
-        if (i > 0 && !solid(i - 1, j, k)) u[i + (long long)(nx + 1) * (j + (long long)ny * k)] = 0.0f;
-        if (i < nx - 1 && !solid(i + 1, j, k)) u[i + 1 + (long long)(nx + 1) * (j + (long long)ny * k)] = 0.0f;
-        if (j > 0 && !solid(i, j - 1, k)) v[i + (long long)nx * (j + (long long)(ny + 1) * k)] = 0.0f;
-        if (j < ny - 1 && !solid(i, j + 1, k)) v[i + (long long)nx * (j + 1 + (long long)(ny + 1) * k)] = 0.0f;
-        if (k > 0 && !solid(i, j, k - 1)) w[i + (long long)nx * (j + (long long)ny * k)] = 0.0f;
-        if (k < nz - 1 && !solid(i, j, k + 1)) w[i + (long long)nx * (j + (long long)ny * (k + 1))] = 0.0f;
+// take the collider velocity (0).  Four cells a thread; a cell outside the
+// collider costs its share of one 16-byte load.
+__global__ void __launch_bounds__(256) k_blocked(G3 g, CompDims c, const float *__restrict__ phi, float *u, float *v,
+                                                 float *w) {
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const unsigned nq = (c.n + 3) / 4;
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
+        const float4 p4 = __ldg(reinterpret_cast<const float4 *>(phi) + q);
+        if (!(p4.x < 0.0f || p4.y < 0.0f || p4.z < 0.0f || p4.w < 0.0f)) continue;
+        const float pv[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const unsigned f = 4 * q + m;
+            if (f >= c.n || !(pv[m] < 0.0f)) continue;
+            int i, j, k;
+            c.at(f, i, j, k);
+            auto solid = [&](int ii, int jj, int kk) { return phi[ii + nx * (jj + ny * kk)] < 0.0f; };
+            if (i > 0 && !solid(i - 1, j, k)) u[i + (nx + 1) * (j + ny * k)] = 0.0f;
+            if (i < nx - 1 && !solid(i + 1, j, k)) u[i + 1 + (nx + 1) * (j + ny * k)] = 0.0f;
+            if (j > 0 && !solid(i, j - 1, k)) v[i + nx * (j + (ny + 1) * k)] = 0.0f;
+            if (j < ny - 1 && !solid(i, j + 1, k)) v[i + nx * (j + 1 + (ny + 1) * k)] = 0.0f;
+            if (k > 0 && !solid(i, j, k - 1)) w[i + nx * (j + ny * k)] = 0.0f;
+            if (k < nz - 1 && !solid(i, j, k + 1)) w[i + nx * (j + ny * (k + 1))] = 0.0f;
+        }
     }
 }
 
-// walls (zeroULeft .. zeroWFront), inflows (buildInflowKernels) and the
-// final clamp (clampComponent, |v| <= 100, non-finite -> 0), per component
-__global__ void __launch_bounds__(256, 6) k_walls_inflow_clamp(G3 g, int a, float *__restrict__ data, int closed, int n_in,
-                                     const float *const *__restrict__ in_phi, const float *__restrict__ in_vel,
-                                     const int *__restrict__ in_mode) {
-    int sx, sy, sz;
-    comp_shape(g, a, sx, sy, sz);
-    const long long n = (long long)sx * sy * sz;
-    const F3 o = comp_origin(g, a);
-    for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < n; f += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        unflatten(f, sx, sy, i, j, k);
-        float val = data[f];
-        const int idx = a == 0 ? i : (a == 1 ? j : k), last = (a == 0 ? sx : (a == 1 ? sy : sz)) - 1;
-        if (((closed >> (2 * a)) & 1) && idx == 0) val = 0.0f;
-        if (((closed >> (2 * a + 1)) & 1) && idx == last) val = 0.0f;
-        if (n_in) {
-            const F3 pt = index_pos(g, o, i, j, k);
-            VelField F{g, nullptr, nullptr, nullptr, nullptr};
-            for (int q = 0; q < n_in; ++q) {
-                if (sample_phi(F, in_phi[q], pt) < 0.0f) {
-                    const float add = in_vel[3 * q + a];
-                    val = in_mode[q] ? val + add : add;
+// the clamp (clampComponent, |v| <= 100, non-finite -> 0) after the walls
+// (zeroULeft .. zeroWFront)
+__device__ __forceinline__ float clamp_vel(float val) {
+    return (isnan(val) || isinf(val)) ? 0.0f : fminf(fmaxf(val, -100.0f), 100.0f);
+}
+__device__ __forceinline__ bool closed_face(const CompDims &c, int a, int closed, int i, int j, int k) {
+    const int idx = a == 0 ? i : (a == 1 ? j : k), last = (a == 0 ? c.sx : (a == 1 ? c.sy : c.sz)) - 1;
+    return (((closed >> (2 * a)) & 1) && idx == 0) || (((closed >> (2 * a + 1)) & 1) && idx == last);
+}
+// walls and clamp, four faces a thread (two quads' loads in flight); a face
+// is written only when its bits change.  Most quads hold no wall face and no
+// value to clamp: a test on the index along the component's axis and one on
+// the magnitudes dismiss them, which keeps the pass near its read of the
+// values (with the full test on each face it was bound by issue: 62 us for
+// 256^3, cold).
+__global__ void __launch_bounds__(256) k_walls_clamp(Comps3 C, int closed) {
+    const int a = blockIdx.z;
+    const CompDims &c = C.c[a];
+    float *__restrict__ data = C.d[a];
+    const unsigned nq = (c.n + 3) / 4, step = gridDim.x * blockDim.x;
+    const unsigned plane = (unsigned)c.sx * (unsigned)c.sy;
+    for (unsigned q0 = blockIdx.x * blockDim.x + threadIdx.x; q0 < nq; q0 += 2 * step) {
+        const bool two = q0 + step < nq;
+        const float4 v4[2] = {reinterpret_cast<const float4 *>(data)[q0],
+                              two ? reinterpret_cast<const float4 *>(data)[q0 + step] : make_float4(0.f, 0.f, 0.f, 0.f)};
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const unsigned f0 = 4 * (q0 + p * step);
+            const float vv[4] = {v4[p].x, v4[p].y, v4[p].z, v4[p].w};
+            // no value to clamp: |v| <= 100 fails for a NaN too
+            const bool plain = fabsf(vv[0]) <= 100.0f && fabsf(vv[1]) <= 100.0f && fabsf(vv[2]) <= 100.0f &&
+                               fabsf(vv[3]) <= 100.0f;
+            // whether f0 .. f0 + 3 can hold a face of the axis' end planes
+            bool edge;
+            const unsigned r = c.dx.div(f0);
+            if (a == 0) {
+                const unsigned i = f0 - r * (unsigned)c.sx;
+                edge = i == 0 || i + 4 >= (unsigned)c.sx;
+            } else if (a == 1) {
+                const unsigned j = r - c.dy.div(r) * (unsigned)c.sy;
+                edge = j == 0 || j + 5 >= (unsigned)c.sy;
+            } else {
+                edge = f0 < plane || f0 + 4 >= c.n - plane;
+            }
+            if (plain && !edge) continue;
+            if (f0 >= c.n) break;
+            int i, j, k;
+            c.at(f0, i, j, k);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const float w = clamp_vel(closed_face(c, a, closed, i, j, k) ? 0.0f : vv[m]);
+                if (__float_as_uint(w) != __float_as_uint(vv[m]) && f0 + m < c.n) data[f0 + m] = w;
+                if (++i == c.sx) {
+                    i = 0;
+                    if (++j == c.sy) j = 0, ++k;
                 }
             }
         }
-        data[f] = (isnan(val) || isinf(val)) ? 0.0f : fminf(fmaxf(val, -100.0f), 100.0f);
+    }
+}
+// the same with inflows (buildInflowKernels) between the walls and the clamp
+__global__ void __launch_bounds__(256, 6) k_walls_inflow_clamp(G3 g, Comps3 C, int closed, int n_in,
+                                                               const float *const *__restrict__ in_phi,
+                                                               const float *__restrict__ in_vel,
+                                                               const int *__restrict__ in_mode) {
+    const int a = blockIdx.z;
+    const CompDims &c = C.c[a];
+    float *__restrict__ data = C.d[a];
+    const F3 o = comp_origin(g, a);
+    const VelField F{g, nullptr, nullptr, nullptr, nullptr};
+    for (unsigned f = blockIdx.x * blockDim.x + threadIdx.x; f < c.n; f += gridDim.x * blockDim.x) {
+        int i, j, k;
+        c.at(f, i, j, k);
+        const float old = data[f];
+        float val = closed_face(c, a, closed, i, j, k) ? 0.0f : old;
+        const F3 pt = index_pos(g, o, i, j, k);
+        for (int q = 0; q < n_in; ++q) {
+            if (sample_phi(F, in_phi[q], pt) < 0.0f) {
+                const float add = in_vel[3 * q + a];
+                val = in_mode[q] ? val + add : add;
+            }
+        }
+        val = clamp_vel(val);
+        if (__float_as_uint(val) != __float_as_uint(old)) data[f] = val;
     }
 }
 
@@ -398,8 +562,7 @@ struct ff_bc_s {
     G3 g{};
     int closed = 63;                       // DIRECTION_ALL_3D
     ff_field phi = nullptr, cw[3] = {};    // borrowed
-    int *marker[3] = {}, *valid[2][3] = {};
-    float *temp[3] = {}, *scratch[3] = {};
+    FaceLists lists{};                     // work arrays (cw filled in per call)
     int n_in = 0;
     const float **in_phi = nullptr;        // device array of n_in pointers
     float *in_vel = nullptr;
@@ -418,12 +581,11 @@ extern "C" int ff_bc3_create(ff_ctx ctx, const int *res, const double *h, const 
     int st = FF_OK;
     for (int a = 0; a < 3 && st == FF_OK; ++a) {
         const size_t n = (size_t)comp_count(b->g, a);
-        st = ff_dev_alloc((void **)&b->marker[a], n * 4, ctx->stream);
-        if (st == FF_OK) st = ff_dev_alloc((void **)&b->valid[0][a], n * 4, ctx->stream);
-        if (st == FF_OK) st = ff_dev_alloc((void **)&b->valid[1][a], n * 4, ctx->stream);
-        if (st == FF_OK) st = ff_dev_alloc((void **)&b->temp[a], n * 4, ctx->stream);
-        if (st == FF_OK) st = ff_dev_alloc((void **)&b->scratch[a], n * 4, ctx->stream);
+        st = ff_dev_alloc((void **)&b->lists.layer[a], n, ctx->stream);
+        if (st == FF_OK) st = ff_dev_alloc((void **)&b->lists.list[a], n * 4, ctx->stream);
+        if (st == FF_OK) st = ff_dev_alloc((void **)&b->lists.temp[a], n * 4, ctx->stream);
     }
+    if (st == FF_OK) st = ff_dev_alloc((void **)&b->lists.count, 3 * sizeof(unsigned), ctx->stream);
     if (st != FF_OK) {
         ff_bc3_destroy(b);
         return st;
@@ -436,12 +598,11 @@ extern "C" int ff_bc3_destroy(ff_bc b) {
     if (!b) return FF_OK;
     cudaStreamSynchronize(b->ctx->stream);
     for (int a = 0; a < 3; ++a) {
-        ff_dev_free(b->marker[a]);
-        ff_dev_free(b->valid[0][a]);
-        ff_dev_free(b->valid[1][a]);
-        ff_dev_free(b->temp[a]);
-        ff_dev_free(b->scratch[a]);
+        ff_dev_free(b->lists.layer[a]);
+        ff_dev_free(b->lists.list[a]);
+        ff_dev_free(b->lists.temp[a]);
     }
+    ff_dev_free(b->lists.count);
     ff_dev_free((void *)b->in_phi);
     ff_dev_free(b->in_vel);
     ff_dev_free(b->in_mode);
@@ -511,42 +672,39 @@ extern "C" int ff_bc3_constrain(ff_bc b, ff_field u, ff_field v, ff_field w, int
         FF_CHECK(field_is(fs[a], comp_count(b->g, a)), FF_E_ARG, "constrainVelocity: velocity component %d shape", a);
     cudaSetDevice(b->ctx->device);
     cudaStream_t s = b->ctx->stream;
-    float *d[3] = {(float *)u->d, (float *)v->d, (float *)w->d};
-    VelField F{b->g, d[0], d[1], d[2], b->phi ? (const float *)b->phi->d : nullptr};
-    if (b->phi) {
-        for (int a = 0; a < 3; ++a) {
-            const long long n = comp_count(b->g, a);
-            k_mark<<<launch_blocks(n), 256, 0, s>>>(F, a, b->cw[a] ? (const float *)b->cw[a]->d : nullptr, d[a],
-                                                    b->marker[a]);
-        }
-        for (int a = 0; a < 3; ++a) {
-            const long long n = comp_count(b->g, a);
-            int sx, sy, sz;
-            comp_shape(b->g, a, sx, sy, sz);
-            FF_CUDA(cudaMemcpyAsync(b->valid[0][a], b->marker[a], n * 4, cudaMemcpyDeviceToDevice, s));
-            float *src = d[a], *dst = b->scratch[a];
-            int *vs = b->valid[0][a], *vd = b->valid[1][a];
-            for (int it = 0; it < depth; ++it) {
-                k_extrapolate<<<launch_blocks(n), 256, 0, s>>>(sx, sy, sz, src, dst, vs, vd);
-                std::swap(src, dst);
-                std::swap(vs, vd);
-            }
-            if (src != d[a]) FF_CUDA(cudaMemcpyAsync(d[a], src, n * 4, cudaMemcpyDeviceToDevice, s));
-        }
-        for (int a = 0; a < 3; ++a) {
-            const long long n = comp_count(b->g, a);
-            k_noflux<<<launch_blocks(n), 256, 0, s>>>(F, a, b->cw[a] ? (const float *)b->cw[a]->d : nullptr, d[a],
-                                                      b->temp[a]);
-        }
-        for (int a = 0; a < 3; ++a)
-            FF_CUDA(cudaMemcpyAsync(d[a], b->temp[a], comp_count(b->g, a) * 4, cudaMemcpyDeviceToDevice, s));
-        k_blocked<<<launch_blocks(comp_count(b->g, 3)), 256, 0, s>>>(b->g, F.phi, d[0], d[1], d[2]);
-    }
+    Comps3 C;
+    long long nmax = 0;
     for (int a = 0; a < 3; ++a) {
-        const long long n = comp_count(b->g, a);
-        k_walls_inflow_clamp<<<launch_blocks(n), 256, 0, s>>>(b->g, a, d[a], b->closed, b->n_in, b->in_phi, b->in_vel,
-                                                              b->in_mode);
+        C.c[a] = comp_dims(b->g, a);
+        C.d[a] = (float *)fs[a]->d;
+        nmax = std::max(nmax, comp_count(b->g, a));
     }
+    const VelField F{b->g, C.d[0], C.d[1], C.d[2], b->phi ? (const float *)b->phi->d : nullptr};
+    const dim3 faces(launch_blocks(nmax), 1, 3), quads(launch_blocks((nmax + 3) / 4), 1, 3);
+    if (b->phi) {
+        FaceLists L = b->lists;
+        for (int a = 0; a < 3; ++a) L.cw[a] = b->cw[a] ? (const float *)b->cw[a]->d : nullptr;
+        // the lists' lengths stay on the device: two blocks an SM and component
+        const dim3 listed((unsigned)std::min<long long>((nmax + 255) / 256, 152LL * 2), 1, 3);
+        FF_CUDA(cudaMemsetAsync(L.count, 0, 3 * sizeof(unsigned), s));
+        if (L.cw[0]) k_mark<<<quads, 256, 0, s>>>(C, L);
+        else k_mark_sdf<<<faces, 256, 0, s>>>(F, C, L);
+        for (int it = 0, t = 1; it < depth; ++it, ++t) {
+            if (t > LAYER_STEPS) {
+                k_fold_list<<<listed, 256, 0, s>>>(L);
+                t = 1;
+            }
+            k_extend_list<<<listed, 256, 0, s>>>(C, L, t);
+        }
+        k_noflux<<<listed, 256, 0, s>>>(F, C, L);
+        k_noflux_write<<<listed, 256, 0, s>>>(C, L);
+        k_blocked<<<launch_blocks((comp_count(b->g, 3) + 3) / 4), 256, 0, s>>>(b->g, comp_dims(b->g, 3), F.phi, C.d[0],
+                                                                              C.d[1], C.d[2]);
+    }
+    if (b->n_in)
+        k_walls_inflow_clamp<<<faces, 256, 0, s>>>(b->g, C, b->closed, b->n_in, b->in_phi, b->in_vel, b->in_mode);
+    else
+        k_walls_clamp<<<quads, 256, 0, s>>>(C, b->closed);
     return post("constrainVelocity");
 }
 

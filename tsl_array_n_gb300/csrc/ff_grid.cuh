@@ -187,34 +187,72 @@ __device__ __forceinline__ float frac_inside_sdf(float p0, float p1) {
     return 0.0f;
 }
 
-// one Jacobi step of createExtrapolateToRegion3 (array_utils3.js:88-150)
-__global__ void __launch_bounds__(256, 8) k_extrapolate(int sx, int sy, int sz, const float *__restrict__ src, float *__restrict__ dst,
-                              const int *__restrict__ vs, int *__restrict__ vd) {
-    const long long n = (long long)sx * sy * sz, sy_ = sx, sz_ = (long long)sx * sy;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        unflatten(c, sx, sy, i, j, k);
-        if (vs[c] != 0) {
-            dst[c] = src[c];
-            vd[c] = 1;
-            continue;
-        }
-        float total = 0.0f;
-        int count = 0;
-        if (i + 1 < sx && vs[c + 1]) { total = total + src[c + 1]; ++count; }
-        if (i > 0 && vs[c - 1]) { total = total + src[c - 1]; ++count; }
-        if (j + 1 < sy && vs[c + sy_]) { total = total + src[c + sy_]; ++count; }
-        if (j > 0 && vs[c - sy_]) { total = total + src[c - sy_]; ++count; }
-        if (k + 1 < sz && vs[c + sz_]) { total = total + src[c + sz_]; ++count; }
-        if (k > 0 && vs[c - sz_]) { total = total + src[c - sz_]; ++count; }
-        if (count > 0) {
-            dst[c] = total / (float)count;
-            vd[c] = 1;
-        } else {
-            dst[c] = src[c];
-            vd[c] = 0;
-        }
+// Division of face indices (below 2^31) by a grid extent as a multiply, an
+// add and a shift: q = (hi(n m) + n) >> s with s = ceil(log2 d) and
+// m = floor(2^32 (2^s - d) / d) + 1 (Granlund and Montgomery 1994).
+struct FastDiv {
+    unsigned d, m, s;
+    __device__ __forceinline__ unsigned div(unsigned n) const { return (__umulhi(n, m) + n) >> s; }
+};
+inline FastDiv fast_div(int d) {
+    unsigned s = 0;
+    while ((1u << s) < (unsigned)d) ++s;
+    const unsigned long long m = ((1ull << 32) * ((1ull << s) - (unsigned)d)) / (unsigned)d + 1;
+    return FastDiv{(unsigned)d, (unsigned)m, s};
+}
+
+// One face component's array extents, and up to three components for one
+// launch (blockIdx.z picks the component).
+struct CompDims {
+    int sx, sy, sz;
+    unsigned n;
+    FastDiv dx, dy;
+    __device__ __forceinline__ void at(unsigned f, int &i, int &j, int &k) const {
+        const unsigned r = dx.div(f), q = dy.div(r);
+        i = (int)(f - r * (unsigned)sx);
+        j = (int)(r - q * (unsigned)sy);
+        k = (int)q;
     }
+};
+inline CompDims comp_dims(const G3 &g, int a) {
+    CompDims c;
+    comp_shape(g, a, c.sx, c.sy, c.sz);
+    c.n = (unsigned)((long long)c.sx * c.sy * c.sz);
+    c.dx = fast_div(c.sx);
+    c.dy = fast_div(c.sy);
+    return c;
+}
+struct Comps3 {
+    CompDims c[3];
+    float *d[3];
+};
+
+// createExtrapolateToRegion3's Jacobi steps (array_utils3.js:88-150) in
+// place.  A face carries one byte: 0 valid from the start, t made valid by
+// step t, LAYER_OPEN not valid yet.  Step t gives a face that is not valid
+// the mean of its neighbours with a byte below t, which no thread of the
+// step writes; a face that the step itself makes valid reads as t or as
+// LAYER_OPEN, and neither is below t.  So one value array and one byte array
+// do for the two value and two marker arrays of the double-buffered form.
+constexpr unsigned LAYER_OPEN = 255;
+constexpr int LAYER_STEPS = 254;   // steps before the bytes are folded back to 0
+
+__device__ __forceinline__ bool extend_face(const CompDims &c, const float *d, const uint8_t *lay, unsigned f, int t,
+                                            float &out) {
+    int i, j, k;
+    c.at(f, i, j, k);
+    const int sy = c.sx, sz = c.sx * c.sy;
+    float total = 0.0f;
+    int count = 0;
+    if (i + 1 < c.sx && lay[f + 1] < t) { total = total + d[f + 1]; ++count; }
+    if (i > 0 && lay[f - 1] < t) { total = total + d[f - 1]; ++count; }
+    if (j + 1 < c.sy && lay[f + sy] < t) { total = total + d[f + sy]; ++count; }
+    if (j > 0 && lay[f - sy] < t) { total = total + d[f - sy]; ++count; }
+    if (k + 1 < c.sz && lay[f + sz] < t) { total = total + d[f + sz]; ++count; }
+    if (k > 0 && lay[f - sz] < t) { total = total + d[f - sz]; ++count; }
+    if (count == 0) return false;
+    out = total / (float)count;
+    return true;
 }
 
 // trilinearGradientAtPosition3 (grid_math3.js:295-352)
