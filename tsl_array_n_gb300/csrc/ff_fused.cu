@@ -2624,6 +2624,101 @@ __device__ void tail_coarse_colour(const TailArgs &a, const TailLevel &C, int co
     }
 }
 
+// All sweeps of a coarsest level of up to TAIL_ONE_BLOCK_COARSE cells in block
+// 0, x in shared memory from the first pass to the last (through L2 a colour
+// pass is two dependent round trips, about 1 us; 40 passes made up most of a
+// small hierarchy's V-cycle).  A cell's operator as the passes use it: the six
+// couplings (0 across the domain edge, where the neighbour index is the cell
+// itself), E, the diagonal and b.
+struct CoarseCell {
+    float k[6], e, D, b;
+    int c, n[6];
+};
+__device__ __forceinline__ CoarseCell coarse_cell(const TailLevel &C, int i, int j, int k) {
+    const Dims d = C.g.d;
+    const int sy = d.nx, sz = d.nx * d.ny;
+    CoarseCell q;
+    q.c = i + sy * j + sz * k;
+    const float4 kc = __ldg(C.coef + q.c);
+    q.e = kc.w;
+    q.D = -(kc.w + kc.x + kc.y + kc.z);
+    const bool in[6] = {i > 0, i < d.nx - 1, j > 0, j < d.ny - 1, k > 0, k < d.nz - 1};
+    const int st[3] = {1, sy, sz};
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+        const int a = f >> 1;
+        q.n[f] = in[f] ? q.c + (f & 1 ? st[a] : -st[a]) : q.c;
+        float kf = 0.f;
+        if (in[f]) {
+            const int cc = f & 1 ? q.n[f] : q.c;
+            kf = a == 0 ? __ldg(&C.coef[cc].x) : (a == 1 ? __ldg(&C.coef[cc].y) : __ldg(&C.coef[cc].z));
+            if (f & 1) q.D -= kf;
+        }
+        q.k[f] = kf;
+    }
+    q.b = __ldcg(C.b + q.c);
+    return q;
+}
+__device__ __forceinline__ void coarse_relax(const CoarseCell &q, float *x, float sor) {
+    const float xc = x[q.c];
+    float s = -q.e * xc;
+#pragma unroll
+    for (int f = 0; f < 6; ++f) s += q.k[f] * (x[q.n[f]] - xc);
+    x[q.c] = xc + ((q.b - s) / q.D) * sor;
+}
+__device__ __forceinline__ void bar_sync_n(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ void tail_coarse_block(const TailArgs &a, const TailLevel &C) {
+    __shared__ float x[TAIL_ONE_BLOCK_COARSE];
+    const Dims d = C.g.d;
+    const int n = (int)d.n(), hx = (d.nx + 1) >> 1, pairs = hx * d.ny * d.nz, tid = threadIdx.x;
+    for (int c = tid; c < n; c += TAIL_NT) x[c] = 0.f;
+    __syncthreads();
+    // cell of colour col of a pair (two neighbours of a row, one of each colour)
+    auto cell_of = [&](int t, int col, int &i, int &j, int &k) {
+        const int r = t / hx;
+        k = r / d.ny;
+        j = r - k * d.ny;
+        i = 2 * (t - r * hx) + ((j + k + col) & 1);
+        return i < d.nx;
+    };
+    if (pairs <= TAIL_NT) {
+        // one pair a thread, its operator in registers; only the warps with
+        // pairs take part in the passes' barriers
+        const int nthr = (pairs + 31) & ~31;
+        if (tid < nthr) {
+            CoarseCell q[2];
+            bool has[2] = {false, false};
+#pragma unroll
+            for (int col = 0; col < 2; ++col) {
+                int i, j, k;
+                if (tid < pairs && cell_of(tid, col, i, j, k)) {
+                    q[col] = coarse_cell(C, i, j, k);
+                    has[col] = true;
+                }
+            }
+            for (int it = 0; it < a.coarse_sweeps; ++it) {
+#pragma unroll
+                for (int col = 0; col < 2; ++col) {
+                    if (has[col]) coarse_relax(q[col], x, a.sor);
+                    bar_sync_n(1, nthr);
+                }
+            }
+        }
+    } else {
+        for (int it = 0; it < 2 * a.coarse_sweeps; ++it) {
+            for (int t = tid; t < pairs; t += TAIL_NT) {
+                int i, j, k;
+                if (cell_of(t, it & 1, i, j, k)) coarse_relax(coarse_cell(C, i, j, k), x, a.sor);
+            }
+            __syncthreads();
+        }
+    }
+    __syncthreads();
+    for (int c = tid; c < n; c += TAIL_NT) C.x[c] = x[c];
+}
+
 // HELD: some levels are held in block 0's shared memory (the instance
 // without them carries none of their dispatch)
 template <bool HELD>
@@ -2728,13 +2823,16 @@ __global__ void __launch_bounds__(TAIL_NT, 1) k_vcycle_tail(TailArgs a) {
     if (ok) {
         const TailLevel &C = a.lv[a.nl - 1];
         if (a.coarse_sweeps > 0) {
-            const bool sc = a.lv[a.nl - 1].g.d.n() <= TAIL_ONE_BLOCK_COARSE;
-            ok = phase(sc, true, [&](long long q0, long long qs) {
-                for (long long c = q0; c < C.g.d.n(); c += qs) C.x[c] = 0.f;
-            });
-            for (int it = 0; it < a.coarse_sweeps && ok; ++it)
-                for (int col = 0; col < 2 && ok; ++col)
-                    ok = phase(sc, true, [&](long long q0, long long qs) { tail_coarse_colour(a, C, col, q0, qs); });
+            if (a.lv[a.nl - 1].g.d.n() <= TAIL_ONE_BLOCK_COARSE) {
+                ok = phase(true, true, [&](long long, long long) { tail_coarse_block(a, C); });
+            } else {
+                ok = phase(false, true, [&](long long q0, long long qs) {
+                    for (long long c = q0; c < C.g.d.n(); c += qs) C.x[c] = 0.f;
+                });
+                for (int it = 0; it < a.coarse_sweeps && ok; ++it)
+                    for (int col = 0; col < 2 && ok; ++col)
+                        ok = phase(false, true, [&](long long q0, long long qs) { tail_coarse_colour(a, C, col, q0, qs); });
+            }
         } else {
             // G b as one FP64 matvec over every block's warps
             ok = phase(false, true, [&](long long, long long) { tail_direct(a, C); });
