@@ -22,7 +22,7 @@
 //    unmasked value) that are not on the domain boundary take a short path:
 //    no coefficient memory, no branches, a reciprocal instead of a divide.
 // Requires nx % 4 == 0 (16-byte rows); other levels use the per-colour path.
-#include "ff_device.cuh"
+#include "ff_stencil.cuh"
 #include <cudaTypedefs.h>
 #include <algorithm>
 
@@ -30,7 +30,7 @@ using namespace ffd;
 
 namespace {
 
-constexpr int TX = 32, TY = 16;   // tile (cells)
+constexpr int TX = BRICK_X, TY = BRICK_Y;   // tile (cells)
 constexpr int PX = TX / 2;        // threads per tile row (one x-pair each)
 constexpr int NT = PX * TY;       // 256 threads
 constexpr int BZ = 8;             // brick depth (bricks are TX x TY x BZ)
@@ -41,14 +41,6 @@ constexpr double MAX_ALPHA_MAGNITUDE = 1e6;
 constexpr double MAX_PAP_GROWTH_FACTOR = 1e8;
 constexpr double PAP_BASELINE_FLOOR = 1e-12;
 constexpr double MAX_RESIDUAL_GROWTH = 100.0;
-
-struct Geo {
-    Dims d;
-    float h2x, h2y, h2z;
-    float dreg;          // diagonal of a regular interior cell: -2(h2x+h2y+h2z)
-    long long sy, sz;
-    int bnx, bny;        // bricks per row / column
-};
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool valid) {
     unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -86,61 +78,6 @@ __device__ __forceinline__ bool brick_regular(const Geo &g, const uint8_t *brick
     if (!bricks) return false;
     int bz = k / BZ;
     return bricks[blockIdx.x + (long long)g.bnx * (blockIdx.y + (long long)g.bny * bz)] != 0;
-}
-
-struct Coef {
-    float kx, ky, kz, e, ux, uy, uz;
-};
-__device__ __forceinline__ Coef coef_at(const Geo &g, const float4 *coef, bool regular, int i, int j,
-                                        int k, long long c) {
-    Coef q;
-    if (regular) {
-        q.kx = i > 0 ? g.h2x : 0.f;
-        q.ky = j > 0 ? g.h2y : 0.f;
-        q.kz = k > 0 ? g.h2z : 0.f;
-        q.e = 0.f;
-        q.ux = i < g.d.nx - 1 ? g.h2x : 0.f;
-        q.uy = j < g.d.ny - 1 ? g.h2y : 0.f;
-        q.uz = k < g.d.nz - 1 ? g.h2z : 0.f;
-    } else {
-        float4 a = __ldg(coef + c);
-        q.kx = i > 0 ? a.x : 0.f;
-        q.ky = j > 0 ? a.y : 0.f;
-        q.kz = k > 0 ? a.z : 0.f;
-        q.e = a.w;
-        q.ux = i < g.d.nx - 1 ? __ldg(&coef[c + 1].x) : 0.f;
-        q.uy = j < g.d.ny - 1 ? __ldg(&coef[c + g.sy].y) : 0.f;
-        q.uz = k < g.d.nz - 1 ? __ldg(&coef[c + g.sz].z) : 0.f;
-    }
-    return q;
-}
-
-// (A v)_c, difference form; absent faces carry zero coefficients and their
-// staged neighbour values are zero-filled (finite).
-__device__ __forceinline__ float apply_q(const Coef &q, float vc, float xm, float xp, float ym, float yp,
-                                         float zm, float zp) {
-    float s = -q.e * vc;
-    s += q.kx * (xm - vc);
-    s += q.ux * (xp - vc);
-    s += q.ky * (ym - vc);
-    s += q.uy * (yp - vc);
-    s += q.kz * (zm - vc);
-    s += q.uz * (zp - vc);
-    return s;
-}
-__device__ __forceinline__ float diag_q(const Coef &q) {
-    return -(q.e + q.kx + q.ux + q.ky + q.uy + q.kz + q.uz);
-}
-// regular interior cell: second differences per axis
-__device__ __forceinline__ float apply_reg(const Geo &g, float vc, float xm, float xp, float ym, float yp,
-                                           float zm, float zp) {
-    float s = g.h2x * ((xm - vc) + (xp - vc));
-    s = __fmaf_rn(g.h2y, (ym - vc) + (yp - vc), s);
-    s = __fmaf_rn(g.h2z, (zm - vc) + (zp - vc), s);
-    return s;
-}
-__device__ __forceinline__ bool interior(const Geo &g, int i, int j, int k) {
-    return i > 0 && i < g.d.nx - 1 && j > 0 && j < g.d.ny - 1 && k > 0 && k < g.d.nz - 1;
 }
 
 // compensated (TwoSum) FP32 accumulation, folded into FP64 once
@@ -386,11 +323,6 @@ __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)_
 // writes are visible (a no-op for an ordinary launch).  Every such kernel
 // calls it before its first global-memory access.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ unsigned long long globaltimer_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
 __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
@@ -426,18 +358,6 @@ __device__ __forceinline__ void tma_load_3d(unsigned dst, const CUtensorMap *map
 }
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-// One relaxation of a cell with the plain couplings (class 0 or 2).  With
-// S the h^-2-weighted sum of the six neighbours (the tensor maps zero-fill
-// those across the domain edge, which drops the absent faces from S) and
-// d = dreg + corr the cell's diagonal (corr = h^-2 summed over the absent
-// faces), the row is (A v) = S + d v and the relaxation
-// v + sor (b - A v) / d = (1 - sor) v + (b - S) rd, rd = sor / d.
-__device__ __forceinline__ float relax_plain(const Geo &g, float omsor, float vc, float xm, float xp, float ym,
-                                             float yp, float zm, float zp, float bval, float rd) {
-    const float s = __fmaf_rn(g.h2z, zm + zp, __fmaf_rn(g.h2y, ym + yp, g.h2x * (xm + xp)));
-    return __fmaf_rn(bval - s, rd, omsor * vc);
 }
 
 // One relaxation by cell class (see SweepMaps), all in the form
@@ -1863,13 +1783,6 @@ constexpr size_t rr_smem() {
     return sizeof(float) * ((size_t)RXSLOTS * XPLANE + (size_t)RBSLOTS * BPLANE + (size_t)(TY + 2) * (TX + 2));
 }
 
-__device__ __forceinline__ void rtap4(int c, int nc, int *idx) {
-    idx[0] = c > 0 ? 2 * c - 1 : 2 * c;
-    idx[1] = 2 * c;
-    idx[2] = 2 * c + 1;
-    idx[3] = c + 1 < nc ? 2 * c + 2 : 2 * c + 1;
-}
-
 __global__ void __launch_bounds__(NT, 4) k_res_restrict(RrArgs a) {
     if (a.st && a.st->stop) return;
     extern __shared__ __align__(16) float dyn[];
@@ -2208,17 +2121,6 @@ __global__ void __launch_bounds__(256) k_restrict_yz4(Dims fd, Dims cd, int dims
 // of fine cells; along x the quad's four cells take (1/4, 3/4), (3/4, 1/4),
 // (1/4, 3/4), (3/4, 1/4) of the coarse cells 2q-1 .. 2q+2 (clamped), along
 // y and z the correctionTapsForAxis pair of its row and plane.
-__device__ __forceinline__ void ptaps2(int f, int nc, int *idx, float *w) {
-    const int ci = f >> 1;
-    if ((f & 1) == 0) {
-        idx[0] = ci > 0 ? ci - 1 : ci; w[0] = 0.25f;
-        idx[1] = ci; w[1] = 0.75f;
-    } else {
-        idx[0] = ci; w[0] = 0.75f;
-        idx[1] = ci < nc - 1 ? ci + 1 : ci; w[1] = 0.25f;
-    }
-}
-
 // Block (32, 8), grid (quads / 32, rows / 8, planes / PL): one quad per
 // thread on PL consecutive planes (2 in 3D: the planes 2c and 2c + 1 share
 // the coarse plane c, and each thread keeps two quads' loads in flight).
@@ -2283,610 +2185,6 @@ __global__ void __launch_bounds__(256) k_prolong4(Dims fd, Dims cd, int dims, co
     }
 }
 
-// ------------------------------------------------- coarse-level V-cycle --
-// The V-cycle below a level (its pre-smoothing, residual and restriction,
-// every coarser level, the direct coarsest solve, the prolongations and the
-// post-smoothing) in one cooperative launch: phases over all cells of one
-// level separated by grid-wide barriers.  Tail levels hold at most 2^18
-// cells (the host picks them so), so cell indices are 32-bit.  The coarse levels are too small
-// to fill the GPU, so one launch per sweep would cost more in launch and
-// pipeline latency than in work.  Colour passes run in place (a colour
-// reads only the other colour); the first pass on a level writes every cell,
-// the level starting from x = 0.  Values written inside the launch are read
-// through L2 (ld.global.cg), never from a possibly stale L1 line.  Per cell the arithmetic is that of the
-// level kernels: the TMA sweep's relaxation by class, k_resid_rx's residual
-// and x-taps followed by k_restrict_yz's y and z taps, k_coarse_direct's
-// row products, k_prolong4's correction.
-constexpr int TAIL_MAXL = 8;
-constexpr int TAIL_NT = 1024;
-// Levels up to this many cells run in one block (measured: a 64 x 64 level
-// gains, a 16^3 level, with its 64-tap restriction and 7-point colours,
-// loses against the grid barriers it saves).
-constexpr int TAIL_ONE_BLOCK_2D = 8192;
-constexpr int TAIL_ONE_BLOCK_3D = 512;
-// the coarsest level's sweeps (7-point colours, no restriction) in 2D and 3D
-constexpr int TAIL_ONE_BLOCK_COARSE = 8192;
-struct TailLevel {
-    Geo g;
-    float *x, *b, *r;              // r: residual scratch of the level
-    // block-0 levels held in shared memory: offset (floats) of the level's
-    // x, b and r there (n floats each), -1 for a level in global memory
-    int smo;
-    // t / hx, t / nx and t / ny as (t m) >> 40 with m = ceil(2^40 / divisor)
-    // (exact for every t below 2^22 and divisor below 2^18)
-    unsigned long long mhx, mnx, mny;
-    const float4 *coef, *gco;
-    const uint8_t *cls, *mask;     // class bytes (cpitch bytes per row), Dirichlet mask (may be null)
-    int cpitch;
-    float rdreg_sor;               // sor / dreg
-};
-struct TailArgs {
-    TailLevel lv[TAIL_MAXL];
-    int nl;                        // levels, the last one the coarsest
-    int down, up, dims;
-    float sor, omsor;
-    const double *G;               // coarsest inverse, nG x nG, row-major (direct mode)
-    int nG;
-    int coarse_sweeps;             // > 0: that many sweeps on the coarsest level instead of G b
-    PcgState *st;                  // may be null
-    unsigned *bar;                 // grid barrier: arrivals, generation, abort
-    int cxo;                       // the coarsest x's copy in shared memory (floats; -1: none)
-};
-
-// Grid-wide barrier of the cooperative launch over three words: a count of
-// arrivals that only grows within a launch (barrier k completes when it
-// reaches k x blocks), the number of blocks done with the launch (the last
-// one clears both counts, once no block polls them), and an abort flag.  A
-// block that waits more than 0.5 s raises the abort flag, which releases
-// every waiting block; all then return false.
-__device__ bool tail_sync(unsigned *bar, unsigned &passed) {
-    __shared__ int ok_s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        volatile unsigned *vb = bar;
-        if (vb[2]) {
-            ok = 0;
-        } else {
-            const unsigned target = (passed + 1) * gridDim.x;
-            __threadfence();
-            atomicAdd(&bar[0], 1u);
-            const unsigned long long t0 = globaltimer_ns();
-            while (vb[0] < target) {
-                if (vb[2]) { ok = 0; break; }
-                if (globaltimer_ns() - t0 > 500000000ull) {
-                    atomicExch(&bar[2], 1u);
-                    ok = 0;
-                    break;
-                }
-            }
-            __threadfence();
-        }
-        ok_s = ok;
-    }
-    __syncthreads();
-    ++passed;
-    return ok_s != 0;
-}
-
-// after a block's last barrier: the last block to get here clears the counts
-__device__ void tail_done(unsigned *bar) {
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(&bar[1], 1u) == gridDim.x - 1) {
-            atomicExch(&bar[0], 0u);
-            atomicExch(&bar[1], 0u);
-        }
-    }
-}
-
-__device__ __forceinline__ unsigned tail_class(const TailLevel &L, int i, int j, int k) {
-    return (__ldg(L.cls + L.cpitch * (j + L.g.d.ny * k) + (i >> 2)) >> (2 * (i & 3))) & 3u;
-}
-
-// the relaxation of one cell by class (the TMA sweep's arithmetic)
-__device__ __forceinline__ float tail_relax(const TailArgs &a, const TailLevel &L, unsigned cl, long long c, int i,
-                                           int j, int k, float vc, float xm, float xp, float ym, float yp, float zm,
-                                           float zp, float bval) {
-    const Geo &g = L.g;
-    if (!(cl & 1u)) {
-        const float corr = g.h2x * (float)((i == 0) + (i == g.d.nx - 1)) +
-                           g.h2y * (float)((j == 0) + (j == g.d.ny - 1)) +
-                           g.h2z * (float)((k == 0) + (k == g.d.nz - 1));
-        const float rd = corr == 0.f ? L.rdreg_sor : a.sor / (g.dreg + corr);
-        return relax_plain(g, a.omsor, vc, xm, xp, ym, yp, zm, zp, bval, rd);
-    }
-    if (cl == 1u) return __fmaf_rn(bval, -a.sor, a.omsor * vc);
-    const float4 lo = __ldg(L.coef + c), hi = __ldg(L.gco + c);
-    float s = lo.x * xm;
-    s = __fmaf_rn(hi.x, xp, s);
-    s = __fmaf_rn(lo.y, ym, s);
-    s = __fmaf_rn(hi.y, yp, s);
-    s = __fmaf_rn(lo.z, zm, s);
-    s = __fmaf_rn(hi.z, zp, s);
-    return __fmaf_rn(bval - s, a.sor * hi.w, a.omsor * vc);
-}
-
-// A 2D level of at most TAIL_SMEM_CELLS cells (and every coarser one but the
-// coarsest) lives in block 0's shared memory while the launch runs: block 0
-// alone runs its phases, so they need no grid barrier and no L2 round
-// trip.  Its b arrives there by the restriction into it (or, for the
-// launch's first level, by a copy from global memory) and its x leaves for
-// global memory after its last pass when the next finer level is a
-// grid-wide one.  SM: the level's arrays are there (plain loads); otherwise
-// loads bypass L1, which other blocks' writes in this launch leave stale.
-constexpr int TAIL_SMEM_CELLS = 8192;
-constexpr int TAIL_SMEM_BYTES = 3 * 4 * 8192 + 3 * 4 * 1024;   // 3 arrays of a 8192- and a 1024-cell level
-__device__ __forceinline__ int tdiv(int t, unsigned long long m) {
-    return (int)(((unsigned long long)(unsigned)t * m) >> 40);
-}
-template <bool SM>
-__device__ __forceinline__ float tld(const float *p) {
-    if constexpr (SM) return *p;
-    else return __ldcg(p);
-}
-struct TailArr {
-    float *x, *b, *r;
-};
-template <bool SM>
-__device__ __forceinline__ TailArr tail_arrays(const TailLevel &L) {
-    if constexpr (SM) {
-        extern __shared__ __align__(16) float tail_sm[];
-        const int n = (int)L.g.d.n();
-        float *x = tail_sm + L.smo;
-        return TailArr{x, x + n, x + 2 * n};
-    } else {
-        return TailArr{L.x, L.b, L.r};
-    }
-}
-
-// one colour pass (colour col = (i + j + k) & 1) in place, one thread per
-// cell of the colour (nx is even: nx / 2 of them per row); `first`: x is 0
-// on entry and the thread also writes 0 to the row neighbour of the other
-// colour
-template <bool SM>
-__device__ void tail_colour(const TailArgs &a, const TailLevel &L, int col, bool first, long long t0,
-                            long long stride) {
-    const Geo &g = L.g;
-    const int nx = g.d.nx, ny = g.d.ny, nz = g.d.nz, hx = nx >> 1;
-    const int n = hx * ny * nz;
-    const TailArr A = tail_arrays<SM>(L);
-    float *x = A.x;
-    for (int t = (int)t0; t < n; t += (int)stride) {
-        const int rr = tdiv(t, L.mhx);
-        const int m = t - rr * hx;
-        const int k = tdiv(rr, L.mny);
-        const int j = rr - k * ny;
-        const int par = (j + k + col) & 1;
-        const int i = 2 * m + par;
-        const int c = i + (int)g.sy * j + (int)g.sz * k;
-        float vc = 0.f, xm = 0.f, xp = 0.f, ym = 0.f, yp = 0.f, zm = 0.f, zp = 0.f;
-        if (first) {
-            x[c + (par ? -1 : 1)] = 0.f;
-        } else {
-            vc = tld<SM>(x + c);
-            if (i > 0) xm = tld<SM>(x + c - 1);
-            if (i < nx - 1) xp = tld<SM>(x + c + 1);
-            if (j > 0) ym = tld<SM>(x + c - g.sy);
-            if (j < ny - 1) yp = tld<SM>(x + c + g.sy);
-            if (k > 0) zm = tld<SM>(x + c - g.sz);
-            if (k < nz - 1) zp = tld<SM>(x + c + g.sz);
-        }
-        x[c] = tail_relax(a, L, tail_class(L, i, j, k), c, i, j, k, vc, xm, xp, ym, yp, zm, zp, tld<SM>(A.b + c));
-    }
-}
-
-// r = b - A x (0 on Dirichlet cells); xzero: x is taken as 0 and cleared
-template <bool SM>
-__device__ void tail_residual(const TailLevel &L, bool xzero, long long t0, long long stride) {
-    const Geo &g = L.g;
-    const int nx = g.d.nx, ny = g.d.ny, nz = g.d.nz;
-    const int n = nx * ny * nz;
-    const TailArr A = tail_arrays<SM>(L);
-    const float *x = A.x;
-    for (int c = (int)t0; c < n; c += (int)stride) {
-        const int rr = tdiv(c, L.mnx);
-        const int i = c - rr * nx;
-        const int k = tdiv(rr, L.mny);
-        const int j = rr - k * ny;
-        const unsigned cl = tail_class(L, i, j, k);
-        if (xzero) {
-            A.r[c] = cl == 1u ? 0.f : tld<SM>(A.b + c);
-            A.x[c] = 0.f;
-            continue;
-        }
-        const float vc = tld<SM>(x + c);
-        const float xm = i > 0 ? tld<SM>(x + c - 1) : vc, xp = i < nx - 1 ? tld<SM>(x + c + 1) : vc;
-        const float ym = j > 0 ? tld<SM>(x + c - g.sy) : vc, yp = j < ny - 1 ? tld<SM>(x + c + g.sy) : vc;
-        const float zm = k > 0 ? tld<SM>(x + c - g.sz) : vc, zp = k < nz - 1 ? tld<SM>(x + c + g.sz) : vc;
-        A.r[c] = resid_cls(g, L.coef, cl, i, j, k, tld<SM>(A.b + c), vc, xm, xp, ym, yp, zm, zp);
-    }
-}
-
-// coarse b = R r (the 1/8, 3/8, 3/8, 1/8 taps per axis), 0 on coarse
-// Dirichlet cells; relax0: also the coarse level's first colour-0 pass
-// (from x = 0 a cell needs only its own b; colour-1 cells get 0)
-template <bool FSM, bool CSM>
-__device__ void tail_restrict(const TailArgs &a, const TailLevel &F, const TailLevel &C, bool relax0, long long t0,
-                              long long stride) {
-    const Dims fd = F.g.d, cd = C.g.d;
-    const TailArr FA = tail_arrays<FSM>(F), CA = tail_arrays<CSM>(C);
-    const int n = cd.nx * cd.ny * cd.nz;
-    const float w4[4] = {0.125f, 0.375f, 0.375f, 0.125f};
-    for (int c = (int)t0; c < n; c += (int)stride) {
-        const int rr = tdiv(c, C.mnx);
-        const int I = c - rr * cd.nx;
-        const int K = tdiv(rr, C.mny);
-        const int J = rr - K * cd.ny;
-        if (C.mask && __ldg(C.mask + c)) {
-            CA.b[c] = 0.f;
-            if (relax0)
-                CA.x[c] = ((I + J + K) & 1) ? 0.f
-                                           : tail_relax(a, C, tail_class(C, I, J, K), c, I, J, K, 0.f, 0.f, 0.f, 0.f,
-                                                        0.f, 0.f, 0.f, 0.f);
-            continue;
-        }
-        int ix[4], jy[4], kz[4];
-        rtap4(I, cd.nx, ix);
-        rtap4(J, cd.ny, jy);
-        int nzt = 4;
-        if (a.dims == 3) rtap4(K, cd.nz, kz);
-        else { kz[0] = K; nzt = 1; }
-        float s = 0.f;
-        for (int q = 0; q < nzt; ++q) {
-            const float wz = a.dims == 3 ? w4[q] : 1.0f;
-            float part = 0.f;
-#pragma unroll
-            for (int p = 0; p < 4; ++p) {
-                const float *row = FA.r + fd.nx * (jy[p] + fd.ny * kz[q]);
-                const float rx = 0.125f * tld<FSM>(row + ix[0]) + 0.375f * tld<FSM>(row + ix[1]) +
-                                 0.375f * tld<FSM>(row + ix[2]) + 0.125f * tld<FSM>(row + ix[3]);
-                part += rx * w4[p];
-            }
-            s += part * wz;
-        }
-        CA.b[c] = s;
-        if (relax0)
-            CA.x[c] = ((I + J + K) & 1) ? 0.f
-                                       : tail_relax(a, C, tail_class(C, I, J, K), c, I, J, K, 0.f, 0.f, 0.f, 0.f, 0.f,
-                                                    0.f, 0.f, s);
-    }
-}
-
-// coarsest x = G b, one warp per row (FP64)
-__device__ void tail_direct(const TailArgs &a, const TailLevel &C) {
-    const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    for (long long row = warp; row < a.nG; row += nwarps) {
-        const double *gr = a.G + row * a.nG;
-        double s = 0.0;
-        for (int j = lane; j < a.nG; j += 32) s += __ldg(gr + j) * (double)__ldcg(C.b + j);
-        s = warp_sum(s);
-        if (lane == 0) C.x[row] = (float)s;
-    }
-}
-
-// fine x += P coarse x, skipped on fine Dirichlet cells
-template <bool CSM, bool FSM>
-__device__ void tail_prolong(const TailArgs &a, const TailLevel &C, const TailLevel &F, long long t0,
-                             long long stride) {
-    const Dims fd = F.g.d, cd = C.g.d;
-    const TailArr CA = tail_arrays<CSM>(C), FA = tail_arrays<FSM>(F);
-    const int n = fd.nx * fd.ny * fd.nz;
-    for (int c = (int)t0; c < n; c += (int)stride) {
-        if (F.mask && __ldg(F.mask + c)) continue;
-        const int rr = tdiv(c, F.mnx);
-        const int i = c - rr * fd.nx;
-        const int k = tdiv(rr, F.mny);
-        const int j = rr - k * fd.ny;
-        int ii[2], jj[2], kk[2];
-        float wi[2], wj[2], wk[2];
-        ptaps2(i, cd.nx, ii, wi);
-        ptaps2(j, cd.ny, jj, wj);
-        int nk = 2;
-        if (a.dims == 3) ptaps2(k, cd.nz, kk, wk);
-        else { kk[0] = 0; wk[0] = 1.f; nk = 1; }
-        float acc = 0.f;
-        for (int b = 0; b < 2; ++b)
-            for (int q = 0; q < nk; ++q) {
-                const float *row = CA.x + cd.nx * (jj[b] + cd.ny * kk[q]);
-                const float w = wj[b] * wk[q];
-                acc += (wi[0] * tld<CSM>(row + ii[0]) + wi[1] * tld<CSM>(row + ii[1])) * w;
-            }
-        FA.x[c] = tld<FSM>(FA.x + c) + acc;
-    }
-}
-
-// one colour pass on the coarsest level from the stored coefficients
-// (k_coarse_sweeps' arithmetic: x += sor (b - A x) / diag)
-__device__ void tail_coarse_colour(const TailArgs &a, const TailLevel &C, int col, long long t0, long long stride) {
-    const Dims d = C.g.d;
-    const int sy = d.nx, sz = d.nx * d.ny, n = (int)d.n();
-    float *x = C.x;
-    for (int c = (int)t0; c < n; c += (int)stride) {
-        const int rr = tdiv(c, C.mnx);
-        const int i = c - rr * d.nx;
-        const int k = tdiv(rr, C.mny);
-        const int j = rr - k * d.ny;
-        if (((i + j + k) & 1) != col) continue;
-        const float xc = __ldcg(x + c);
-        const float4 kc = __ldg(C.coef + c);
-        float s = -kc.w * xc;
-        float D = -(kc.w + kc.x + kc.y + kc.z);
-        if (i > 0) s += kc.x * (__ldcg(x + c - 1) - xc);
-        if (i < d.nx - 1) { const float k1 = __ldg(&C.coef[c + 1].x); s += k1 * (__ldcg(x + c + 1) - xc); D -= k1; }
-        if (j > 0) s += kc.y * (__ldcg(x + c - sy) - xc);
-        if (j < d.ny - 1) { const float k1 = __ldg(&C.coef[c + sy].y); s += k1 * (__ldcg(x + c + sy) - xc); D -= k1; }
-        if (k > 0) s += kc.z * (__ldcg(x + c - sz) - xc);
-        if (k < d.nz - 1) { const float k1 = __ldg(&C.coef[c + sz].z); s += k1 * (__ldcg(x + c + sz) - xc); D -= k1; }
-        x[c] = xc + ((__ldcg(C.b + c) - s) / D) * a.sor;
-    }
-}
-
-// All sweeps of a coarsest level of up to TAIL_ONE_BLOCK_COARSE cells in block
-// 0, x in shared memory from the first pass to the last (through L2 a colour
-// pass is two dependent round trips, about 1 us; 40 passes made up most of a
-// small hierarchy's V-cycle).  A cell's operator as the passes use it: the six
-// couplings (0 across the domain edge, where the neighbour index is the cell
-// itself), E, the diagonal and b.
-struct CoarseCell {
-    float k[6], e, D, b;
-    int c, n[6];
-};
-__device__ __forceinline__ CoarseCell coarse_cell(const TailLevel &C, int i, int j, int k) {
-    const Dims d = C.g.d;
-    const int sy = d.nx, sz = d.nx * d.ny;
-    CoarseCell q;
-    q.c = i + sy * j + sz * k;
-    const float4 kc = __ldg(C.coef + q.c);
-    q.e = kc.w;
-    q.D = -(kc.w + kc.x + kc.y + kc.z);
-    const bool in[6] = {i > 0, i < d.nx - 1, j > 0, j < d.ny - 1, k > 0, k < d.nz - 1};
-    const int st[3] = {1, sy, sz};
-#pragma unroll
-    for (int f = 0; f < 6; ++f) {
-        const int a = f >> 1;
-        q.n[f] = in[f] ? q.c + (f & 1 ? st[a] : -st[a]) : q.c;
-        float kf = 0.f;
-        if (in[f]) {
-            const int cc = f & 1 ? q.n[f] : q.c;
-            kf = a == 0 ? __ldg(&C.coef[cc].x) : (a == 1 ? __ldg(&C.coef[cc].y) : __ldg(&C.coef[cc].z));
-            if (f & 1) q.D -= kf;
-        }
-        q.k[f] = kf;
-    }
-    q.b = __ldcg(C.b + q.c);
-    return q;
-}
-__device__ __forceinline__ void coarse_relax(const CoarseCell &q, float *x, float sor) {
-    const float xc = x[q.c];
-    float s = -q.e * xc;
-#pragma unroll
-    for (int f = 0; f < 6; ++f) s += q.k[f] * (x[q.n[f]] - xc);
-    x[q.c] = xc + ((q.b - s) / q.D) * sor;
-}
-__device__ __forceinline__ void bar_sync_n(int id, int threads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-__device__ void tail_coarse_block(const TailArgs &a, const TailLevel &C) {
-    __shared__ float x[TAIL_ONE_BLOCK_COARSE];
-    const Dims d = C.g.d;
-    const int n = (int)d.n(), hx = (d.nx + 1) >> 1, pairs = hx * d.ny * d.nz, tid = threadIdx.x;
-    for (int c = tid; c < n; c += TAIL_NT) x[c] = 0.f;
-    __syncthreads();
-    // cell of colour col of a pair (two neighbours of a row, one of each colour)
-    auto cell_of = [&](int t, int col, int &i, int &j, int &k) {
-        const int r = t / hx;
-        k = r / d.ny;
-        j = r - k * d.ny;
-        i = 2 * (t - r * hx) + ((j + k + col) & 1);
-        return i < d.nx;
-    };
-    if (pairs <= TAIL_NT) {
-        // one pair a thread, its operator in registers; only the warps with
-        // pairs take part in the passes' barriers
-        const int nthr = (pairs + 31) & ~31;
-        if (tid < nthr) {
-            CoarseCell q[2];
-            bool has[2] = {false, false};
-#pragma unroll
-            for (int col = 0; col < 2; ++col) {
-                int i, j, k;
-                if (tid < pairs && cell_of(tid, col, i, j, k)) {
-                    q[col] = coarse_cell(C, i, j, k);
-                    has[col] = true;
-                }
-            }
-            for (int it = 0; it < a.coarse_sweeps; ++it) {
-#pragma unroll
-                for (int col = 0; col < 2; ++col) {
-                    if (has[col]) coarse_relax(q[col], x, a.sor);
-                    bar_sync_n(1, nthr);
-                }
-            }
-        }
-    } else {
-        for (int it = 0; it < 2 * a.coarse_sweeps; ++it) {
-            for (int t = tid; t < pairs; t += TAIL_NT) {
-                int i, j, k;
-                if (cell_of(t, it & 1, i, j, k)) coarse_relax(coarse_cell(C, i, j, k), x, a.sor);
-            }
-            __syncthreads();
-        }
-    }
-    __syncthreads();
-    for (int c = tid; c < n; c += TAIL_NT) C.x[c] = x[c];
-}
-
-// HELD: some levels are held in block 0's shared memory (the instance
-// without them carries none of their dispatch)
-template <bool HELD>
-__global__ void __launch_bounds__(TAIL_NT, 1) k_vcycle_tail(TailArgs a) {
-    PcgState *st = a.st;
-    if (st && (st->stop || st->err)) return;
-    unsigned *bar = a.bar;
-    unsigned passed = 0;
-    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    // A phase over a level of at most one_block cells, or held in block 0's
-    // shared memory, runs in block 0 alone, with a block barrier after it; a
-    // phase over a larger level runs on every block with a grid barrier
-    // after it, and one more grid barrier first when block-0 phases precede
-    // it.  Every block takes the same sequence of grid barriers (the choice
-    // depends only on level sizes).
-    bool solo_prev = false;
-    const int one_block = a.dims == 3 ? TAIL_ONE_BLOCK_3D : TAIL_ONE_BLOCK_2D;
-    auto held = [&](int l) { return HELD && a.lv[l].smo >= 0; };
-    auto small = [&](int l) { return held(l) || a.lv[l].g.d.n() <= one_block; };
-    auto phase = [&](bool solo, bool sync_after, auto &&work) -> bool {
-        if (solo) {
-            if (blockIdx.x == 0) {
-                work((long long)threadIdx.x, (long long)blockDim.x);
-                __syncthreads();
-            }
-            solo_prev = true;
-            return true;
-        }
-        if (solo_prev) {
-            solo_prev = false;
-            if (!tail_sync(bar, passed)) return false;
-        }
-        work(t0, stride);
-        return sync_after ? tail_sync(bar, passed) : true;
-    };
-    // a held level's x to global memory, or its b and x from there (block 0)
-    auto copy_x_out = [&](int l) {
-        if constexpr (!HELD) return;
-        const TailArr A = tail_arrays<true>(a.lv[l]);
-        const int n = (int)a.lv[l].g.d.n();
-        for (int c = threadIdx.x; c < n; c += blockDim.x) a.lv[l].x[c] = A.x[c];
-    };
-    auto copy_in = [&](int l) {
-        if constexpr (!HELD) return;
-        const TailArr A = tail_arrays<true>(a.lv[l]);
-        const int n = (int)a.lv[l].g.d.n();
-        for (int c = threadIdx.x; c < n; c += blockDim.x) {
-            A.b[c] = __ldcg(a.lv[l].b + c);
-            A.x[c] = __ldcg(a.lv[l].x + c);
-        }
-    };
-    bool ok = true;
-    if (held(0))
-        ok = phase(true, true, [&](long long q0, long long qs) {
-            const TailArr A = tail_arrays<true>(a.lv[0]);
-            for (long long c = q0; c < a.lv[0].g.d.n(); c += qs) A.b[c] = __ldcg(a.lv[0].b + c);
-        });
-    // the coarse level's first colour-0 pass rides on the restriction into it
-    // (not into the coarsest level, which is solved directly or swept)
-    for (int l = 0; l < a.nl - 1 && ok; ++l) {
-        const TailLevel &L = a.lv[l];
-        const bool fused0 = l > 0 && a.down > 0, sl = small(l), hl = held(l);
-        for (int it = 0; it < a.down && ok; ++it) {
-            if (!(fused0 && it == 0))
-                ok = phase(sl, true, [&](long long q0, long long qs) {
-                    if (hl) tail_colour<true>(a, L, 0, it == 0, q0, qs);
-                    else tail_colour<false>(a, L, 0, it == 0, q0, qs);
-                });
-            if (ok) ok = phase(sl, true, [&](long long q0, long long qs) {
-                if (hl) tail_colour<true>(a, L, 1, false, q0, qs);
-                else tail_colour<false>(a, L, 1, false, q0, qs);
-            });
-        }
-        if (!ok) break;
-        ok = phase(sl, true, [&](long long q0, long long qs) {
-            if (hl) tail_residual<true>(L, a.down == 0, q0, qs);
-            else tail_residual<false>(L, a.down == 0, q0, qs);
-        });
-        if (!ok) break;
-        // the restriction runs over the coarse level's cells; into a held
-        // level from a grid-wide one it runs grid-wide into the level's global
-        // arrays, which block 0 then takes into shared memory
-        const bool relax0 = l + 1 < a.nl - 1 && a.down > 0, hc = held(l + 1);
-        if (!HELD) {
-            ok = phase(small(l + 1), true, [&](long long q0, long long qs) {
-                tail_restrict<false, false>(a, L, a.lv[l + 1], relax0, q0, qs);
-            });
-        } else if (hc && !hl) {
-            ok = phase(false, true, [&](long long q0, long long qs) {
-                tail_restrict<false, false>(a, L, a.lv[l + 1], relax0, q0, qs);
-            });
-            if (ok) ok = phase(true, true, [&](long long, long long) { copy_in(l + 1); });
-        } else {
-            ok = phase(small(l + 1), true, [&](long long q0, long long qs) {
-                if (hl && hc) tail_restrict<true, true>(a, L, a.lv[l + 1], relax0, q0, qs);
-                else if (hl) tail_restrict<true, false>(a, L, a.lv[l + 1], relax0, q0, qs);
-                else tail_restrict<false, false>(a, L, a.lv[l + 1], relax0, q0, qs);
-            });
-        }
-    }
-    if (ok) {
-        const TailLevel &C = a.lv[a.nl - 1];
-        if (a.coarse_sweeps > 0) {
-            if (a.lv[a.nl - 1].g.d.n() <= TAIL_ONE_BLOCK_COARSE) {
-                ok = phase(true, true, [&](long long, long long) { tail_coarse_block(a, C); });
-            } else {
-                ok = phase(false, true, [&](long long q0, long long qs) {
-                    for (long long c = q0; c < C.g.d.n(); c += qs) C.x[c] = 0.f;
-                });
-                for (int it = 0; it < a.coarse_sweeps && ok; ++it)
-                    for (int col = 0; col < 2 && ok; ++col)
-                        ok = phase(false, true, [&](long long q0, long long qs) { tail_coarse_colour(a, C, col, q0, qs); });
-            }
-        } else {
-            // G b as one FP64 matvec over every block's warps
-            ok = phase(false, true, [&](long long, long long) { tail_direct(a, C); });
-        }
-    }
-    for (int l = a.nl - 2; l >= 0 && ok; --l) {
-        const TailLevel &L = a.lv[l];
-        const bool sl = small(l), hl = held(l);
-        // a held coarse level is read from shared memory only by a held fine
-        // level's phase (block 0); a grid-wide phase reads its global copy
-        const bool hc = hl && held(l + 1);
-        const bool out = hl && (l == 0 || !held(l - 1));
-        ok = phase(sl, true, [&](long long q0, long long qs) {
-            if (hl && hc) {
-                tail_prolong<true, true>(a, a.lv[l + 1], L, q0, qs);
-            } else if (hl && l + 1 == a.nl - 1 && a.cxo >= 0) {
-                // the coarsest x (global, written grid-wide) into shared memory first
-                extern __shared__ __align__(16) float tail_sm[];
-                const TailLevel &C = a.lv[l + 1];
-                for (long long c = q0; c < C.g.d.n(); c += qs) tail_sm[a.cxo + c] = __ldcg(C.x + c);
-                __syncthreads();
-                TailLevel Cs = C;
-                Cs.smo = a.cxo;
-                tail_prolong<true, true>(a, Cs, L, q0, qs);
-            } else if (hl) {
-                tail_prolong<false, true>(a, a.lv[l + 1], L, q0, qs);
-            } else {
-                tail_prolong<false, false>(a, a.lv[l + 1], L, q0, qs);
-            }
-            if (out && a.up == 0) {
-                __syncthreads();
-                copy_x_out(l);
-            }
-        });
-        for (int it = 0; it < a.up && ok; ++it) {
-            ok = phase(sl, true, [&](long long q0, long long qs) {
-                if (hl) tail_colour<true>(a, L, 1, false, q0, qs);
-                else tail_colour<false>(a, L, 1, false, q0, qs);
-            });
-            // the kernel's end orders the last pass before the next launch
-            if (ok) ok = phase(sl, !(l == 0 && it == a.up - 1), [&](long long q0, long long qs) {
-                if (hl) tail_colour<true>(a, L, 0, false, q0, qs);
-                else tail_colour<false>(a, L, 0, false, q0, qs);
-                if (out && it == a.up - 1) {
-                    __syncthreads();
-                    copy_x_out(l);
-                }
-            });
-        }
-    }
-    if (ok) tail_done(bar);
-    else if (threadIdx.x == 0 && st) atomicOr(&st->err, 2);
-}
-
 // ----------------------------------------------------------- cell classes --
 // Two bits per cell, one byte per x-quad (rows `pitch` bytes apart): 0 an
 // interior cell whose six couplings are the plain h^-2 and E = 0; 1 a
@@ -2903,12 +2201,12 @@ __global__ void k_coef_classes(Geo g, int dims, const float *__restrict__ wu, co
                                float hz2, float4 *__restrict__ coef, uint2 *__restrict__ coef16,
                                uint8_t *__restrict__ cls, int pitch, float4 *__restrict__ gco) {
     // one thread per cell (coalesced coefficient stores); the four lanes of
-    // an x-quad (nx % 4 == 0, blockDim.x a multiple of 32) merge their
-    // classes into the quad's byte with shuffles
+    // an x-quad (blockDim.x is a multiple of 32) merge their classes into the
+    // quad's byte with shuffles, cells past the row's end as class 0
     const Dims d = g.d;
     const int ir = blockIdx.x * blockDim.x + threadIdx.x;
     const int jr = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    const bool in = ir < d.nx && jr < d.ny;   // whole quads are in or out
+    const bool in = ir < d.nx && jr < d.ny;
     const int i = in ? ir : 0, j = in ? jr : 0;
     auto W = [](const float *w, long long f) { return w ? w[f] : 1.f; };
     auto P = [&](long long n) { return mask ? mask[n] != 0 : false; };
@@ -2936,7 +2234,7 @@ __global__ void k_coef_classes(Geo g, int dims, const float *__restrict__ wu, co
     const bool pinned = e == 1.f && kx == 0.f && ky == 0.f && kz == 0.f && ux == 0.f && uy == 0.f && uz == 0.f;
     const bool inner = i > 0 && i < d.nx - 1 && j > 0 && j < d.ny - 1 && k > 0 && k < d.nz - 1;
     const unsigned cl = plain ? (inner ? 0u : 2u) : (pinned ? 1u : 3u);
-    unsigned byte = cl << (2 * (ir & 3));
+    unsigned byte = in ? cl << (2 * (ir & 3)) : 0u;
     byte |= __shfl_xor_sync(0xffffffffu, byte, 1);
     byte |= __shfl_xor_sync(0xffffffffu, byte, 2);
     if (!in) return;
@@ -3063,20 +2361,6 @@ __global__ void k_brick_flags(Geo g, const float4 *coef, uint8_t *bricks) {
     }
     ok = __syncthreads_and(ok);
     if (threadIdx.x == 0) bricks[bx + (long long)g.bnx * (by + (long long)g.bny * bz)] = (uint8_t)ok;
-}
-
-Geo make_geo(const Level &L) {
-    Geo g;
-    g.d = L.d;
-    g.h2x = L.h2inv[0];
-    g.h2y = L.h2inv[1];
-    g.h2z = L.d.nz > 1 ? L.h2inv[2] : 0.f;
-    g.dreg = -2.f * (g.h2x + g.h2y + g.h2z);
-    g.sy = L.d.nx;
-    g.sz = (long long)L.d.nx * L.d.ny;
-    g.bnx = (L.d.nx + TX - 1) / TX;
-    g.bny = (L.d.ny + TY - 1) / TY;
-    return g;
 }
 
 int zchunk(const Dims &d, int sm_count, int blocks_per_sm) {
@@ -3266,7 +2550,7 @@ static int encode_planes(CUtensorMap *m, const float *base, const Dims &d, int r
     return FF_OK;
 }
 
-static int cls_pitch(const Dims &d) { return ((d.nx / 4 + 15) / 16) * 16; }
+static int cls_pitch(const Dims &d) { return (((d.nx + 3) / 4 + 15) / 16) * 16; }
 
 size_t sweep_tma_cls_bytes(const Dims &d) { return (size_t)cls_pitch(d) * d.ny * d.nz; }
 
@@ -3316,7 +2600,6 @@ int coef_classes(const Level &L, const SweepMaps &m, uint8_t *bricks, int dims, 
     // 128 cells) x rows
     const int bx = std::min(128, (L.d.nx + 31) / 32 * 32), by = 256 / bx;
     dim3 grid((L.d.nx + bx - 1) / bx, (L.d.ny + by - 1) / by, L.d.nz);
-    FF_CHECK(L.d.nx % 4 == 0, FF_E_STATE, "cell classes need nx %% 4 == 0");
     k_coef_classes<<<grid, dim3(bx, by), 0, s>>>(g, dims, L.w[0], L.w[1], L.w[2], L.mask, L.h2inv[0], L.h2inv[1],
                                                   L.h2inv[2], L.coef, want16 ? L.coef16 : nullptr, m.cls_ptr,
                                                   m.cls_pitch, m.gco);
@@ -3572,93 +2855,5 @@ int x_residual_tma(const Level &L0, const SweepMaps &sm, const CgMaps &m, float 
 
 
 size_t cls_row_pitch(const Dims &d) { return (size_t)cls_pitch(d); }
-
-int vcycle_tail(const Level *lv, const SweepMaps *sm, int nl, int dims, int down, int up, float sor,
-                const double *G, int nG, int coarse_sweeps, PcgState *st, unsigned *bar, int sm_count,
-                cudaStream_t s) {
-    FF_CHECK(nl >= 2 && nl <= TAIL_MAXL, FF_E_ARG, "coarse V-cycle: %d levels (2..%d)", nl, TAIL_MAXL);
-    FF_CHECK(bar, FF_E_ARG, "coarse V-cycle: no barrier words");
-    FF_CHECK(coarse_sweeps > 0 || (G && nG == lv[nl - 1].d.n()), FF_E_STATE, "coarse V-cycle: no coarsest inverse");
-    TailArgs a;
-    for (int l = 0; l < nl; ++l) {
-        TailLevel &t = a.lv[l];
-        const Level &L = lv[l];
-        t.g = make_geo(L);
-        t.x = (float *)L.x;
-        t.b = (float *)L.b;
-        t.r = (float *)L.buf;
-        t.coef = L.coef;
-        t.mask = L.mask;
-        t.rdreg_sor = sor / t.g.dreg;
-        t.smo = -1;
-        auto magic = [](long long d) { return ((1ULL << 40) + (unsigned long long)d - 1) / (unsigned long long)d; };
-        t.mhx = magic(std::max(1, L.d.nx / 2));
-        t.mnx = magic(L.d.nx);
-        t.mny = magic(L.d.ny);
-        if (l < nl - 1) {
-            FF_CHECK(sm[l].cls_ptr && sm[l].gco && L.buf, FF_E_STATE, "coarse V-cycle: level %d lacks classes", l);
-            t.cls = sm[l].cls_ptr;
-            t.cpitch = sm[l].cls_pitch;
-            t.gco = sm[l].gco;
-        } else {
-            t.cls = nullptr;
-            t.cpitch = 0;
-            t.gco = nullptr;
-        }
-    }
-    a.nl = nl;
-    a.down = down;
-    a.up = up;
-    a.dims = dims;
-    a.sor = sor;
-    a.omsor = 1.f - sor;
-    a.G = G;
-    a.nG = nG;
-    a.coarse_sweeps = coarse_sweeps;
-    a.st = st;
-    a.bar = bar;
-    // levels held in block 0's shared memory (2D): from the last but one
-    // upward while they have at most TAIL_SMEM_CELLS cells and fit the budget
-    // (and, beside the last but one, a copy of the coarsest x).  In 3D the
-    // 16^3 level held there made the 256^3 V-cycle slower (0.587 -> 0.596
-    // ms: its block-0 phases cost more than the grid barriers they saved), so
-    // 3D levels stay grid-wide.
-    int smem = 0;
-    const long long nc = lv[nl - 1].d.n();
-    for (int l = nl - 2; l >= 0 && dims == 2; --l) {
-        const long long n = lv[l].d.n();
-        if (n > TAIL_SMEM_CELLS || smem + 12 * n + (l == nl - 2 ? 4 * nc : 0) > TAIL_SMEM_BYTES) break;
-        a.lv[l].smo = smem / 4;
-        smem += (int)(12 * n);
-    }
-    a.cxo = -1;
-    if (a.lv[nl - 2].smo >= 0) {
-        a.cxo = smem / 4;
-        smem += (int)(4 * nc);
-    }
-    static int per_sm = -1, per_sm_held = -1;
-    if (per_sm < 0) {
-        FF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_vcycle_tail<false>, TAIL_NT, 0));
-        FF_CUDA(cudaFuncSetAttribute(k_vcycle_tail<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     TAIL_SMEM_BYTES));
-        FF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_held, k_vcycle_tail<true>, TAIL_NT,
-                                                              TAIL_SMEM_BYTES));
-    }
-    FF_CHECK(per_sm >= 1 && per_sm_held >= 1 && smem <= TAIL_SMEM_BYTES, FF_E_CUDA,
-             "coarse V-cycle kernel does not fit an SM");
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)sm_count);
-    cfg.blockDim = dim3(TAIL_NT);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (smem > 0) FF_CUDA(cudaLaunchKernelEx(&cfg, k_vcycle_tail<true>, a));
-    else FF_CUDA(cudaLaunchKernelEx(&cfg, k_vcycle_tail<false>, a));
-    return post("vcycle_tail");
-}
 
 }  // namespace ffk

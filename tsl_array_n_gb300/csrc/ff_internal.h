@@ -246,11 +246,20 @@ int coef_classes(const Level &L, const SweepMaps &m, uint8_t *bricks, int dims, 
 size_t cls_row_pitch(const Dims &d);
 // the V-cycle from level lv[0] down to the coarsest lv[nl-1] and back, one
 // cooperative launch (coarse_sweeps > 0: sweeps instead of G b at the bottom)
-// bar: three words (arrivals, generation, abort), zero before the first
+// bar: three words (arrivals, blocks done, abort), zero before the first
 // launch and after a failed one; st may be null (no stop or error flags)
 int vcycle_tail(const Level *lv, const SweepMaps *sm, int nl, int dims, int down, int up, float sor,
                 const double *G, int nG, int coarse_sweeps, PcgState *st, unsigned *bar, int sm_count,
                 cudaStream_t s);
+// a whole PCG solve (after k_state_init) in one cooperative launch, for
+// hierarchies of at most 12 levels with classes on all but the coarsest
+// and at least one sweep before and after the correction; levels' x and b as in
+// the V-cycle (lv[0]: z and r); partials: 8 sums of sm_count doubles
+constexpr long long PCG_RESIDENT_CELLS = 1LL << 20;
+int pcg_resident(const Level *lv, const SweepMaps *sm, int nl, int dims, int down, int up, int fin, float sor,
+                 const double *G, int nG, int coarse_sweeps, const float *b, float *p0, float *p1, float *xh0, float *xl0,
+                 float *xh1, float *xl1, int ds, PcgState *st, double *partials, unsigned *bar, int sm_count,
+                 cudaStream_t s);
 int cg_tma_maps(const Level &L0, const float *z0, const float *z1, const float *p0, const float *p1,
                 const float *xh0, const float *xl0, const float *xh1, const float *xl1, const float *b, bool ds,
                 CgMaps &m);
