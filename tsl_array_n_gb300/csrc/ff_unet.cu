@@ -59,13 +59,6 @@ __host__ __device__ __forceinline__ long long g8(long long v, int c, long long n
     return ((long long)(c >> 3) * n + v) * 8 + (c & 7);
 }
 
-// offset of tap t (0..26) in (dz, dy, dx) = (t/9 - 1, (t/3)%3 - 1, t%3 - 1)
-__device__ __forceinline__ void tap_offset(int t, int &dx, int &dy, int &dz) {
-    dz = t / 9 - 1;
-    dy = (t / 3) % 3 - 1;
-    dx = t % 3 - 1;
-}
-
 // ---- tcgen05 helpers -----------------------------------------------------
 // 3x3x3 convolutions, zero padding 1: Y[v, co] = act(sum_{t, ci} X[v + off(t),
 // ci] W[t, ci, co] + bias[co]), as implicit GEMMs on the 5th-generation
@@ -92,11 +85,10 @@ __device__ __forceinline__ uint64_t tc_sdesc(uint32_t addr, uint32_t lbo, uint32
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo & 0x3FFFFu) >> 4) << 16) |
            ((uint64_t)((sbo & 0x3FFFFu) >> 4) << 32) | (1ull << 46);
 }
-// instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, K-major
-// (or, mn_major, both MN-major: bits 15 and 16), N >> 3 at bit 17, M >> 4 at bit 24
-__host__ __device__ constexpr uint32_t tc_idesc(int m, int n, bool mn_major = false) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (mn_major ? (3u << 15) : 0u) | ((uint32_t)(n >> 3) << 17) |
-           ((uint32_t)(m >> 4) << 24);
+// instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, K-major,
+// N >> 3 at bit 17, M >> 4 at bit 24
+__host__ __device__ constexpr uint32_t tc_idesc(int m, int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 __device__ __forceinline__ void mbar_init(uint32_t bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
@@ -465,156 +457,145 @@ __global__ void __launch_bounds__(ZM_THREADS) k_conv3_zm(const __grid_constant__
     }
 }
 
-// weight gradient on tcgen05: dW[t, ci, co] += sum_v X[v + off(t), ci] G[v, co]
-// over a chunk of WG_VC voxels; block = (chunk, tap).  The GEMM runs
-// transposed, D[co][ci] = sum_v G[v][co] X[v + off(t)][ci]: M = Cout padded
-// to 128 (columns past Cout stay zero), N = Cin, K = the chunk's voxels in
-// stages of 64.  Both operands are MN-major in the canonical no-swizzle
-// layout: a core matrix is 8 K-rows (voxels) of 16 bytes (8 consecutive
-// channels), i.e. rows of the 8-channel group planes copied as they are; core matrices 128
-// bytes apart along K (LBO) and 1 KB apart along M / N (SBO).  The
-// accumulators are added to dW with FP32 atomics (order-dependent in the
-// last bits).
-constexpr int WG_KC = 64, WG_VC = 1024, WG_MAXQ = 10;   // rows per thread: 64 (Cin + Cout) / 8 / 128
+// Weight and bias gradients: dW[t, ci, co] += sum_v X[v + off(t), ci] G[v, co],
+// db[co] += sum_v G[v, co], as 27 small GEMMs over K = voxels with M = 16 MT
+// input channels and N = 8 NTL output channels.  With 16 to 64 channels on either
+// side a tcgen05 tile (M = 128) would be three quarters padding or more, and its
+// shared-memory reads are those of the padded tile: 32 clocks for one tap's 16
+// voxels, against 4 for the operands themselves.  So this contraction runs on
+// mma.sync (m16n8k16, FP32 accumulators in registers for a whole column).
+//
+// A block marches along z with an 8 x 16 tile: planes of X (tile and halo, 10 x
+// 18 voxels) in a ring of four slots and planes of G in two, by cp.async one plane
+// ahead.  Warp w holds the three dx taps of (dy, dz) = (w % 3, w / 3) - 1: the
+// halo'd plane is read as it is, a tap being a shift of the ldmatrix rows (16
+// bytes a voxel and 8-channel group; both operands have voxels as rows, so both
+// are transposed on the way).  Voxels outside the domain are zero in X and G.
+// The bias rides along as a tap whose A is all ones.  The sums of a column are
+// added to dW with FP32 atomics (order-dependent in the last bits).
+// 128^3, one launch: 16 -> 16 channels 116 us, 48 -> 16 291 us, all ten 0.96 ms,
+// against 9.9 ms for tcgen05 tiles of one tap and 1024 voxels a block (each tap
+// read both operands again) and 0.79 ms of bias passes.  Bound by the issue of
+// mma.sync: 19 clocks for one m16n8k16 and quarter of an SM.
+namespace wg {
+constexpr int TX = 16, TY = 8, HX = TX + 2, HY = TY + 2, HV = HX * HY, TV = TX * TY;
+constexpr int XSLOTS = 4, GSLOTS = 2, NT = 288;
+}  // namespace wg
 
-__global__ void __launch_bounds__(128) k_conv3_wgrad_tc(Vol v, const bf16 *__restrict__ X, int cin,
-                                                       const bf16 *__restrict__ G, int cout, float *__restrict__ dW,
-                                                       int *__restrict__ err) {
-    extern __shared__ unsigned char tc_smem[];
-    __shared__ __align__(8) uint64_t bars[2];
-    __shared__ uint32_t tmem_slot;
-    const int tcols = cin <= 32 ? 32 : (cin <= 64 ? 64 : 128);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int a_bytes = TC_M * WG_KC * 2, b_bytes = cin * WG_KC * 2;
-    const int stage_bytes = (a_bytes + b_bytes + 1023) & ~1023;
-    const uint32_t raw = smem_u32(tc_smem);
-    unsigned char *stages = tc_smem + (((raw + 1023u) & ~1023u) - raw);
-    const uint32_t bar0 = smem_u32(&bars[0]), bar1 = smem_u32(&bars[1]);
-    // A rows at or past Cout are never written below: zero both stages' A once
-    for (int q = tid; q < a_bytes / 16; q += TC_M) {
-        reinterpret_cast<uint4 *>(stages)[q] = make_uint4(0, 0, 0, 0);
-        reinterpret_cast<uint4 *>(stages + stage_bytes)[q] = make_uint4(0, 0, 0, 0);
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(tcols));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-        asm volatile("tcgen05.fence::before_thread_sync;");
-    }
-    if (tid == 0) {
-        mbar_init(bar0, 1);
-        mbar_init(bar1, 1);
-    }
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = tmem_slot;
-    const int t = blockIdx.y;
-    int dx, dy, dz;
-    tap_offset(t, dx, dy, dz);
-    const long long nvox = v.n();
-    const long long vbeg = (long long)blockIdx.x * WG_VC;
-    const int nst = (int)std::min<long long>(WG_VC / WG_KC, (nvox - vbeg + WG_KC - 1) / WG_KC);
-    const uint32_t idesc = tc_idesc(TC_M, cin, true);
-    constexpr uint32_t SBO = (WG_KC / 8) * 128;   // 8-channel groups along M or N
-    const int gco = cout >> 3, gci = cin >> 3;
-    // a stage is 64 (Cout / 8) A rows then 64 (Cin / 8) B rows of 16 bytes;
-    // thread tid moves rows tid + 128 j (the A/B boundary is a multiple of
-    // 128, so row j is A or B for the whole block).  The next stage's rows
-    // are loaded into registers while the current stage's MMAs run.
-    const int na = WG_KC * gco, nrows = WG_KC * (gco + gci), nq = nrows / TC_M;
-    uint4 pre[WG_MAXQ];
-    auto fetch = [&](int sidx) {
-        const long long k0 = vbeg + (long long)sidx * WG_KC;
+__device__ __forceinline__ void cp16(uint32_t dst, const void *src, bool valid) {
+    const int sz = valid ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(sz) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                 "{%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <int MT, int NTL>
+__global__ void __launch_bounds__(wg::NT, MT * NTL <= 6 ? 2 : 1) k_conv3_wgrad(Vol v, const bf16 *__restrict__ X, int cin,
+                                                        const bf16 *__restrict__ G, float *__restrict__ dW,
+                                                        float *__restrict__ db, int gx, int zc) {
+    using namespace wg;
+    constexpr int XG = 2 * MT, GG = NTL, COUT = 8 * NTL;   // 8-channel groups of X (this slice) and G
+    constexpr uint32_t XPL = XG * HV * 16, GPL = GG * TV * 16;
+    extern __shared__ __align__(128) unsigned char wsm[];
+    const uint32_t xs = smem_u32(wsm), gs = xs + XSLOTS * XPL;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int x0 = (int)(blockIdx.x % gx) * TX, y0 = (int)(blockIdx.x / gx) * TY;
+    const int k0 = (int)blockIdx.y * zc, k1 = min(k0 + zc, v.nz), c0 = (int)blockIdx.z * 16 * MT;
+    const long long nvox = v.n(), pl = (long long)v.nx * v.ny;
+    const bf16 *Xc = X + (long long)(c0 >> 3) * nvox * 8;
+    auto load_x = [&](int k) {
+        const uint32_t dst = xs + (uint32_t)((k - k0 + 1) & (XSLOTS - 1)) * XPL;
+        const bool zin = k >= 0 && k < v.nz;
+        for (int q = tid; q < XG * HV; q += NT) {
+            const int g = q / HV, r = q - g * HV, hy = r / HX, hx = r - hy * HX;
+            const int x = x0 - 1 + hx, y = y0 - 1 + hy;
+            const bool in = zin && x >= 0 && x < v.nx && y >= 0 && y < v.ny;
+            cp16(dst + 16u * q, in ? Xc + (g * nvox + k * pl + (long long)y * v.nx + x) * 8 : X, in);
+        }
+    };
+    auto load_g = [&](int k) {
+        const uint32_t dst = gs + (uint32_t)((k - k0) & (GSLOTS - 1)) * GPL;
+        for (int q = tid; q < GG * TV; q += NT) {
+            const int g = q / TV, r = q % TV, x = x0 + r % TX, y = y0 + r / TX;
+            const bool in = x < v.nx && y < v.ny;
+            cp16(dst + 16u * q, in ? G + (g * nvox + k * pl + (long long)y * v.nx + x) * 8 : G, in);
+        }
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    load_x(k0 - 1);
+    load_x(k0);
+    load_x(k0 + 1);
+    load_g(k0);
+    commit();
+    const int dyi = warp % 3, dzi = warp / 3;
+    const bool bias = warp == 4 && c0 == 0;   // (dy, dz) = (0, 0)
+    float acc[3][MT][NTL][4] = {}, accb[NTL][4] = {};
+    // this lane's ldmatrix rows: X rows are voxels (8 by lane & 7, 8 more by
+    // bit 4), the matrix by bit 3 the channel group; G the other way round
+    const uint32_t xoff = 16u * (((lane >> 3) & 1) * HV + dyi * HX + 8 * (lane >> 4) + (lane & 7));
+    const uint32_t goff = 16u * ((lane >> 4) * TV + 8 * ((lane >> 3) & 1) + (lane & 7));
+    const uint32_t ones[4] = {0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u};
+    for (int k = k0; k < k1; ++k) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();   // the planes of this step are in; the last step's slots are free
+        if (k + 1 < k1) {
+            load_x(k + 2);
+            load_g(k + 1);
+        }
+        commit();
+        const uint32_t xa = xs + (uint32_t)((k + dzi - k0) & (XSLOTS - 1)) * XPL + xoff;
+        const uint32_t ga = gs + (uint32_t)((k - k0) & (GSLOTS - 1)) * GPL + goff;
+#pragma unroll 2
+        for (int y = 0; y < TY; ++y) {
+            uint32_t bq[NTL / 2][4];
 #pragma unroll
-        for (int j = 0; j < WG_MAXQ; ++j) {
-            if (j >= nq) break;
-            const int q = tid + TC_M * j;
-            const bool isa = q < na;
-            const int qq = isa ? q : q - na;
-            const int r = qq % WG_KC, cg = qq / WG_KC;
-            const long long vv = k0 + r;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (vv < nvox) {
-                if (isa) {
-                    val = __ldg(reinterpret_cast<const uint4 *>(G + g8(vv, 8 * cg, nvox)));
-                } else {
-                    const int x = (int)(vv % v.nx), y = (int)((vv / v.nx) % v.ny),
-                              z = (int)(vv / ((long long)v.nx * v.ny));
-                    const int sx = x + dx, sy = y + dy, sz = z + dz;
-                    if (sx >= 0 && sx < v.nx && sy >= 0 && sy < v.ny && sz >= 0 && sz < v.nz)
-                        val = __ldg(reinterpret_cast<const uint4 *>(
-                            X + g8(sx + (long long)v.nx * (sy + (long long)v.ny * sz), 8 * cg, nvox)));
+            for (int n = 0; n < NTL / 2; ++n) ldsm4t(ga + 16u * (y * TX + 2 * n * TV), bq[n]);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    uint32_t aq[4];
+                    ldsm4t(xa + 16u * (y * HX + d + 2 * m * HV), aq);
+#pragma unroll
+                    for (int n = 0; n < NTL; ++n)
+                        mma16816(acc[d][m][n], aq, bq[n / 2][2 * (n & 1)], bq[n / 2][2 * (n & 1) + 1]);
                 }
             }
-            pre[j] = val;
-        }
-    };
-    // row (cg, r) of A or B: one 16-byte row of core matrix (cg, r / 8)
-    auto put = [&](unsigned char *stg) {
-        uint4 *A = reinterpret_cast<uint4 *>(stg), *B = reinterpret_cast<uint4 *>(stg + a_bytes);
+            if (bias)
 #pragma unroll
-        for (int j = 0; j < WG_MAXQ; ++j) {
-            if (j >= nq) break;
-            const int q = tid + TC_M * j;
-            const bool isa = q < na;
-            const int qq = isa ? q : q - na;
-            const int r = qq % WG_KC, cg = qq / WG_KC;
-            (isa ? A : B)[(cg * (WG_KC / 8) + (r >> 3)) * 8 + (r & 7)] = pre[j];
+                for (int n = 0; n < NTL; ++n) mma16816(accb[n], ones, bq[n / 2][2 * (n & 1)], bq[n / 2][2 * (n & 1) + 1]);
         }
-    };
-    bool ok = true;
-    int last = -1;
-    fetch(0);
-    for (int sidx = 0; sidx < nst; ++sidx) {
-        const int st = sidx & 1;
-        unsigned char *stg = stages + st * stage_bytes;
-        // the stage's previous MMAs (stage sidx - 2) must be done before it is overwritten
-        if (sidx >= 2) ok = mbar_wait(st ? bar1 : bar0, (uint32_t)(((sidx >> 1) - 1) & 1));
-        if (!__syncthreads_and(ok)) {
-            ok = false;
-            break;
-        }
-        put(stg);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;");
-            const uint32_t a0 = smem_u32(stg), b0 = a0 + (uint32_t)a_bytes;
-#pragma unroll
-            for (int kc = 0; kc < WG_KC / 16; ++kc)
-                tc_mma(tmem, tc_sdesc(a0 + 256u * kc, 128u, SBO), tc_sdesc(b0 + 256u * kc, 128u, SBO), idesc,
-                       (sidx > 0 || kc > 0) ? 1 : 0);
-            tc_commit(st ? bar1 : bar0);
-        }
-        last = sidx;
-        if (sidx + 1 < nst) fetch(sidx + 1);
     }
-    if (last >= 0) {
-        const bool done = mbar_wait((last & 1) ? bar1 : bar0, (uint32_t)((last >> 1) & 1));
-        ok = ok && done;
-    }
-    ok = __syncthreads_and(ok);
-    if (ok && last >= 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const int co = warp * 32 + lane;
-        const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int c0 = 0; c0 < cin; c0 += 16) {
-            float acc[16];
-            tc_ld16(lane_addr + (uint32_t)c0, acc);
-            if (co < cout) {
+    const int row = lane >> 2, col = 2 * (lane & 3);
 #pragma unroll
-                for (int q = 0; q < 16; ++q) atomicAdd(dW + ((long long)t * cin + c0 + q) * cout + co, acc[q]);
+    for (int d = 0; d < 3; ++d) {
+        const int t = 9 * dzi + 3 * dyi + d;
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int n = 0; n < NTL; ++n) {
+                float *w = dW + ((long long)t * cin + c0 + 16 * m + row) * COUT + 8 * n + col;
+                atomicAdd(w, acc[d][m][n][0]);
+                atomicAdd(w + 1, acc[d][m][n][1]);
+                atomicAdd(w + 8 * COUT, acc[d][m][n][2]);
+                atomicAdd(w + 8 * COUT + 1, acc[d][m][n][3]);
             }
+    }
+    if (bias && row == 0)
+#pragma unroll
+        for (int n = 0; n < NTL; ++n) {
+            atomicAdd(db + 8 * n + col, accb[n][0]);
+            atomicAdd(db + 8 * n + col + 1, accb[n][1]);
         }
-    } else if (!ok && tid == 0) {
-        atomicExch(err, 1);
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    if (warp == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tcols));
-    }
 }
 
 // G = dY * gelu'(Z) in BF16 (the GEMM operand of both backward convolutions),
@@ -637,16 +618,36 @@ __global__ void k_act_grad(long long nvox, int C, const float *__restrict__ dY, 
     }
 }
 
-// bias gradient: db[c] += sum_v G[v, c] (G in 8-channel group planes: the
-// flat index i runs over group planes, channel (i / (8 nvox)) 8 + i % 8)
-__global__ void k_bias_grad(long long nvox, int C, const bf16 *__restrict__ G, float *__restrict__ db) {
-    extern __shared__ float sb[];
-    for (int c = threadIdx.x; c < C; c += blockDim.x) sb[c] = 0.f;
-    __syncthreads();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvox * C; i += (long long)gridDim.x * blockDim.x)
-        atomicAdd(&sb[(int)(i / (8 * nvox)) * 8 + (int)(i & 7)], __bfloat162float(G[i]));
-    __syncthreads();
-    for (int c = threadIdx.x; c < C; c += blockDim.x) atomicAdd(&db[c], sb[c]);
+// k_act_grad for an encoder's skip tensor, whose gradient has two parts: the
+// pooled path's (dP / 8 of the coarse voxel) and the concatenation's (the last C
+// of the C1 + C channels of dcat)
+__global__ void __launch_bounds__(256) k_skip_act_grad(Vol f, int C, int C1, const float *__restrict__ dP,
+                                                       const float *__restrict__ dcat, const float *__restrict__ Z,
+                                                       bf16 *__restrict__ G) {
+    const int ng = C >> 3, cx = f.nx / 2, cy = f.ny / 2;
+    const long long nvox = f.n();
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvox * ng;
+         i += (long long)gridDim.x * blockDim.x) {
+        const long long v = i / ng;
+        const int g = (int)(i - v * ng);
+        const int x = (int)(v % f.nx);
+        const long long yz = v / f.nx;
+        const int y = (int)(yz % f.ny), z = (int)(yz / f.ny);
+        const long long cv = (x / 2) + (long long)cx * ((y / 2) + (long long)cy * (z / 2));
+        const float4 *p = reinterpret_cast<const float4 *>(dP + cv * C + 8 * g);
+        const float4 *d = reinterpret_cast<const float4 *>(dcat + v * (C1 + C) + C1 + 8 * g);
+        const float4 *q = reinterpret_cast<const float4 *>(Z + v * C + 8 * g);
+        __align__(16) bf16 o[8];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float4 a = __ldg(p + h), b = __ldg(d + h), c = __ldg(q + h);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w}, zv[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                o[4 * h + k] = __float2bfloat16_rn(__fadd_rn(__fmul_rn(av[k], 0.125f), bv[k]) * gelu_grad(zv[k]));
+        }
+        *reinterpret_cast<uint4 *>(G + g8(v, 8 * g, nvox)) = *reinterpret_cast<const uint4 *>(o);
+    }
 }
 
 // W'[t', co, ci] = W[26 - t', ci, co]: the input-gradient convolution's
@@ -710,20 +711,6 @@ __global__ void k_pool(Vol c, int C, const bf16 *__restrict__ X, bf16 *__restric
         *reinterpret_cast<uint4 *>(Y + g8(vv, 8 * g, nc)) = *reinterpret_cast<const uint4 *>(o);
     }
 }
-__global__ void k_pool_grad(Vol c, int C, const float *__restrict__ dY, float *__restrict__ dX, int accumulate) {
-    const long long n = c.n() * C;
-    const int fx = 2 * c.nx, fy = 2 * c.ny;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const long long vv = i / C;
-        const int ch = (int)(i % C);
-        const int x = (int)(vv % c.nx), y = (int)((vv / c.nx) % c.ny), z = (int)(vv / ((long long)c.nx * c.ny));
-        const float g = dY[i] * 0.125f;
-        for (int q = 0; q < 8; ++q) {
-            const long long f = (2 * x + (q & 1)) + (long long)fx * ((2 * y + ((q >> 1) & 1)) + (long long)fy * (2 * z + (q >> 2)));
-            dX[f * C + ch] = (accumulate ? dX[f * C + ch] : 0.f) + g;
-        }
-    }
-}
 
 // nearest 2x upsampling of X (C1 channels) into the first C1 / 8 group
 // planes of the concat buffer Y; the skip tensor's planes follow them in
@@ -743,8 +730,7 @@ __global__ void k_up_concat(Vol f, int C1, const bf16 *__restrict__ X, bf16 *__r
         *reinterpret_cast<uint4 *>(Y + g8(vv, 8 * g, nf)) = __ldg(reinterpret_cast<const uint4 *>(X + g8(cv, 8 * g, nc)));
     }
 }
-// backward of k_up_concat: dX (coarse, C1) = sum over the 8 children, and
-// the skip part added into dS (C2)
+// backward of k_up_concat: dX (coarse, C1) = sum over the 8 children
 __global__ void k_up_concat_grad(Vol c, int C1, int C2, const float *__restrict__ dY, float *__restrict__ dX) {
     const int C = C1 + C2;
     const long long n = c.n() * C1;
@@ -759,14 +745,6 @@ __global__ void k_up_concat_grad(Vol c, int C1, int C2, const float *__restrict_
             s += dY[f * C + ch];
         }
         dX[i] = s;
-    }
-}
-__global__ void k_skip_grad_add(long long nvox, int C1, int C2, const float *__restrict__ dY, float *__restrict__ dS) {
-    const int C = C1 + C2;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvox * C2; i += (long long)gridDim.x * blockDim.x) {
-        const long long vv = i / C2;
-        const int ch = (int)(i % C2);
-        dS[i] += dY[vv * C + C1 + ch];
     }
 }
 
@@ -846,22 +824,42 @@ __global__ void k_loss_grad(Vol v, const float *__restrict__ e, float *__restric
         d_to_draw[i] = (2.0f * d_to_draw[i] + 2.0f * LAP_W * graph_lap(e, v, x, y, z, i)) * inv;
     }
 }
-// head backward: dY[v, c] = draw[v] w[c]; dw[c] += sum draw y; db += sum draw
-__global__ void k_head_grad(long long n, const float *__restrict__ Zin, const float *__restrict__ w,
-                            const float *__restrict__ draw, float *__restrict__ dY, float *__restrict__ dw) {
+// head backward: dw[c] += sum_v draw[v] y[v, c], db += sum_v draw[v], and the last
+// convolution's pre-activation gradient G = bf16(draw w[c] gelu'(Z)) (dL/dy is
+// not stored: the two passes over 134 MB at 128^3 that wrote and read it back,
+// and scalar strided loads, took 300 + 64 us; this takes 45).  One
+// thread per voxel and 8-channel group, so lanes of one parity share a group.
+__global__ void __launch_bounds__(256) k_head_grad(long long n, const float *__restrict__ Z, const float *__restrict__ w,
+                                                   const float *__restrict__ draw, bf16 *__restrict__ G,
+                                                   float *__restrict__ dw) {
     __shared__ float sw[17];
     if (threadIdx.x < 17) sw[threadIdx.x] = 0.f;
     __syncthreads();
-    float lw[17] = {};
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
-        const float g = draw[v];
-        for (int c = 0; c < 16; ++c) {
-            dY[v * 16 + c] = g * w[c];
-            lw[c] += g * gelu(Zin[v * 16 + c]);
+    const int g = threadIdx.x & 1;   // blockDim.x and the stride are even
+    float wc[8], lw[9] = {};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) wc[k] = __ldg(w + 8 * g + k);
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 2 * n; i += (long long)gridDim.x * blockDim.x) {
+        const long long v = i >> 1;
+        const float d = __ldg(draw + v);
+        const float4 za = __ldg(reinterpret_cast<const float4 *>(Z + v * 16 + 8 * g));
+        const float4 zb = __ldg(reinterpret_cast<const float4 *>(Z + v * 16 + 8 * g) + 1);
+        const float z[8] = {za.x, za.y, za.z, za.w, zb.x, zb.y, zb.z, zb.w};
+        __align__(16) bf16 o[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            lw[k] += d * gelu(z[k]);
+            o[k] = __float2bfloat16_rn(d * wc[k] * gelu_grad(z[k]));
         }
-        lw[16] += g;
+        lw[8] += d;
+        *reinterpret_cast<uint4 *>(G + g8(v, 8 * g, n)) = *reinterpret_cast<const uint4 *>(o);
     }
-    for (int c = 0; c < 17; ++c) atomicAdd(&sw[c], lw[c]);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+#pragma unroll
+        for (int m = 2; m < 32; m <<= 1) lw[k] += __shfl_xor_sync(0xffffffffu, lw[k], m);
+        if ((threadIdx.x & 31) < (k < 8 ? 2 : 1)) atomicAdd(&sw[k < 8 ? 8 * g + k : 16], lw[k]);
+    }
     __syncthreads();
     if (threadIdx.x < 17) atomicAdd(&dw[threadIdx.x], sw[threadIdx.x]);
 }
@@ -1107,20 +1105,39 @@ int launch_conv(int cout, Vol v, const bf16 *X, int cin, const bf16 *W, const fl
     }
 }
 
-int launch_wgrad(int cin, int cout, Vol v, const bf16 *X, const bf16 *G, float *dW, int *err, cudaStream_t s) {
-    if (cin % 16 || cin > 96 || cout % 16 || cout > TC_M || WG_KC * (cin + cout) / 8 > TC_M * WG_MAXQ)
-        return ff_set_error(FF_E_ARG, "unet: no weight-gradient kernel for %d -> %d", cin, cout);
-    // two stages of (128 x 64 A + cin x 64 B) BF16, 1 KB aligned, + alignment slack
-    const int stage = (TC_M * WG_KC * 2 + cin * WG_KC * 2 + 1023) & ~1023;
-    const int smem = 2 * stage + 1024;
-    static int configured = 0;
-    if (smem > configured) {
-        FF_CUDA(cudaFuncSetAttribute(k_conv3_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        configured = smem;
+template <int MT, int NTL>
+int launch_wgrad_t(int cin, Vol v, const bf16 *X, const bf16 *G, float *dW, float *db, cudaStream_t s) {
+    constexpr int smem = 16 * (wg::XSLOTS * 2 * MT * wg::HV + wg::GSLOTS * NTL * wg::TV);
+    FF_CUDA(cudaFuncSetAttribute(k_conv3_wgrad<MT, NTL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const int gx = (v.nx + wg::TX - 1) / wg::TX, gy = (v.ny + wg::TY - 1) / wg::TY, slices = cin / (16 * MT);
+    static int per_sm = 0;
+    if (!per_sm)
+        FF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv3_wgrad<MT, NTL>, wg::NT, smem));
+    // the z-segments of a column (each reads two planes more) that take the
+    // fewest plane steps over the waves they need
+    const long long cols = (long long)gx * gy * slices, slots = (long long)std::max(1, per_sm) * sm_count();
+    int zc = v.nz;
+    long long best = -1;
+    for (int segs = 1; segs <= v.nz; ++segs) {
+        const int z = (v.nz + segs - 1) / segs;
+        const long long n = cols * ((v.nz + z - 1) / z), cost = (n + slots - 1) / slots * (z + 2);
+        if (best < 0 || cost < best) best = cost, zc = z;
+        if (n > 4 * slots) break;
     }
-    dim3 grid((unsigned)((v.n() + WG_VC - 1) / WG_VC), 27);
-    k_conv3_wgrad_tc<<<grid, TC_M, smem, s>>>(v, X, cin, G, cout, dW, err);
-    return post("conv3 wgrad tcgen05");
+    dim3 grid((unsigned)(gx * gy), (unsigned)((v.nz + zc - 1) / zc), (unsigned)slices);
+    k_conv3_wgrad<MT, NTL><<<grid, wg::NT, smem, s>>>(v, X, cin, G, dW, db, gx, zc);
+    return post("conv3 wgrad");
+}
+// input channels a block holds: with 32 output channels 16 (two blocks an SM of
+// 48 accumulators a thread beat one of 96), else as many as keep the
+// accumulators (12 MT NTL a thread) below 100 registers
+int launch_wgrad(int cin, int cout, Vol v, const bf16 *X, const bf16 *G, float *dW, float *db, cudaStream_t s) {
+    if (cout == 16 && cin % 48 == 0) return launch_wgrad_t<3, 2>(cin, v, X, G, dW, db, s);
+    if (cout == 16 && cin % 32 == 0) return launch_wgrad_t<2, 2>(cin, v, X, G, dW, db, s);
+    if (cout == 16 && cin % 16 == 0) return launch_wgrad_t<1, 2>(cin, v, X, G, dW, db, s);
+    if (cout == 32 && cin % 16 == 0) return launch_wgrad_t<1, 4>(cin, v, X, G, dW, db, s);
+    if (cout == 64 && cin % 16 == 0) return launch_wgrad_t<1, 8>(cin, v, X, G, dW, db, s);
+    return ff_set_error(FF_E_ARG, "unet: no weight-gradient kernel for %d -> %d", cin, cout);
 }
 
 // deterministic Gaussian initialisation: mulberry32 + Box-Muller
@@ -1228,8 +1245,10 @@ static int ensure_shape(ff_unet u, Vol v, bool train) {
         long long maxc = 0;
         for (int s = 0; s < 15; ++s) {
             const long long nv = n0 >> (3 * SLOT_LEVEL[s]);
-            FF_TRY(alloc_owned(u, (void **)&u->grad[s], (size_t)nv * SLOT_C[s] * sizeof(float)));
             maxc = std::max(maxc, nv * SLOT_C[s]);
+            // the input's, the skip tensors' and the last convolution's are never stored
+            if (s == 0 || s == 2 || s == 5 || s == 14) continue;
+            FF_TRY(alloc_owned(u, (void **)&u->grad[s], (size_t)nv * SLOT_C[s] * sizeof(float)));
         }
         u->pre.resize(10);
         for (int l = 0; l < 10; ++l) {
@@ -1404,61 +1423,75 @@ static int forward(ff_unet u, const float *b, const uint8_t *mask, const float *
     return post("unet forward");
 }
 
-// gradient of conv l: input gradient into grad[CONV_IN[l]] (unless l == 0),
-// weight and bias gradients; grad[CONV_OUT[l]] holds dL/d(output)
-static int conv_backward(ff_unet u, int l, bool accumulate_input) {
+// dL/d(pre-activation) of conv l into gbuf, from dL/d(output) in grad[CONV_OUT[l]]
+static int act_backward(ff_unet u, int l) {
+    const ConvLayer &c = u->convs[l];
+    const int so = CONV_OUT[l];
+    const Vol v = level_vol(u, SLOT_LEVEL[so]);
+    k_act_grad<<<gblocks(v.n() * c.cout / 8), 256, 0, u->ctx->stream>>>(v.n(), c.cout, u->grad[so], u->pre[l], c.act,
+                                                                        u->gbuf);
+    return post("act grad");
+}
+// the same for the skip tensor conv l writes: grad[pool] holds the gradient of
+// the pooled tensor, grad[cat] that of the concatenation (c1 channels before it)
+static int skip_backward(ff_unet u, int l, int pool, int cat, int c1) {
+    const ConvLayer &c = u->convs[l];
+    const Vol v = level_vol(u, SLOT_LEVEL[CONV_OUT[l]]);
+    k_skip_act_grad<<<gblocks(v.n() * c.cout / 8), 256, 0, u->ctx->stream>>>(v, c.cout, c1, u->grad[pool], u->grad[cat],
+                                                                             u->pre[l], u->gbuf);
+    return post("skip act grad");
+}
+
+// gradient of conv l from its pre-activation's in gbuf: input gradient into
+// grad[CONV_IN[l]] (unless l == 0), weight and bias gradients
+static int conv_backward(ff_unet u, int l) {
     cudaStream_t s = u->ctx->stream;
     const ConvLayer &c = u->convs[l];
     const int si = CONV_IN[l], so = CONV_OUT[l];
     const Vol v = level_vol(u, SLOT_LEVEL[so]);
-    const long long nout = v.n() * c.cout;
-    k_act_grad<<<gblocks(nout / 8), 256, 0, s>>>(v.n(), c.cout, u->grad[so], u->pre[l], c.act, u->gbuf);
-    FF_TRY(post("act grad"));
     if (c.cin == c.cin_real) {
-        FF_TRY(launch_wgrad(c.cin, c.cout, v, u->act[si], u->gbuf, u->g + c.w_off, u->tc_err, s));
+        FF_TRY(launch_wgrad(c.cin, c.cout, v, u->act[si], u->gbuf, u->g + c.w_off, u->g + c.b_off, s));
     } else {
         // padded input channels: accumulate over all 16, keep the real ones
         FF_CUDA(cudaMemsetAsync(u->g0, 0, 27LL * c.cin * c.cout * 4, s));
-        FF_TRY(launch_wgrad(c.cin, c.cout, v, u->act[si], u->gbuf, u->g0, u->tc_err, s));
+        FF_TRY(launch_wgrad(c.cin, c.cout, v, u->act[si], u->gbuf, u->g0, u->g + c.b_off, s));
         k_gather_rows<<<gblocks(27LL * c.cin_real * c.cout), 256, 0, s>>>(c.cin_real, c.cin, c.cout, u->g0,
                                                                           u->g + c.w_off);
     }
-    k_bias_grad<<<std::min(gblocks(nout), 1024), 256, c.cout * 4, s>>>(v.n(), c.cout, u->gbuf, u->g + c.b_off);
-    FF_TRY(post("bias grad"));
     if (l == 0) return FF_OK;
     k_flip_transpose<<<gblocks(27LL * c.cin * c.cout), 256, 0, s>>>(c.cin_real, c.cin, c.cout, u->w + c.w_off, u->wt);
     // dX = conv(G, W') with cin = cout_fwd, cout = cin_fwd; written as FP32
     // through the pre-activation output of the conv kernel
-    float *dst = u->grad[si];
-    if (accumulate_input) return ff_set_error(FF_E_STATE, "unet: accumulate not supported");
-    FF_TRY(launch_conv(c.cin, v, u->gbuf, c.cout, u->wt, nullptr, 0, dst, nullptr, u->wpk, u->tc_err, s));
+    FF_TRY(launch_conv(c.cin, v, u->gbuf, c.cout, u->wt, nullptr, 0, u->grad[si], nullptr, u->wpk, u->tc_err, s));
     return FF_OK;
 }
 
 static int backward(ff_unet u) {
     cudaStream_t s = u->ctx->stream;
     const long long n0 = u->vol.n();
-    k_head_grad<<<std::min(gblocks(n0), 1024), 256, 0, s>>>(n0, u->pre[9], u->w + u->head_off, u->draw, u->grad[14],
-                                                             u->g + u->head_off);
+    auto conv = [&](int l) {
+        FF_TRY(act_backward(u, l));
+        return conv_backward(u, l);
+    };
+    k_head_grad<<<std::min(gblocks(2 * n0), 152 * 8), 256, 0, s>>>(n0, u->pre[9], u->w + u->head_off, u->draw, u->gbuf,
+                                                                   u->g + u->head_off);
     FF_TRY(post("head grad"));
-    FF_TRY(conv_backward(u, 9, false));   // grad[13]
-    FF_TRY(conv_backward(u, 8, false));   // grad[12] (cat0: 32 up + 16 skip)
+    FF_TRY(conv_backward(u, 9));   // grad[13]
+    FF_TRY(conv(8));               // grad[12] (cat0: 32 up + 16 skip)
     const Vol v1 = level_vol(u, 1), v2 = level_vol(u, 2);
     k_up_concat_grad<<<gblocks(v1.n() * 32), 256, 0, s>>>(v1, 32, 16, u->grad[12], u->grad[11]);
-    FF_TRY(conv_backward(u, 7, false));   // grad[10]
-    FF_TRY(conv_backward(u, 6, false));   // grad[9] (cat1: 64 up + 32 skip)
+    FF_TRY(conv(7));               // grad[10]
+    FF_TRY(conv(6));               // grad[9] (cat1: 64 up + 32 skip)
     k_up_concat_grad<<<gblocks(v2.n() * 64), 256, 0, s>>>(v2, 64, 32, u->grad[9], u->grad[8]);
-    FF_TRY(conv_backward(u, 5, false));   // grad[7]
-    FF_TRY(conv_backward(u, 4, false));   // grad[6]
-    // skip1 (slot 5) gets the pooled path and the concat path
-    k_pool_grad<<<gblocks(v2.n() * 32), 256, 0, s>>>(v2, 32, u->grad[6], u->grad[5], 0);
-    k_skip_grad_add<<<gblocks(v1.n() * 32), 256, 0, s>>>(v1.n(), 64, 32, u->grad[9], u->grad[5]);
-    FF_TRY(conv_backward(u, 3, false));   // grad[4]
-    FF_TRY(conv_backward(u, 2, false));   // grad[3]
-    k_pool_grad<<<gblocks(v1.n() * 16), 256, 0, s>>>(v1, 16, u->grad[3], u->grad[2], 0);
-    k_skip_grad_add<<<gblocks(n0 * 16), 256, 0, s>>>(n0, 32, 16, u->grad[12], u->grad[2]);
-    FF_TRY(conv_backward(u, 1, false));   // grad[1]
-    FF_TRY(conv_backward(u, 0, false));
+    FF_TRY(conv(5));               // grad[7]
+    FF_TRY(conv(4));               // grad[6]
+    // the skip tensors (slots 5 and 2) get the pooled path and the concat path
+    FF_TRY(skip_backward(u, 3, 6, 9, 64));
+    FF_TRY(conv_backward(u, 3));   // grad[4]
+    FF_TRY(conv(2));               // grad[3]
+    FF_TRY(skip_backward(u, 1, 3, 12, 32));
+    FF_TRY(conv_backward(u, 1));   // grad[1]
+    FF_TRY(conv(0));
     return post("unet backward");
 }
 
