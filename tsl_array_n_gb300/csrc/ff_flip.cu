@@ -37,12 +37,13 @@ __device__ __forceinline__ long long cell_of(const G3 &g, const float *p) {
 // particles of a one-cell-thick grid standing in for a 2D one stay on their
 // plane (the trace leaves z alone there anyway, except for the rounding of
 // the collider-crossing blend)
-__global__ void k_flip_advect(VelField F, long long n, float *__restrict__ pos, float dt, int max_substeps, F3 mn,
+template <bool P2>
+__global__ void k_flip_advect(const __grid_constant__ VelField F, long long n, float *__restrict__ pos, float dt, int max_substeps, F3 mn,
                               F3 mx, float push_thresh, float push_shift, int keep_z) {
     const F3 oc = comp_origin(F.g, 3);
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const F3 prev{pos[3 * p], pos[3 * p + 1], pos[3 * p + 2]};
-        const F3 tr = back_trace(F, prev, dt, -1.0f, max_substeps);
+        const F3 tr = back_trace<P2>(F, prev, dt, -1.0f, max_substeps, NAN);
         const bool bad = nonfinite(tr.x) || nonfinite(tr.y) || nonfinite(tr.z);
         F3 q{fminf(fmaxf(bad ? prev.x : tr.x, mn.x), mx.x), fminf(fmaxf(bad ? prev.y : tr.y, mn.y), mx.y),
              fminf(fmaxf(bad ? prev.z : tr.z, mn.z), mx.z)};
@@ -1291,13 +1292,13 @@ extern "C" int ff_flip3_stage(ff_flip f, int stage) {
     switch (stage) {
     case FF_FLIP_ADVECT_PARTICLES: {
         if (n == 0) return FF_OK;
-        VelField F{g, uvw[0], uvw[1], uvw[2], f->phi ? (const float *)f->phi->d : nullptr};
+        const VelField F = trace_field({g, uvw[0], uvw[1], uvw[2], f->phi ? (const float *)f->phi->d : nullptr});
         // minPos / maxPos (:927-929): the extent in doubles, stored as f32
         const F3 ext{(float)(d.resolution[0] * d.grid_spacing[0]), (float)(d.resolution[1] * d.grid_spacing[1]),
                      (float)(d.resolution[2] * d.grid_spacing[2])};
         const F3 mn{g.ox + 1e-4f, g.oy + 1e-4f, g.oz + 1e-4f};
         const F3 mx{(g.ox + ext.x) - 1e-4f, (g.oy + ext.y) - 1e-4f, (g.oz + ext.z) - 1e-4f};
-        k_flip_advect<<<blocks_for(n), 256, 0, s>>>(F, n, pos, (float)d.dt, d.max_substeps, mn, mx,
+        (F.pow2 ? k_flip_advect<true> : k_flip_advect<false>)<<<blocks_for(n), 256, 0, s>>>(F, n, pos, (float)d.dt, d.max_substeps, mn, mx,
                                                     (float)d.collider_push_thresh, (float)d.collider_push_shift, 0);
         return post("advectParticles");
     }
@@ -1905,12 +1906,12 @@ extern "C" int ff_twophase2_stage(ff_twophase t, int stage) {
         // advectParticles + pushOutOfCollider (:1098-1124)
         if (!three) FF_CUDA(cudaMemsetAsync(w, 0, comp_n(g, 2) * 4, s));
         if (n == 0) return FF_OK;
-        VelField F{g, uvw[0], uvw[1], w, t->phi ? (const float *)t->phi->d : nullptr};
+        const VelField F = trace_field({g, uvw[0], uvw[1], w, t->phi ? (const float *)t->phi->d : nullptr});
         const F3 mn{g.ox + 1e-4f, g.oy + 1e-4f, g.oz + 1e-4f};
         const F3 mx{(g.ox + (float)(d.resolution[0] * d.grid_spacing[0])) - 1e-4f,
                     (g.oy + (float)(d.resolution[1] * d.grid_spacing[1])) - 1e-4f,
                     three ? (g.oz + (float)(d.resolution[2] * d.grid_spacing[2])) - 1e-4f : (g.oz + g.hz) - 1e-4f};
-        k_flip_advect<<<blocks_for(n), 256, 0, s>>>(F, n, pos, (float)d.dt, d.max_substeps, mn, mx,
+        (F.pow2 ? k_flip_advect<true> : k_flip_advect<false>)<<<blocks_for(n), 256, 0, s>>>(F, n, pos, (float)d.dt, d.max_substeps, mn, mx,
                                                     (float)d.collider_push_thresh, (float)d.collider_push_shift,
                                                     three ? 0 : 1);
         return post("advectParticles");

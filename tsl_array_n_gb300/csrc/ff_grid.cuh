@@ -110,11 +110,38 @@ __device__ float tricubic(const float *__restrict__ d, int sx, int sy, int sz, c
     return mono_cubic(zv[0], zv[1], zv[2], zv[3], fz);
 }
 
+typedef unsigned long long f32x2;   // two packed floats
+
+// what one axis of the grid gives the samples of the trace (trace_field)
+struct TraceAxis {
+    float h, r;      // spacing, reciprocal
+    float o[2];      // origin of the face grid (0) and of the centre grid (1)
+    int end[2];      // below it an index has both linear taps inside
+};
 struct VelField {
     G3 g;
     const float *u, *v, *w;   // velocity the trace follows
     const float *phi;         // collider SDF (cell centred) or null
+    // for the trace and the samples along it (trace_field)
+    TraceAxis ax[3];
+    f32x2 nzero;              // (-0, -0), see prod2
+    int pow2;                 // all three spacings are powers of two
 };
+inline VelField trace_field(VelField F) {
+    const float h[3] = {F.g.hx, F.g.hy, F.g.hz}, o[3] = {F.g.ox, F.g.oy, F.g.oz};
+    const int n[3] = {F.g.nx, F.g.ny, F.g.nz};
+    F.nzero = 0x8000000080000000ull;
+    F.pow2 = 1;
+    for (int a = 0; a < 3; ++a) {
+        int e;
+        F.pow2 = F.pow2 && frexpf(h[a], &e) == 0.5f;
+        // (split() takes coordinates below 2^22; a grid one cell thick has one
+        // centre plane, both of its taps)
+        const int end = std::min(n[a], 1 << 22);
+        F.ax[a] = TraceAxis{h[a], 1.0f / h[a], {o[a], o[a] + h[a] * 0.5f}, {end, a == 2 && n[a] == 1 ? 1 : end - 1}};
+    }
+    return F;
+}
 
 __device__ __forceinline__ F3 sample_vel(const VelField &F, F3 p) {
     int sx, sy, sz;
@@ -132,29 +159,261 @@ __device__ __forceinline__ float sample_phi(const VelField &F, const float *phi,
     return trilinear(phi, F.g.nx, F.g.ny, F.g.nz, F.g, comp_origin(F.g, 3), p);
 }
 
+// ---- samples away from the array ends -----------------------------------
+// The trace and the tricubic sample are bound by issue and by instruction
+// fetch (about 2300 instructions a face in the straightforward form), so where
+// no tap needs clamping they run in a shorter form of the same operations: the
+// six coordinates that the three face grids and the cell grid share are formed
+// once, the division by h is a multiplication where h is a power of two (P2) and
+// a corrected product elsewhere, floor is an addition, taps of a row share an
+// address, and two samples run in one packed FP32 pair (add, sub and mul round
+// each half as the scalar instruction does).  A point with a tap past an end
+// takes the functions above.
+
+// a / h, correctly rounded: with r the correctly rounded 1 / h, one Newton
+// correction makes the product faithful and a second, by Markstein's theorem
+// (1990), correct; exact for a power of two.  For quotients from 1e-20 to 2e8,
+// where the remainders are exact.
+template <bool P2>
+__device__ __forceinline__ float div_in(float a, float h, float r) {
+    const float q = a * r;
+    if (P2) return q;
+    const float q1 = __fmaf_rn(__fmaf_rn(-q, h, a), r, q);
+    return __fmaf_rn(__fmaf_rn(-q1, h, a), r, q1);
+}
+__device__ __noinline__ float div_any(float a, float h) { return a / h; }
+template <bool P2>
+__device__ __forceinline__ float div_h(float a, float h, float r) {
+    const float q = div_in<P2>(a, h, r);
+    if (P2) return q;
+    return q < 2.0e8f && q > 1.0e-20f ? q : div_any(a, h);
+}
+// index and fraction of a coordinate in [0, 2^22): 1.5 * 2^23 added rounding
+// down leaves the floor in the low bits of the significand (floorf and the
+// conversion run at a quarter of the rate).  As an unsigned number the index is
+// 2^22 or more for a larger or negative coordinate and for a NaN.
+__device__ __forceinline__ void split(float q, int &i, float &f) {
+    const float t = __fadd_rd(q, 12582912.0f);
+    i = __float_as_int(t) - 0x4b400000;
+    f = q - (t - 12582912.0f);
+}
+// one axis: index and fraction of a point on the face (0) or centre (1) grid;
+// false where a tap is outside, or the coordinate below div_in's range
+template <bool P2>
+__device__ __forceinline__ bool axis_at(const TraceAxis &A, int c, float p, int &i, float &f) {
+    const float q = div_in<P2>(p - A.o[c], A.h, A.r);
+    split(q, i, f);
+    return (unsigned)i < (unsigned)A.end[c] && (P2 || q > 1.0e-20f);
+}
+
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ void unpack2(f32x2 d, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(d));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// a product that is an operand of a sum: the compiler contracts add2(c, mul2(a,
+// b)) to one rounding whatever -fmad says.  A fused a b + (-0) is the rounded
+// product, sign of zero included, and where the compiler cannot see that the
+// addend z is -0 it stays two operations; z therefore comes with the arguments.
+__device__ __forceinline__ f32x2 prod2(f32x2 a, f32x2 b, f32x2 z) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(z));
+    return d;
+}
+struct Axis6 {
+    int i[2];
+    float f[2];
+};
+struct Point6 {
+    Axis6 x, y, z;
+};
+template <bool P2>
+__device__ __forceinline__ bool point6(const VelField &F, F3 p, Point6 &q) {
+    bool in = true;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        in &= axis_at<P2>(F.ax[0], c, p.x, q.x.i[c], q.x.f[c]);
+        in &= axis_at<P2>(F.ax[1], c, p.y, q.y.i[c], q.y.f[c]);
+        in &= axis_at<P2>(F.ax[2], c, p.z, q.z.i[c], q.z.f[c]);
+    }
+    return in;
+}
+// trilinear() at index (i, j, k) with all taps inside, planes dz apart (0 for
+// the centre plane of a grid one cell thick)
+__device__ __forceinline__ float lin1(const float *__restrict__ d, int sx, int sy, int dz, int i, int j, int k, float fx,
+                                      float fy, float fz) {
+    const float *r0 = d + (i + sx * (j + sy * k)), *r1 = r0 + sx, *r2 = r0 + dz, *r3 = r2 + sx;
+    const float ux = 1.0f - fx, uy = 1.0f - fy, uz = 1.0f - fz;
+    const float w00 = ux * uy, w10 = fx * uy, w01 = ux * fy, w11 = fx * fy;
+    float s = __ldg(r0) * (w00 * uz);
+    s = s + __ldg(r0 + 1) * (w10 * uz);
+    s = s + __ldg(r1) * (w01 * uz);
+    s = s + __ldg(r1 + 1) * (w11 * uz);
+    s = s + __ldg(r2) * (w00 * fz);
+    s = s + __ldg(r2 + 1) * (w10 * fz);
+    s = s + __ldg(r3) * (w01 * fz);
+    return s + __ldg(r3 + 1) * (w11 * fz);
+}
+// two of them, u and v
+__device__ __forceinline__ void lin_uv(const VelField &F, const Point6 &q, float &u, float &v) {
+    const int nx = F.g.nx, ny = F.g.ny;
+    const float *a0 = F.u + (q.x.i[0] + (nx + 1) * (q.y.i[1] + ny * q.z.i[1]));
+    const float *b0 = F.v + (q.x.i[1] + nx * (q.y.i[0] + (ny + 1) * q.z.i[1]));
+    const bool flat = F.g.nz == 1;
+    const float *a1 = a0 + (nx + 1), *a2 = a0 + (flat ? 0 : (nx + 1) * ny), *a3 = a2 + (nx + 1);
+    const float *b1 = b0 + nx, *b2 = b0 + (flat ? 0 : nx * (ny + 1)), *b3 = b2 + nx;
+    const f32x2 one = pack2(1.0f, 1.0f);
+    const f32x2 fx = pack2(q.x.f[0], q.x.f[1]), fy = pack2(q.y.f[1], q.y.f[0]), fz = pack2(q.z.f[1], q.z.f[1]);
+    const f32x2 ux = sub2(one, fx), uy = sub2(one, fy), uz = sub2(one, fz);
+    const f32x2 w00 = mul2(ux, uy), w10 = mul2(fx, uy), w01 = mul2(ux, fy), w11 = mul2(fx, fy);
+    auto d = [](const float *a, const float *b) { return pack2(__ldg(a), __ldg(b)); };
+    f32x2 s = prod2(d(a0, b0), mul2(w00, uz), F.nzero);
+    s = add2(s, prod2(d(a0 + 1, b0 + 1), mul2(w10, uz), F.nzero));
+    s = add2(s, prod2(d(a1, b1), mul2(w01, uz), F.nzero));
+    s = add2(s, prod2(d(a1 + 1, b1 + 1), mul2(w11, uz), F.nzero));
+    s = add2(s, prod2(d(a2, b2), mul2(w00, fz), F.nzero));
+    s = add2(s, prod2(d(a2 + 1, b2 + 1), mul2(w10, fz), F.nzero));
+    s = add2(s, prod2(d(a3, b3), mul2(w01, fz), F.nzero));
+    s = add2(s, prod2(d(a3 + 1, b3 + 1), mul2(w11, fz), F.nzero));
+    unpack2(s, u, v);
+}
+__device__ __noinline__ F3 sample_vel_ends(const VelField &F, F3 p) { return sample_vel(F, p); }
+__device__ __noinline__ float sample_phi_ends(const VelField &F, F3 p) { return sample_phi(F, F.phi, p); }
+template <bool P2>
+__device__ __forceinline__ F3 trace_vel(const VelField &F, F3 p) {
+    Point6 q;
+    if (!point6<P2>(F, p, q)) return sample_vel_ends(F, p);
+    F3 r;
+    lin_uv(F, q, r.x, r.y);
+    r.z = lin1(F.w, F.g.nx, F.g.ny, F.g.nx * F.g.ny, q.x.i[1], q.y.i[1], q.z.i[0], q.x.f[1], q.y.f[1], q.z.f[0]);
+    return r;
+}
+template <bool P2>
+__device__ __forceinline__ float trace_phi(const VelField &F, F3 p) {
+    if (!F.phi) return 1.0f;
+    int i, j, k;
+    float fx, fy, fz;
+    bool in = axis_at<P2>(F.ax[0], 1, p.x, i, fx);
+    in &= axis_at<P2>(F.ax[1], 1, p.y, j, fy);
+    in &= axis_at<P2>(F.ax[2], 1, p.z, k, fz);
+    if (!in) return sample_phi_ends(F, p);
+    const G3 &g = F.g;
+    return lin1(F.phi, g.nx, g.ny, g.nz == 1 ? 0 : g.nx * g.ny, i, j, k, fx, fy, fz);
+}
+
+// mono_cubic on two rows of taps at once
+__device__ __forceinline__ f32x2 mono_cubic2(f32x2 f0, f32x2 f1, f32x2 f2, f32x2 f3, f32x2 f, f32x2 z) {
+    const f32x2 half = pack2(0.5f, 0.5f);
+    const f32x2 D1 = sub2(f2, f1), r1 = mul2(sub2(f2, f0), half), r2 = mul2(sub2(f3, f1), half);
+    float Da, Db, r1a, r1b, r2a, r2b, p1a, p1b, p2a, p2b;
+    unpack2(D1, Da, Db);
+    unpack2(r1, r1a, r1b);
+    unpack2(r2, r2a, r2b);
+    unpack2(mul2(r1, D1), p1a, p1b);
+    unpack2(mul2(r2, D1), p2a, p2b);
+    const bool fa = fabsf(Da) < 1e-12f, fb = fabsf(Db) < 1e-12f;
+    const f32x2 d1 = pack2((fa || p1a < 0.0f) ? 0.0f : r1a, (fb || p1b < 0.0f) ? 0.0f : r1b);
+    const f32x2 d2 = pack2((fa || p2a < 0.0f) ? 0.0f : r2a, (fb || p2b < 0.0f) ? 0.0f : r2b);
+    const f32x2 three = pack2(3.0f, 3.0f);
+    const f32x2 a3 = sub2(add2(d1, d2), add2(D1, D1));
+    const f32x2 a2 = sub2(sub2(prod2(D1, three, z), add2(d1, d1)), d2);
+    f32x2 t = prod2(mul2(mul2(a3, f), f), f, z);
+    t = add2(t, prod2(mul2(a2, f), f, z));
+    t = add2(t, prod2(d1, f, z));
+    return add2(t, f1);
+}
+__device__ __noinline__ float tricubic_ends(const float *__restrict__ d, int sx, int sy, int sz, const G3 &g, F3 o, F3 p) {
+    return tricubic(d, sx, sy, sz, g, o, p);
+}
+// tricubic() on component a (3: cells): rows of two z taps at a time
+template <bool P2>
+__device__ __forceinline__ float trace_cubic(const VelField &F, int a, const float *__restrict__ d, int sx, int sy, int sz,
+                                             F3 o, F3 p) {
+    int i, j, k;
+    float fx, fy, fz;
+    bool in = axis_at<P2>(F.ax[0], a != 0, p.x, i, fx);
+    in &= axis_at<P2>(F.ax[1], a != 1, p.y, j, fy);
+    in &= axis_at<P2>(F.ax[2], a != 2, p.z, k, fz);
+    // one plane: every z tap is that plane
+    const int z0 = sz == 1 ? 0 : 1, dz = sz == 1 ? 0 : sx * sy;
+    if (!(in && i >= 1 && i <= sx - 3 && j >= 1 && j <= sy - 3 && k >= z0 && (sz == 1 || k <= sz - 3)))
+        return tricubic_ends(d, sx, sy, sz, F.g, o, p);
+    const f32x2 fx2 = pack2(fx, fx), fy2 = pack2(fy, fy);
+    const float *r = d + ((i - 1) + sx * ((j - 1) + sy * (k - z0)));
+    float z[4];
+#pragma unroll 1
+    for (int c = 0; c < 2; ++c) {
+        f32x2 row[4];
+        const float *ra = r, *rb = r + dz;
+#pragma unroll
+        for (int b = 0; b < 4; ++b, ra += sx, rb += sx)
+            row[b] = mono_cubic2(pack2(__ldg(ra), __ldg(rb)), pack2(__ldg(ra + 1), __ldg(rb + 1)),
+                                 pack2(__ldg(ra + 2), __ldg(rb + 2)), pack2(__ldg(ra + 3), __ldg(rb + 3)), fx2, F.nzero);
+        z[0] = z[2], z[1] = z[3];
+        unpack2(mono_cubic2(row[0], row[1], row[2], row[3], fy2, F.nzero), z[2], z[3]);
+        r += 2 * dz;
+    }
+    return mono_cubic(z[0], z[1], z[2], z[3], fz);
+}
+
 // backTrace (advection_solver3.js:20-62): RK2 midpoint substeps of at most
-// one cell, stopping on the collider with a linear blend of the last step
-__device__ F3 back_trace(const VelField &F, F3 pos, float dt, float dirn, int max_substeps) {
+// one cell, stopping on the collider with a linear blend of the last step.
+// phi0: the collider's value at pos, if the caller has it (else a NaN); a
+// substep's end is the next one's start, with its value.
+template <bool P2>
+__device__ __forceinline__ F3 back_trace(const VelField &F, F3 pos, float dt, float dirn, int max_substeps, float phi0) {
     const float h = fminf(F.g.hx, fminf(F.g.hy, F.g.hz));
+    const float rh = h == F.g.hx ? F.ax[0].r : (h == F.g.hy ? F.ax[1].r : F.ax[2].r);
     F3 pt = pos;
     float T = dt;
+#pragma unroll 1
     for (int s = 0; s < max_substeps; ++s) {
         if (T <= 1e-6f) break;
-        const F3 v0 = sample_vel(F, pt);
-        const float len = sqrtf(v0.x * v0.x + v0.y * v0.y + v0.z * v0.z);
-        const float nsub = fmaxf(ceilf(len * T / h), 1.0f);
-        const float sdt = T / nsub;
-        const float hs = sdt * 0.5f;
-        const F3 mid{pt.x - v0.x * hs * dirn, pt.y - v0.y * hs * dirn, pt.z - v0.z * hs * dirn};
-        const F3 mv = sample_vel(F, mid);
-        const F3 nxt{pt.x - mv.x * sdt * dirn, pt.y - mv.y * sdt * dirn, pt.z - mv.z * sdt * dirn};
-        const float phi0 = sample_phi(F, F.phi, pt), phi1 = sample_phi(F, F.phi, nxt);
+        F3 at = pt;
+        float sdt = 0.0f;
+        // one copy of the sample's code for the start and the midpoint
+#pragma unroll 1
+        for (int mid = 0; mid < 2; ++mid) {
+            const F3 v = trace_vel<P2>(F, at);
+            float step;
+            if (mid == 0) {
+                const float len = sqrtf(v.x * v.x + v.y * v.y + v.z * v.z);
+                const float nsub = fmaxf(ceilf(div_h<P2>(len * T, h, rh)), 1.0f);
+                sdt = nsub == 1.0f ? T : T / nsub;
+                step = sdt * 0.5f;
+            } else {
+                step = sdt;
+            }
+            at = F3{pt.x - v.x * step * dirn, pt.y - v.y * step * dirn, pt.z - v.z * step * dirn};
+        }
+        const F3 nxt = at;
+        const float phi1 = trace_phi<P2>(F, nxt);
         if (phi1 <= 0.0f) {
+            if (s == 0 && isnan(phi0)) phi0 = trace_phi<P2>(F, pt);
             const float w = fabsf(phi1) / (fabsf(phi0) + fabsf(phi1));
             const float wm = 1.0f - w;
             pt = F3{pt.x * w + nxt.x * wm, pt.y * w + nxt.y * wm, pt.z * w + nxt.z * wm};
             break;
         }
+        phi0 = phi1;
         T = T - sdt;
         pt = nxt;
     }
