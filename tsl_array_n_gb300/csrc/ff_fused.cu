@@ -80,18 +80,6 @@ __device__ __forceinline__ bool brick_regular(const Geo &g, const uint8_t *brick
     return bricks[blockIdx.x + (long long)g.bnx * (blockIdx.y + (long long)g.bny * bz)] != 0;
 }
 
-// compensated (TwoSum) FP32 accumulation, folded into FP64 once
-struct Acc {
-    float s = 0.f, e = 0.f;
-    __device__ __forceinline__ void add(float v) {
-        float t, err;
-        two_sum(s, v, t, err);
-        s = t;
-        e = __fadd_rn(e, err);
-    }
-    __device__ __forceinline__ double value() const { return (double)s + (double)e; }
-};
-
 // ----------------------------------------------------------------- sweep --
 struct SweepArgs {
     Geo g;
@@ -285,7 +273,7 @@ __global__ void __launch_bounds__(NT, 4) k_sweep(SweepArgs a) {
 // Waits are bounded in time: a block that gives up records bit 0 of
 // PcgState::err and stops (the host then reports the solve as failed).
 namespace tq {
-constexpr int TX = 64, TY = 16, QX = TX / 4, NT = QX * TY;   // 16 x 16 threads
+constexpr int TX = DOT_TX, TY = DOT_TY, QX = TX / 4, NT = QX * TY;   // 16 x 16 threads
 constexpr int RW = TX + 8;                  // staged columns i0-4 .. i0+TX+3
 constexpr int XR = TY + 4, BR = TY + 2;     // staged rows of x and of b
 constexpr int SD = 3;                       // stages in flight
@@ -514,7 +502,7 @@ __global__ void __launch_bounds__(tq::NT, 4)
     const Geo &g = a.g;
     // warp w holds rows r and r+2 (same colour parity), r = 4(w/2) + w%2
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int qx = lane & (QX - 1), ty = 4 * (warp >> 1) + (warp & 1) + 2 * (lane >> 4);
+    const int qx = dot_quad(tid), ty = dot_row(tid);
     // the TMA issuer is the last thread, which has no ring cell
     constexpr int ISSUER = tq::NT - 1;
     static_assert(ISSUER / 32 >= 3, "issuer carries no ring cell");
@@ -851,7 +839,7 @@ __global__ void __launch_bounds__(tq::NT, 4)
 // zero-filled neighbour entered as 0 - v), -v for a Dirichlet row (class 1),
 // the stored couplings otherwise (class 3).
 namespace tcg {
-constexpr int TX = 64, TY = 16, QX = TX / 4, NT = QX * TY;
+constexpr int TX = DOT_TX, TY = DOT_TY, QX = TX / 4, NT = QX * TY;
 constexpr int RW = TX + 8, PR = TY + 2;   // staged columns i0-4 .. i0+TX+3, rows j0-1 .. j0+TY
 constexpr int PPL = ((PR * RW * 4 + 127) / 128) * 32;   // plane slot (1312 floats)
 constexpr int BPL = TY * RW;                            // b: rows j0 .. j0+TY-1 (1152 floats)
@@ -882,41 +870,6 @@ __device__ __forceinline__ float4 fma4(float s, const float4 &a, const float4 &b
 }
 __device__ __forceinline__ void st4(float *p, const float4 &v) { *reinterpret_cast<float4 *>(p) = v; }
 
-// A neighbour across the domain edge stands in as the cell itself, so the
-// absent face's difference is an exact zero.  (Adding h^-2 v back to a
-// zero-filled neighbour's -h^-2 v cancels to within a rounding of h^-2 |v|:
-// near a wall under a hydrostatic pressure that is far above the residual
-// the solve has to reach.)
-__device__ __forceinline__ void edge_self(const Geo &g, int i, int j, int k, float vc, float &xm, float &xp,
-                                          float &ym, float &yp, float &zm, float &zp) {
-    if (i == 0) xm = vc;
-    if (i == g.d.nx - 1) xp = vc;
-    if (j == 0) ym = vc;
-    if (j == g.d.ny - 1) yp = vc;
-    if (k == 0) zm = vc;
-    if (k == g.d.nz - 1) zp = vc;
-}
-
-// (A v)_c of one cell by class; ci its index.
-__device__ __forceinline__ float ap_cell(const Geo &g, const float4 *coef, const float4 *gco, unsigned c, int i,
-                                         int j, int k, long long ci, float vc, float xm, float xp, float ym, float yp,
-                                         float zm, float zp) {
-    if (c == 2u) edge_self(g, i, j, k, vc, xm, xp, ym, yp, zm, zp);
-    const float ar = apply_reg(g, vc, xm, xp, ym, yp, zm, zp);
-    if (c == 0u || c == 2u) return ar;
-    if (c == 1u) return -vc;
-    const float4 lo = __ldg(coef + ci), hi = __ldg(gco + ci);
-    Coef q;
-    q.kx = i > 0 ? lo.x : 0.f;
-    q.ky = j > 0 ? lo.y : 0.f;
-    q.kz = k > 0 ? lo.z : 0.f;
-    q.e = lo.w;
-    q.ux = hi.x;
-    q.uy = hi.y;
-    q.uz = hi.z;
-    return apply_q(q, vc, xm, xp, ym, yp, zm, zp);
-}
-
 __global__ void __launch_bounds__(tcg::NT, 4)
     k_p_pap_tma(TcgArgs a, const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUtensorMap p0map,
                 const __grid_constant__ CUtensorMap p1map, const __grid_constant__ CUtensorMap cmap) {
@@ -934,7 +887,7 @@ __global__ void __launch_bounds__(tcg::NT, 4)
     const unsigned bar0 = smem_u32(cs + SD * CPL);
     const Geo &g = a.g;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int qx = lane & (QX - 1), ty = 4 * (warp >> 1) + (warp & 1) + 2 * (lane >> 4);
+    const int qx = dot_quad(tid), ty = dot_row(tid);
     constexpr int ISSUER = tcg::NT - 1;
     const int pc = st->p_cur;
     const bool first = st->first != 0;
@@ -1080,79 +1033,6 @@ __global__ void __launch_bounds__(tcg::NT, 4)
     }
 }
 
-// r = b - A x in double-single for one cell of class 1 or 3: each coupling
-// term K (x_n - x_c) formed from (hi, lo) with an error-free difference and
-// product, summed with TwoSum (the general path of the cp.async kernel).
-__device__ __forceinline__ float resid_ds_general(const Coef &q, float bc, float chv, float clv, float xmh,
-                                                  float xml, float xph, float xpl, float ymh, float yml, float yph,
-                                                  float ypl, float zmh, float zml, float zph, float zpl) {
-    float S = 0.f, Se = 0.f;
-    auto term = [&](float K, float hn, float ln) {
-        float dh, de;
-        two_sum(hn, -chv, dh, de);
-        de = __fadd_rn(de, __fsub_rn(ln, clv));
-        float pr, pe;
-        two_prod(K, dh, pr, pe);
-        pe = __fmaf_rn(K, de, pe);
-        float s2, e2;
-        two_sum(S, pr, s2, e2);
-        S = s2;
-        Se = __fadd_rn(Se, __fadd_rn(e2, pe));
-    };
-    term(q.kx, xmh, xml);
-    term(q.ux, xph, xpl);
-    term(q.ky, ymh, yml);
-    term(q.uy, yph, ypl);
-    term(q.kz, zmh, zml);
-    term(q.uz, zph, zpl);
-    {
-        float pr, pe;
-        two_prod(-q.e, chv, pr, pe);
-        pe = __fmaf_rn(-q.e, clv, pe);
-        float s2, e2;
-        two_sum(S, pr, s2, e2);
-        S = s2;
-        Se = __fadd_rn(Se, __fadd_rn(e2, pe));
-    }
-    float r0, e0;
-    two_sum(bc, -S, r0, e0);
-    return __fadd_rn(r0, __fsub_rn(e0, Se));
-}
-
-// One cell's residual by class (hi/lo of the cell and its six neighbours).
-template <bool DS>
-__device__ __forceinline__ float resid_cell(const Geo &g, const float4 *coef, const float4 *gco, unsigned c, int i,
-                                            int j, int k, long long ci, float bc, float ch, float cl, float xmh,
-                                            float xml, float xph, float xpl, float ymh, float yml, float yph,
-                                            float ypl, float zmh, float zml, float zph, float zpl) {
-    if (!(c & 1u)) {
-        if (c == 2u) {
-            edge_self(g, i, j, k, ch, xmh, xph, ymh, yph, zmh, zph);
-            if (DS) edge_self(g, i, j, k, cl, xml, xpl, yml, ypl, zml, zpl);
-        }
-        float ax = apply_reg(g, ch, xmh, xph, ymh, yph, zmh, zph);
-        if (DS) ax += apply_reg(g, cl, xml, xpl, yml, ypl, zml, zpl);
-        return bc - ax;
-    }
-    Coef q;
-    if (c == 1u) {
-        q.kx = q.ky = q.kz = q.ux = q.uy = q.uz = 0.f;
-        q.e = 1.f;
-    } else {
-        const float4 lo = __ldg(coef + ci), hi = __ldg(gco + ci);
-        q.kx = i > 0 ? lo.x : 0.f;
-        q.ky = j > 0 ? lo.y : 0.f;
-        q.kz = k > 0 ? lo.z : 0.f;
-        q.e = lo.w;
-        q.ux = hi.x;
-        q.uy = hi.y;
-        q.uz = hi.z;
-    }
-    if (DS)
-        return resid_ds_general(q, bc, ch, cl, xmh, xml, xph, xpl, ymh, yml, yph, ypl, zmh, zml, zph, zpl);
-    return bc - apply_q(q, ch, xmh, xph, ymh, yph, zmh, zph);
-}
-
 template <bool SETUP, bool DS>
 __global__ void __launch_bounds__(tcg::NT, 2)
     k_x_residual_tma(TcgArgs a, const __grid_constant__ CUtensorMap h0map, const __grid_constant__ CUtensorMap h1map,
@@ -1176,7 +1056,7 @@ __global__ void __launch_bounds__(tcg::NT, 2)
     const unsigned bar0 = smem_u32(cs + SD * CPL);
     const Geo &g = a.g;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int qx = lane & (QX - 1), ty = 4 * (warp >> 1) + (warp & 1) + 2 * (lane >> 4);
+    const int qx = dot_quad(tid), ty = dot_row(tid);
     constexpr int ISSUER = tcg::NT - 1;
     const int xc = SETUP ? 0 : st->x_cur;
     const CUtensorMap *hm = xc ? &h1map : &h0map, *lm = xc ? &l1map : &l0map;
@@ -2515,6 +2395,10 @@ static int cg_bps(int which) { return which == 0 ? 4 : 2; }
 size_t cg_tma_items(const Dims &d, int sm_count, int which) {
     const int zc = tma_zchunk_bps(d, sm_count, cg_bps(which), tcg::TX, tcg::TY);
     return (size_t)((d.nx + tcg::TX - 1) / tcg::TX) * ((d.ny + tcg::TY - 1) / tcg::TY) * ((d.nz + zc - 1) / zc);
+}
+
+int cg_tma_planes(const Dims &d, int sm_count, int which) {
+    return which == 2 ? tma_zchunk(d, sm_count) : tma_zchunk_bps(d, sm_count, cg_bps(which), tcg::TX, tcg::TY);
 }
 
 size_t sweep_tma_blocks(const Dims &d, int sm_count) {

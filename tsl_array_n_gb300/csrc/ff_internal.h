@@ -251,15 +251,18 @@ size_t cls_row_pitch(const Dims &d);
 int vcycle_tail(const Level *lv, const SweepMaps *sm, int nl, int dims, int down, int up, float sor,
                 const double *G, int nG, int coarse_sweeps, PcgState *st, unsigned *bar, int sm_count,
                 cudaStream_t s);
-// a whole PCG solve (after k_state_init) in one cooperative launch, for
+// a whole PCG solve (after k_state_init) in one launch, for
 // hierarchies of at most 12 levels with classes on all but the coarsest
 // and at least one sweep before and after the correction; levels' x and b as in
 // the V-cycle (lv[0]: z and r); partials: 8 sums of sm_count doubles
+// alt: scratch of level 0's size (values at tile edges)
+// cluster: blocks of one cluster that the device can run (cluster_blocks()), 0: none
 constexpr long long PCG_RESIDENT_CELLS = 1LL << 20;
+int cluster_blocks();
 int pcg_resident(const Level *lv, const SweepMaps *sm, int nl, int dims, int down, int up, int fin, float sor,
                  const double *G, int nG, int coarse_sweeps, const float *b, float *p0, float *p1, float *xh0, float *xl0,
                  float *xh1, float *xl1, int ds, PcgState *st, double *partials, unsigned *bar, int sm_count,
-                 cudaStream_t s);
+                 int cluster, float *alt, cudaStream_t s);
 int cg_tma_maps(const Level &L0, const float *z0, const float *z1, const float *p0, const float *p1,
                 const float *xh0, const float *xl0, const float *xh1, const float *xl1, const float *b, bool ds,
                 CgMaps &m);
@@ -272,6 +275,8 @@ int sweep_tma(const Level &L, const SweepMaps &m, const uint8_t *bricks, int in,
 size_t sweep_tma_blocks(const Dims &d, int sm_count);
 // work items of the level-0 TMA CG kernels (which: 0 p.Ap, 1 x + alpha p)
 size_t cg_tma_items(const Dims &d, int sm_count, int which);
+// planes of a work item (which: 0 p.Ap, 1 x + alpha p, 2 the sweep)
+int cg_tma_planes(const Dims &d, int sm_count, int which);
 int res_restrict(const Level &f, const uint8_t *bricks, const float *x, Level &c, int dims,
                  const PcgState *st, int sm_count, cudaStream_t s);
 int fused_p_pap(const Level &L0, const uint8_t *bricks, const float *z, float *p0, float *p1,

@@ -61,6 +61,7 @@ struct ff_pressure_s {
     int tail_l = -1;
     // level 0 is small enough for the whole solve in one cooperative launch
     bool resident_fits = false;
+    int cluster = 0;                // blocks of a cluster for the resident solve
     bool use_tail = true;
     unsigned *tail_bar = nullptr;   // its grid barrier: arrivals, generation, abort
     // learned warm start (borrowed network), its guess field, last choice
@@ -252,10 +253,7 @@ extern "C" int ff_pressure3_create(ff_ctx ctx, const ff_pressure_desc *desc, ff_
                        div_up(g.ny, 256 / (g.nx >= 128 ? 128 : g.nx >= 64 ? 64 : 32)) * g.nz;
     blocks = std::max(blocks, (long long)div_up(n, 1024));
     blocks = std::max(blocks, (long long)ffk::fused_blocks(ps->d, ctx->sm_count));
-    // the whole solve in one launch: every level but the coarsest keeps classes
-    ps->resident_fits = desc->vcycle_storage == FF_STORE_FP32 && L >= 2 && n <= ffk::PCG_RESIDENT_CELLS;
-    if (ps->resident_fits) blocks = std::max(blocks, 4LL * ctx->sm_count);
-    if (ps->fused || ps->resident_fits) ps->smaps = new SweepMaps[L];
+    if (ps->fused) ps->smaps = new SweepMaps[L];
     if (ps->fused) {
         for (int l = 0; l < L; ++l) {
             Level &v = ps->lv[l];
@@ -290,7 +288,13 @@ extern "C" int ff_pressure3_create(ff_ctx ctx, const ff_pressure_desc *desc, ff_
             for (int q = l; q < L - 1; ++q) ok = ok && ps->lv[q].d.nx % 4 == 0 && ps->lv[q].buf;
             if (ok) ps->tail_l = l;
         }
+        // the whole solve in one launch (resident()): where level 0 takes the TMA
+        // kernels and every level below it the coarse V-cycle's
+        ps->resident_fits = desc->vcycle_storage == FF_STORE_FP32 && L >= 2 && n <= ffk::PCG_RESIDENT_CELLS &&
+                            ffk::sweep_tma_ok(ps->lv[0].d) && ps->lv[0].buf && (L == 2 || ps->tail_l == 1) &&
+                            (desc->mg_coarse_mode == FF_COARSE_DIRECT || ps->lv[L - 1].d.n() <= 16384);
     }
+    if (ps->resident_fits) ps->cluster = ffk::cluster_blocks();
     if ((ps->tail_l >= 0 || ps->resident_fits) &&
         (st = ff_dev_alloc((void **)&ps->tail_bar, 4 * sizeof(unsigned), s)))
         return bail(st);
@@ -946,14 +950,12 @@ static int build_graphs(ff_pressure ps) {
 
 // The whole solve in one launch: a multigrid-preconditioned solve with a
 // small level 0, with none of the settings that ask for the separate
-// kernels.  Measured against the graph of separate launches (whole projection):
-// 48 x 24 x 24 1.11 -> 0.47 ms, 2D 128^2 3.67 -> 1.73, 90 x 54 x 66 7.15 -> 5.45
-// (per-colour kernels), 1024 x 256 channel step 18.4 -> 10.9.
-// The line lies where the two meet: 96^3 3.32 -> 2.94 ms (10.9 -> 8.7 with
-// variable density), 2D 1024^2 25.3 -> 23.1, 128 x 96 x 96 (1.2M cells) 6.69 against
-// 6.67, 128^3 9.3 against 11.7.
+// kernels, whose results it gives bit for bit (a rounding of its own would, in a
+// slowly converging solve, now and then end it an iteration earlier or later).
+// Measured against the graph of separate launches (whole projection): 48 x 24 x 24
+// 1.11 -> 0.38 ms, 2D 128^2 3.69 -> 1.24, 1024 x 256 channel step 16.6 -> 10.6.
 static bool resident(const ff_pressure ps) {
-    return ps->resident_fits && ps->use_graph && ps->use_tma && ps->use_tail &&
+    return ps->resident_fits && ps->use_graph && cg_tma(ps) && ps->use_tail &&
            ps->desc.preconditioner == FF_PRE_MULTIGRID && ps->desc.mg_down > 0 && ps->desc.mg_final > 0 &&
            (ps->desc.mg_coarse_mode == FF_COARSE_DIRECT ? ps->G != nullptr : ps->desc.mg_coarsest > 0);
 }
@@ -968,7 +970,7 @@ static int run_solve(ff_pressure ps) {
                                  ps->desc.mg_up, ps->desc.mg_final, (float)ps->desc.mg_sor, direct ? ps->G : nullptr,
                                  direct ? ps->nG : 0, direct ? 0 : ps->desc.mg_coarsest, (const float *)ps->bfield->d,
                                  ps->p0, ps->p1, ps->xh0(), ps->x_lo0, ps->x_hi1, ps->x_lo1, ps->ds(), ps->st,
-                                 ps->partials, ps->tail_bar, ps->ctx->sm_count, s);
+                                 ps->partials, ps->tail_bar, ps->ctx->sm_count, ps->cluster, ps->x2[0], s);
     }
     if (ps->use_graph) {
         if (!ps->setup_exec) FF_TRY(build_graphs(ps));
