@@ -12,7 +12,7 @@ from test_resident_gpu import solver_for
 pytestmark = pytest.mark.gpu
 
 CASES = [((32, 4, 2), 2, "sweeps"), ((36, 6, 1), 2, "sweeps"), ((32, 26, 22), 2, "sweeps"), ((66 * 2, 20, 6), 2, "sweeps"),
-         ((64, 32, 32), 4, "sweeps"), ((256, 256, 1), 5, "sweeps"), ((32, 2048, 1), 4, "sweeps"), ((68, 70, 1), 2, "sweeps"),
+         ((64, 32, 32), 4, "sweeps"), ((256, 192, 1), 4, "sweeps"), ((256, 256, 1), 5, "sweeps"), ((32, 2048, 1), 4, "sweeps"), ((68, 70, 1), 2, "sweeps"),
          ((32, 12, 8), 2, "direct"), ((32, 24, 24), 2, "direct"), ((48, 24, 16), 3, "direct"), ((96, 64, 1), 3, "direct"),
          ((64, 64, 48), 4, "sweeps"), ((320, 240, 1), 5, "sweeps"), ((64, 48, 40), 3, "direct"), ((36, 44, 42), 2, "sweeps")]
 
@@ -29,7 +29,6 @@ def test_one_launch_is_the_same_solve(gpu, shape, levels, coarse, precision):
         for _ in range(2):   # from zero, then from the first solve's pressure
             d = dict(s.project(grid, out)())
             runs.append((d["iterations"], d["residual"], s.pressure.to_array().copy(), [np.array(v) for v in out.get()]))
-        s.reset() if hasattr(s, "reset") else None
         got.append(runs)
     for a, b in zip(*got):
         assert a[0] == b[0] and a[1] == b[1]

@@ -254,7 +254,8 @@ int vcycle_tail(const Level *lv, const SweepMaps *sm, int nl, int dims, int down
 // a whole PCG solve (after k_state_init) in one launch, for
 // hierarchies of at most 12 levels with classes on all but the coarsest
 // and at least one sweep before and after the correction; levels' x and b as in
-// the V-cycle (lv[0]: z and r); partials: 8 sums of sm_count doubles
+// the V-cycle (lv[0]: z and r); partials: four times the work items of the largest
+// of level 0's dot products
 // alt: scratch of level 0's size (values at tile edges)
 // cluster: blocks of one cluster that the device can run (cluster_blocks()), 0: none
 constexpr long long PCG_RESIDENT_CELLS = 1LL << 20;

@@ -305,7 +305,9 @@ extern "C" int ff_pressure3_create(ff_ctx ctx, const ff_pressure_desc *desc, ff_
         if ((st = ff_dev_alloc((void **)&m.gco, (size_t)ps->lv[l].d.n() * sizeof(float4), s))) return bail(st);
         m.cls_pitch = (int)ffk::cls_row_pitch(ps->lv[l].d);
     }
-    if ((st = ff_dev_alloc((void **)&ps->partials, (size_t)blocks * 2 * sizeof(double), s))) return bail(st);
+    // (one launch keeps the sums of p.Ap, r.r with b.b, and r.z apart)
+    if ((st = ff_dev_alloc((void **)&ps->partials, (size_t)blocks * (ps->resident_fits ? 4 : 2) * sizeof(double), s)))
+        return bail(st);
     if (ps->smaps && ps->smaps[0].ok &&
         (st = ffk::cg_tma_maps(ps->lv[0], (const float *)ps->z, ps->x2[0], ps->p0, ps->p1, ps->xh0(), ps->x_lo0,
                                ps->x_hi1, ps->x_lo1, (const float *)ps->bfield->d, ps->ds(), ps->cgm)))
@@ -953,7 +955,10 @@ static int build_graphs(ff_pressure ps) {
 // kernels, whose results it gives bit for bit (a rounding of its own would, in a
 // slowly converging solve, now and then end it an iteration earlier or later).
 // Measured against the graph of separate launches (whole projection): 48 x 24 x 24
-// 1.11 -> 0.38 ms, 2D 128^2 3.69 -> 1.24, 1024 x 256 channel step 16.6 -> 10.6.
+// 1.32 -> 0.45 ms, 2D 128^2 3.73 -> 1.25, 1024 x 256 channel step 16.2 -> 9.6.  The
+// line lies where the two meet: 96^3 3.32 -> 3.10 ms (10.9 -> 9.3 with variable
+// density), 1024 x 768 19.7 -> 18.3, 1024^2 25.3 -> 23.6, 128 x 96 x 96 (1.2M cells)
+// 6.69 against 6.67.
 static bool resident(const ff_pressure ps) {
     return ps->resident_fits && ps->use_graph && cg_tma(ps) && ps->use_tail &&
            ps->desc.preconditioner == FF_PRE_MULTIGRID && ps->desc.mg_down > 0 && ps->desc.mg_final > 0 &&

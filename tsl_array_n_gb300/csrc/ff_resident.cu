@@ -837,6 +837,7 @@ __device__ __forceinline__ void held_coarse_in() {
 // cluster barrier (480 cycles) and a remote round trip (240) where a grid-wide
 // phase costs a grid barrier (3000) and L2 round trips.
 constexpr int CLUSTER_CELLS = 1 << 16;  // level spread over a cluster
+constexpr int CLUSTER_SOLVE_2D = 3 << 14;   // level 0 of a 2D solve on one cluster
 constexpr int BLOCK_CELLS = 2048;       // level held in one block of a cluster
 constexpr int CLUSTER_DIRECT = 384;     // unknowns of a direct coarsest solve on one cluster
 constexpr int ROW_WORDS = 8;
@@ -1358,6 +1359,161 @@ __device__ void low_up() {
     }
 }
 
+// ------------------------------------------------------------ dot products --
+// A thread's share of an item's sum: the products of its quad on the item's planes;
+// ld gives the four products of a quad.  `any`: whether any lane of the warp has
+// cells (a warp without adds exact zeros).
+template <class LD>
+__device__ __forceinline__ double item_share(const DotOrder &o, const Dims &d, int item, int tid, bool &any, LD ld) {
+    const int i = (item % o.gx) * DOT_TX + 4 * dot_quad(tid), j = ((item / o.gx) % o.gy) * DOT_TY + dot_row(tid);
+    const int k0 = (item / (o.gx * o.gy)) * o.zc, k1 = min(k0 + o.zc, d.nz);
+    const bool in = i < d.nx && j < d.ny;
+    Acc acc;
+    if (in)
+#pragma unroll 4
+        for (int k = k0; k < k1; ++k) {
+            const float4 v = ld(i, j, k);
+            acc.add(v.x);
+            acc.add(v.y);
+            acc.add(v.z);
+            acc.add(v.w);
+        }
+    any = __any_sync(0xffffffffu, in);
+    return any ? acc.value() : 0.0;
+}
+// the item's sum, in thread 0 of the DOT_THREADS threads of half `half` of the block
+__device__ __forceinline__ double item_sum(double v, bool any, int half) {
+    __shared__ double sred[NT / 32];
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 7;
+    const double w = any ? warp_sum(v) : 0.0;
+    bar_sync_n(2 + half, DOT_THREADS);   // (the last item's sums are read)
+    if (lane == 0) sred[8 * half + warp] = w;
+    bar_sync_n(2 + half, DOT_THREADS);
+    double t = 0.0;
+    if (warp == 0) {
+        // warp_sum over 32 lanes of which eight hold a sum
+        t = lane < 8 ? sred[8 * half + lane] : 0.0;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    }
+    return t;
+}
+// the items' sums added up, in warp 0
+template <class LD>
+__device__ __forceinline__ double items_total(int items, LD ld) {
+    __shared__ double sred[DOT_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (items <= 32) return tid < 32 ? warp_sum(lane < items ? ld(lane) : 0.0) : 0.0;
+    if (tid < DOT_THREADS) {
+        double s = 0.0;
+        for (int b = tid; b < items; b += DOT_THREADS) s += ld(b);
+        s = warp_sum(s);
+        if (lane == 0) sred[tid >> 5] = s;
+    }
+    __syncthreads();
+    double t = 0.0;
+    if (tid < 32) {
+        t = lane < DOT_THREADS / 32 ? sred[lane] : 0.0;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    }
+    __syncthreads();
+    return t;
+}
+// the barrier after the items' sums, and their totals in thread 0 of every block
+// (the dots have places of their own: a block may write the next one's sums while
+// another still reads the last one's)
+__device__ __noinline__ bool grid_total(int which, bool two, const double *partials, unsigned &passed, double &sum,
+                                        double &sum2) {
+    if (!grid_sync(SA.bar, passed)) return false;
+    const int items = SA.dot[which].items;
+    const double *at = partials + SA.dot[which].first;
+    sum = items_total(items, [&](int b) { return __ldcg(at + b); });
+    if (two) sum2 = items_total(items, [&](int b) { return __ldcg(at + items + b); });
+    return true;
+}
+// Grid-wide: the sum of the products q that the phase before left (q2: of another
+// set too), in thread 0 of every block, in the order of `which`.  Two barriers.
+__device__ __noinline__ bool grid_dot(int which, const float *q, const float *q2, double *partials, unsigned &passed,
+                                      double &sum, double &sum2) {
+    if (!grid_sync(SA.bar, passed)) return false;
+    const DotOrder o = SA.dot[which];
+    const Dims d = SA.lv[0].g.d;
+    const int half = threadIdx.x >> 8, tid = threadIdx.x & (DOT_THREADS - 1);
+    for (int item = blockIdx.x + half * gridDim.x; item < o.items; item += 2 * gridDim.x) {
+        for (int set = 0; set < (q2 ? 2 : 1); ++set) {
+            const float *src = set ? q2 : q;
+            bool any;
+            const double v = item_share(o, d, item, tid, any, [&](int i, int j, int k) {
+                return __ldcg(reinterpret_cast<const float4 *>(src + i + d.nx * (j + d.ny * k)));
+            });
+            const double t = item_sum(v, any, half);
+            if (tid == 0) partials[o.first + set * o.items + item] = t;
+        }
+    }
+    return grid_total(which, q2 != nullptr, partials, passed, sum, sum2);
+}
+
+
+// In 2D an item is one plane: its 256 threads have the quads of the phase itself,
+// and the sums need no products in memory and one barrier less.  (In 3D a thread
+// would march an item's planes, 16 cells or more each: 64^3 2.13 ms against 1.85,
+// 80^3 4.57 against 4.19; 2D 1024 x 768 18.9 against 20.4 for the products.)
+// quad(i, j, acc) adds up the products of the quad at (i, j).
+template <int SETS, class F>
+__device__ __forceinline__ void quad_items(int which, double *partials, F quad) {
+    const DotOrder o = SA.dot[which];
+    const Dims d = SA.lv[0].g.d;
+    const int half = threadIdx.x >> 8, tid = threadIdx.x & (DOT_THREADS - 1);
+    for (int item = blockIdx.x + half * gridDim.x; item < o.items; item += 2 * gridDim.x) {
+        const int i = (item % o.gx) * DOT_TX + 4 * dot_quad(tid), j = (item / o.gx) * DOT_TY + dot_row(tid);
+        const bool in = i < d.nx && j < d.ny, any = __any_sync(0xffffffffu, in);
+        Acc acc[SETS];
+        if (in) quad(i, j, acc);
+#pragma unroll
+        for (int q = 0; q < SETS; ++q) {
+            const double t = item_sum(any ? acc[q].value() : 0.0, any, half);
+            if (tid == 0) partials[o.first + q * o.items + item] = t;
+        }
+    }
+}
+__device__ __forceinline__ float4 ldcg4(const float *p) { return __ldcg(reinterpret_cast<const float4 *>(p)); }
+__device__ __forceinline__ void st4(float *p, const float4 &v) { *reinterpret_cast<float4 *>(p) = v; }
+__device__ __forceinline__ float at4(const float4 &v, int o) { return o == 0 ? v.x : o == 1 ? v.y : o == 2 ? v.z : v.w; }
+__device__ __forceinline__ unsigned quad_class(const RLevel &L, int i, int j) {
+    return __ldg(L.cls + L.cpitch * j + (i >> 2));
+}
+// 2D: the last colour pass of level 0 (colour 0), and the items' sums of r.z
+__device__ __noinline__ void quad_last_colour(int edge, double *partials) {
+    const RLevel L = SA.lv[0];
+    const Relax a = relax_of();
+    const int nx = L.g.d.nx, ny = L.g.d.ny;
+    float *x = L.x;
+    const float *alt = SA.alt;
+    quad_items<1>(2, partials, [&](int i, int j, Acc (&acc)[1]) {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int c = i + nx * j, P = j & 1, t = i & (DOT_TX - 1);   // cells P and P + 2 are of colour 0
+        const unsigned cb = quad_class(L, i, j);
+        const float4 bq = ldcg4(L.b + c), q = ldcg4(x + c);
+        const float4 ym = j > 0 ? ldcg4(x + c - nx) : zero, yp = j < ny - 1 ? ldcg4(x + c + nx) : zero;
+        float s = 0.f;   // the neighbour outside the quad
+        if (P == 0 && i > 0) s = __ldcg((edge == EDGE_USE && t == 0 ? alt : x) + c - 1);
+        if (P == 1 && i + 4 < nx) s = __ldcg((edge == EDGE_USE && t == DOT_TX - 4 ? alt : x) + c + 4);
+        const unsigned cl0 = cb >> (2 * P) & 3u, cl1 = cb >> (2 * P + 4) & 3u;
+        const bool pair = (cl0 | cl1) & 1u;
+        const float n0 = relax_cell<false>(a, L, cl0, c + P, i + P, j, 0, P ? q.y : q.x, P ? q.x : s, P ? q.z : q.y,
+                                           P ? ym.y : ym.x, P ? yp.y : yp.x, 0.f, 0.f, P ? bq.y : bq.x, pair);
+        const float n1 = relax_cell<false>(a, L, cl1, c + P + 2, i + P + 2, j, 0, P ? q.w : q.z, P ? q.z : q.y,
+                                           P ? s : q.w, P ? ym.w : ym.z, P ? yp.w : yp.z, 0.f, 0.f, P ? bq.w : bq.z, pair);
+        x[c + P] = n0;
+        x[c + P + 2] = n1;
+        acc[0].add(bq.x * (P ? q.x : n0));
+        acc[0].add(bq.y * (P ? n0 : q.y));
+        acc[0].add(bq.z * (P ? q.z : n1));
+        acc[0].add(bq.w * (P ? n1 : q.w));
+    });
+}
+
 // ---------------------------------------------------------------- V-cycle --
 // block 0, the first level below the grid-wide ones: its b from global memory, or
 // its x back there
@@ -1377,11 +1533,12 @@ __device__ __noinline__ void tier_copy(int l, bool in) {
 }
 
 // z = M r on lv[0] (x = z, b = r).  first_done: the caller made the first
-// colour-0 pass.  RZ: the last pass leaves the products of r.z in lv[0].r (lv[0]
-// is one of the grid-wide levels).  The caller takes the last barrier.  Every block takes the same sequence of barriers
+// colour-0 pass.  RZ: the last pass leaves the products of r.z in lv[0].r, in 2D
+// the items' sums (lv[0] is one of the grid-wide levels).  The caller takes the last
+// barrier.  Every block takes the same sequence of barriers
 // (it depends only on the levels).  False when a barrier gave up.
 template <bool D3, bool RZ>
-__device__ bool vcycle(unsigned &passed, bool first_done) {
+__device__ bool vcycle(unsigned &passed, bool first_done, double *partials) {
     const int nl = SA.nl, clu = SA.clu, down = SA.down, sweeps = SA.coarse_sweeps, nc = (int)SA.lv[nl - 1].g.d.n();
     unsigned *bar = SA.bar;
     const bool low = blockIdx.x == 0;   // this block has the levels from clu down
@@ -1439,8 +1596,12 @@ __device__ bool vcycle(unsigned &passed, bool first_done) {
             if (!grid_sync(bar, passed)) return false;
             g_colour<D3, false>(l, 1, false, keep);
             if (!grid_sync(bar, passed)) return false;
-            if (RZ && l == 0 && it == up - 1) g_colour<D3, true>(l, 0, false, use);
-            else g_colour<D3, false>(l, 0, false, use);
+            if (RZ && l == 0 && it == up - 1) {
+                if (D3) g_colour<D3, true>(l, 0, false, use);
+                else quad_last_colour(use, partials);
+            } else {
+                g_colour<D3, false>(l, 0, false, use);
+            }
         }
     }
     return true;
@@ -1461,7 +1622,7 @@ __global__ void __launch_bounds__(NT, 1) k_vcycle_tail(const __grid_constant__ V
     unsigned passed = 0;
     load_args(a);
     if (blockIdx.x == 0) low_init<D3, false>();
-    if (vcycle<D3, false>(passed, false)) grid_done(SA.bar);
+    if (vcycle<D3, false>(passed, false, nullptr)) grid_done(SA.bar);
     else if (threadIdx.x == 0 && st) atomicOr(&st->err, 2);
 }
 
@@ -1482,7 +1643,7 @@ constexpr double MAX_RESIDUAL_GROWTH = 100.0;   // linalg.js:1095
 struct PcgArgs {
     const float *b;                // right-hand side
     float *p[2], *xh[2], *xl[2];   // search direction and iterate, ping-pong
-    double *partials;              // 8 sums of gridDim.x partials
+    double *partials;              // the work items' sums
     PcgState *st;
 };
 
@@ -1551,91 +1712,6 @@ __device__ void after_solve(PcgState &S) {
     if (S.maxiter <= 0) return;
     S.last_iters = S.stop == FF_STOP_CONVERGED ? S.stop_iter : S.iter;
     S.last_valid = 1;
-}
-
-// A thread's share of an item's sum: the products of its quad on the item's planes;
-// ld gives the four products of a quad.  `any`: whether any lane of the warp has
-// cells (a warp without adds exact zeros).
-template <class LD>
-__device__ __forceinline__ double item_share(const DotOrder &o, const Dims &d, int item, int tid, bool &any, LD ld) {
-    const int i = (item % o.gx) * DOT_TX + 4 * dot_quad(tid), j = ((item / o.gx) % o.gy) * DOT_TY + dot_row(tid);
-    const int k0 = (item / (o.gx * o.gy)) * o.zc, k1 = min(k0 + o.zc, d.nz);
-    const bool in = i < d.nx && j < d.ny;
-    Acc acc;
-    if (in)
-#pragma unroll 4
-        for (int k = k0; k < k1; ++k) {
-            const float4 v = ld(i, j, k);
-            acc.add(v.x);
-            acc.add(v.y);
-            acc.add(v.z);
-            acc.add(v.w);
-        }
-    any = __any_sync(0xffffffffu, in);
-    return any ? acc.value() : 0.0;
-}
-// the item's sum, in thread 0 of the DOT_THREADS threads of half `half` of the block
-__device__ __forceinline__ double item_sum(double v, bool any, int half) {
-    __shared__ double sred[NT / 32];
-    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 7;
-    const double w = any ? warp_sum(v) : 0.0;
-    bar_sync_n(2 + half, DOT_THREADS);   // (the last item's sums are read)
-    if (lane == 0) sred[8 * half + warp] = w;
-    bar_sync_n(2 + half, DOT_THREADS);
-    double t = 0.0;
-    if (warp == 0) {
-        // warp_sum over 32 lanes of which eight hold a sum
-        t = lane < 8 ? sred[8 * half + lane] : 0.0;
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    }
-    return t;
-}
-// the items' sums added up, in warp 0
-template <class LD>
-__device__ __forceinline__ double items_total(int items, LD ld) {
-    __shared__ double sred[DOT_THREADS / 32];
-    const int tid = threadIdx.x, lane = tid & 31;
-    if (items <= 32) return tid < 32 ? warp_sum(lane < items ? ld(lane) : 0.0) : 0.0;
-    if (tid < DOT_THREADS) {
-        double s = 0.0;
-        for (int b = tid; b < items; b += DOT_THREADS) s += ld(b);
-        s = warp_sum(s);
-        if (lane == 0) sred[tid >> 5] = s;
-    }
-    __syncthreads();
-    double t = 0.0;
-    if (tid < 32) {
-        t = lane < DOT_THREADS / 32 ? sred[lane] : 0.0;
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    }
-    __syncthreads();
-    return t;
-}
-// Grid-wide: the sum of the products q that the phase before left (q2: of another
-// set too), in thread 0 of every block, in the order of `which`.  Two barriers.
-__device__ __noinline__ bool grid_dot(int which, const float *q, const float *q2, double *partials, unsigned &passed,
-                                      double &sum, double &sum2) {
-    if (!grid_sync(SA.bar, passed)) return false;
-    const DotOrder o = SA.dot[which];
-    const Dims d = SA.lv[0].g.d;
-    const int half = threadIdx.x >> 8, tid = threadIdx.x & (DOT_THREADS - 1);
-    for (int item = blockIdx.x + half * gridDim.x; item < o.items; item += 2 * gridDim.x) {
-        for (int set = 0; set < (q2 ? 2 : 1); ++set) {
-            const float *src = set ? q2 : q;
-            bool any;
-            const double v = item_share(o, d, item, tid, any, [&](int i, int j, int k) {
-                return __ldcg(reinterpret_cast<const float4 *>(src + i + d.nx * (j + d.ny * k)));
-            });
-            const double t = item_sum(v, any, half);
-            if (tid == 0) partials[set * o.items + item] = t;
-        }
-    }
-    if (!grid_sync(SA.bar, passed)) return false;
-    sum = items_total(o.items, [&](int b) { return __ldcg(partials + b); });
-    if (q2) sum2 = items_total(o.items, [&](int b) { return __ldcg(partials + o.items + b); });
-    return true;
 }
 
 // p = z + beta p (FIRST: z itself); leaves p Ap in lv[0].r.
@@ -1709,6 +1785,103 @@ __device__ __noinline__ void pcg_x(const float *b, const float *xh, const float 
     }
 }
 
+// The 2D forms of pcg_p and pcg_x: a thread has an x-quad, and the items' sums come
+// out of the phase.  A neighbour across the domain edge is any finite value.
+template <bool FIRST>
+__device__ __noinline__ void quad_p(const float *pold, float *pnew, float beta, double *partials) {
+    const RLevel L = SA.lv[0];
+    const int nx = L.g.d.nx, ny = L.g.d.ny;
+    const float *z = L.x;
+    auto P1 = [&](int c) {
+        const float zc = __ldcg(z + c);
+        return FIRST ? zc : __fmaf_rn(beta, __ldcg(pold + c), zc);
+    };
+    auto P4 = [&](int c) {
+        const float4 zq = ldcg4(z + c);
+        if (FIRST) return zq;
+        const float4 q = ldcg4(pold + c);
+        return make_float4(__fmaf_rn(beta, q.x, zq.x), __fmaf_rn(beta, q.y, zq.y), __fmaf_rn(beta, q.z, zq.z),
+                           __fmaf_rn(beta, q.w, zq.w));
+    };
+    quad_items<1>(0, partials, [&](int i, int j, Acc (&acc)[1]) {
+        const int c = i + nx * j;
+        const unsigned cb = quad_class(L, i, j);
+        const float4 q = P4(c), ym = P4(j > 0 ? c - nx : c), yp = P4(j < ny - 1 ? c + nx : c);
+        const float xl = P1(i > 0 ? c - 1 : c), xr = P1(i + 4 < nx ? c + 4 : c + 3);
+        st4(pnew + c, q);
+        auto add = [&](int o, float pc, float xm, float xp) {
+            const float v = ap_cell(L.g, L.coef, L.gco, cb >> (2 * o) & 3u, i + o, j, 0, c + o, pc, xm, xp, at4(ym, o),
+                                    at4(yp, o), pc, pc);
+            acc[0].add(pc * v);
+        };
+        add(0, q.x, xl, q.y);
+        add(1, q.y, q.x, q.z);
+        add(2, q.z, q.y, q.w);
+        add(3, q.w, q.z, xr);
+    });
+}
+template <bool DS, bool SETUP>
+__device__ __noinline__ void quad_x(const float *b, const float *xh, const float *xl, const float *p, float *oh, float *ol,
+                                    double alpha, double *partials) {
+    const RLevel L = SA.lv[0];
+    const Relax a = relax_of();
+    const int nx = L.g.d.nx, ny = L.g.d.ny;
+    const float ahi = (float)alpha, alo = (float)(alpha - (double)ahi);
+    struct Quad {
+        float4 h, l;
+    };
+    auto form = [&](float pv, float &h, float &l) {
+        if (DS) ds_axpy(h, l, ahi, alo, pv, h, l);
+        else h = __fmaf_rn(ahi, pv, h);
+    };
+    auto X1 = [&](int c, float &h, float &l) {
+        h = __ldcg(xh + c);
+        l = DS ? __ldcg(xl + c) : 0.f;
+        if (!SETUP) form(__ldcg(p + c), h, l);
+    };
+    auto X4 = [&](int c) {
+        Quad q{ldcg4(xh + c), DS ? ldcg4(xl + c) : make_float4(0.f, 0.f, 0.f, 0.f)};
+        if (!SETUP) {
+            const float4 pv = ldcg4(p + c);
+            form(pv.x, q.h.x, q.l.x);
+            form(pv.y, q.h.y, q.l.y);
+            form(pv.z, q.h.z, q.l.z);
+            form(pv.w, q.h.w, q.l.w);
+        }
+        return q;
+    };
+    quad_items<SETUP ? 2 : 1>(1, partials, [&](int i, int j, Acc (&acc)[SETUP ? 2 : 1]) {
+        const int c = i + nx * j;
+        const unsigned cb = quad_class(L, i, j);
+        const float4 bq = __ldg(reinterpret_cast<const float4 *>(b + c));
+        const Quad q = X4(c), ym = X4(j > 0 ? c - nx : c), yp = X4(j < ny - 1 ? c + nx : c);
+        float xlh, xll, xrh, xrl;
+        X1(i > 0 ? c - 1 : c, xlh, xll);
+        X1(i + 4 < nx ? c + 4 : c + 3, xrh, xrl);
+        if (!SETUP) {
+            st4(oh + c, q.h);
+            if (DS) st4(ol + c, q.l);
+        }
+        auto res = [&](int o, float bc, float h, float l, float xmh, float xml, float xph, float xpl) {
+            const float r = resid_by_class<DS>(L.g, cb >> (2 * o) & 3u, i + o, j, 0, bc, h, l, xmh, xml, xph, xpl,
+                                               at4(ym.h, o), at4(ym.l, o), at4(yp.h, o), at4(yp.l, o), h, l, h, l,
+                                               [&] { return general_coef(L.coef, L.gco, i + o, j, 0, c + o); });
+            acc[0].add(r * r);
+            if (SETUP) acc[SETUP ? 1 : 0].add(bc * bc);
+            return r;
+        };
+        float4 r;
+        r.x = res(0, bq.x, q.h.x, q.l.x, xlh, xll, q.h.y, q.l.y);
+        r.y = res(1, bq.y, q.h.y, q.l.y, q.h.x, q.l.x, q.h.z, q.l.z);
+        r.z = res(2, bq.z, q.h.z, q.l.z, q.h.y, q.l.y, q.h.w, q.l.w);
+        r.w = res(3, bq.w, q.h.w, q.l.w, q.h.z, q.l.z, xrh, xrl);
+        st4(L.b + c, r);
+        auto first = [&](int o, float rc) { return relax_zero<false>(a, L, cb >> (2 * o) & 3u, c + o, i + o, j, 0, rc); };
+        st4(L.x + c, j & 1 ? make_float4(0.f, first(1, r.y), 0.f, first(3, r.w))
+                           : make_float4(first(0, r.x), 0.f, first(2, r.z), 0.f));
+    });
+}
+
 template <bool D3, bool DS>
 __global__ void __launch_bounds__(NT, 1) k_pcg_resident(const __grid_constant__ VArgs a, const __grid_constant__ PcgArgs A) {
     __shared__ PcgState S;
@@ -1718,44 +1891,55 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(const __grid_constant__ 
     if (blockIdx.x == 0) low_init<D3, false>();
     bool ok = true;
     double sum = 0.0, sum2 = 0.0;
-    auto x_phase = [&](auto setup) {
-        const int c = S.x_cur;
-        pcg_x<D3, DS, decltype(setup)::value>(A.b, c ? A.xh[1] : A.xh[0], c ? A.xl[1] : A.xl[0],
-                                              S.p_cur ? A.p[1] : A.p[0], c ? A.xh[0] : A.xh[1],
-                                              c ? A.xl[0] : A.xl[1], S.alpha, A.p[0]);
+    const float *products = a.lv[0].r;
+    // a phase and its sum (3D: the phase leaves products; 2D: the items' sums)
+    auto total = [&](int which, const float *second = nullptr) {
+        if constexpr (D3) return grid_dot(which, products, second, A.partials, passed, sum, sum2);
+        else return grid_total(which, second != nullptr, A.partials, passed, sum, sum2);
     };
-    const float *q = a.lv[0].r;
+    auto x_phase = [&](auto setup) {
+        constexpr bool SETUP = decltype(setup)::value;
+        const int c = S.x_cur;
+        const float *xh = c ? A.xh[1] : A.xh[0], *xl = c ? A.xl[1] : A.xl[0], *p = S.p_cur ? A.p[1] : A.p[0];
+        float *oh = c ? A.xh[0] : A.xh[1], *ol = c ? A.xl[0] : A.xl[1];
+        if constexpr (D3) pcg_x<D3, DS, SETUP>(A.b, xh, xl, p, oh, ol, S.alpha, A.p[0]);
+        else quad_x<DS, SETUP>(A.b, xh, xl, p, oh, ol, S.alpha, A.partials);
+        return total(1, SETUP ? A.p[0] : nullptr);
+    };
+    auto p_phase = [&](auto first) {
+        constexpr bool FIRST = decltype(first)::value;
+        const float *po = S.p_cur ? A.p[1] : A.p[0];
+        const float beta = FIRST ? 0.f : (float)S.beta;
+        float *pn = S.p_cur ? A.p[0] : A.p[1];
+        if constexpr (D3) pcg_p<D3, FIRST>(po, pn, beta);
+        else quad_p<FIRST>(po, pn, beta, A.partials);
+        return total(0);
+    };
     // setup (linalg.js:1627-1637): r = b - A x, its norm and b's, z = M r, r.z
-    x_phase(std::true_type());
-    ok = grid_dot(1, q, A.p[0], A.partials, passed, sum, sum2);
+    ok = x_phase(std::true_type());
     if (ok && threadIdx.x == 0) after_setup(S, sum, sum2);
     __syncthreads();
     if (ok && S.stop == 0) {
-        ok = vcycle<D3, true>(passed, true) && grid_dot(2, q, nullptr, A.partials, passed, sum, sum2);
+        ok = vcycle<D3, true>(passed, true, A.partials) && total(2);
         if (ok && threadIdx.x == 0) after_first_rz(S, sum);
         __syncthreads();
     }
     while (ok && S.stop == 0 && S.iter < S.maxiter) {
-        const float *po = S.p_cur ? A.p[1] : A.p[0];
-        float *pn = S.p_cur ? A.p[0] : A.p[1];
-        if (S.first) pcg_p<D3, true>(po, pn, 0.f);
-        else pcg_p<D3, false>(po, pn, (float)S.beta);
-        if (!(ok = grid_dot(0, q, nullptr, A.partials, passed, sum, sum2))) break;
+        if (!(ok = S.first ? p_phase(std::true_type()) : p_phase(std::false_type()))) break;
         if (threadIdx.x == 0) {
             after_pap(S, sum);
             S.p_cur ^= 1;
         }
         __syncthreads();
         if (S.stop) break;
-        x_phase(std::false_type());
-        if (!(ok = grid_dot(1, q, nullptr, A.partials, passed, sum, sum2))) break;
+        if (!(ok = x_phase(std::false_type()))) break;
         if (threadIdx.x == 0) {
             S.x_cur ^= 1;
             after_rr(S, sum);
         }
         __syncthreads();
         if (S.stop) break;
-        if (!(ok = vcycle<D3, true>(passed, true) && grid_dot(2, q, nullptr, A.partials, passed, sum, sum2))) break;
+        if (!(ok = vcycle<D3, true>(passed, true, A.partials) && total(2))) break;
         if (threadIdx.x == 0) after_rz(S, sum);
         __syncthreads();
     }
@@ -1773,9 +1957,10 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(const __grid_constant__ 
 // phase of one pair a thread takes about 1100 cycles with its barrier, where a
 // grid-wide one takes 5000; a dot product 3000 to 4000 (FP64 runs at two lanes a
 // clock here), the coarsest level's 40 passes in one block 8000 to 13000.
-// Whole projections, over the grid and here: 48 x 32 x 32 0.91 and 0.72 ms, 192 x 128
-// 2.50 and 1.85.  The line, CLUSTER_CELLS, lies where both meet (64 x 32 x 32 0.81
-// and 0.78, 256^2 3.65 and 3.80) and where the arrays still fit.
+// Whole projections, over the grid and here: 48 x 32 x 32 0.91 and 0.72 ms, 64 x 32 x
+// 24 1.18 and 1.04, 192 x 128 2.43 and 1.85.  The line lies where both meet (64 x 32 x
+// 32 0.83 and 0.77; 256 x 192 3.66 and 3.41, 256^2 3.52 and 3.78) and where the arrays
+// still fit.
 // A cluster in a launch over the whole GPU, for the lower levels of larger solves,
 // was slower: 8 blocks a cluster leave 120 of 152 SMs to the grid-wide phases, and a
 // spread phase of eight pairs a thread takes as long as a grid-wide one.
@@ -2098,6 +2283,7 @@ VArgs make_args(const Level *lv, const SweepMaps *sm, int nl, int dims, int down
         o.gy = (d.ny + DOT_TY - 1) / DOT_TY;
         o.zc = zc;
         o.items = o.gx * o.gy * ((d.nz + zc - 1) / zc);
+        o.first = w == 0 ? 0 : a.dot[w - 1].first + w * a.dot[w - 1].items;   // (r.r comes with b.b)
     }
     a.pairs = solver;
     smem = place(a, dims == 3, solver);
@@ -2186,7 +2372,7 @@ int pcg_resident(const Level *lv, const SweepMaps *sm, int nl, int dims, int dow
     VArgs a;
     void *args[] = {&a, &A};
     // on one cluster, if level 0 fits it
-    if (cluster > 0 && lv[0].d.n() <= CLUSTER_CELLS && (coarse_sweeps > 0 || nG <= CLUSTER_DIRECT)) {
+    if (cluster > 0 && lv[0].d.n() <= (dims == 3 ? CLUSTER_CELLS : CLUSTER_SOLVE_2D) && (coarse_sweeps > 0 || nG <= CLUSTER_DIRECT)) {
         a = make_args(lv, sm, nl, dims, down, up, fin, sor, G, nG, coarse_sweeps, bar, cluster, true, sm_count, smem);
         const void *k = dims == 3 ? (ds ? (const void *)k_pcg_cluster<true, true> : (const void *)k_pcg_cluster<true, false>)
                                   : (ds ? (const void *)k_pcg_cluster<false, true> : (const void *)k_pcg_cluster<false, false>);

@@ -234,6 +234,7 @@ __device__ __forceinline__ float resid_cell(const Geo &g, const float4 *coef, co
 constexpr int DOT_TX = 64, DOT_TY = 16, DOT_THREADS = 256;
 struct DotOrder {
     int gx, gy, zc, items;
+    int first;   // place of the items' sums among the solver's
 };
 // quad and row in its tile of a thread of an item
 __device__ __forceinline__ int dot_quad(int tid) { return tid & (DOT_TX / 4 - 1); }
