@@ -147,7 +147,9 @@ __global__ void __launch_bounds__(256) k_fold_list(FaceLists L) {
 // on one plane, whose taps share rows in L1 (a run of 256 faces of one row reads
 // four times the lines), and the last columns, fewer than 32, as runs over (x, y).
 struct TileMap {
-    int sx, sy, tiles_x, full, edge;   // full tiles a row of them, full and edge blocks a plane
+    int sx, sy, tiles_x, full;   // full tiles a row of them and a plane
+    __host__ __device__ TileMap(int x, int y) : sx(x), sy(y), tiles_x(x / 32), full(x / 32 * ((y + 7) / 8)) {}
+    int blocks() const { return full + (int)(((long long)(sx - 32 * tiles_x) * sy + 255) / 256); }
     __device__ __forceinline__ bool at(int &i, int &j) const {
         const int t = threadIdx.x;
         if ((int)blockIdx.x < full) {
@@ -156,56 +158,61 @@ struct TileMap {
             return j < sy;
         }
         const unsigned w = (unsigned)(sx - 32 * tiles_x), e = (blockIdx.x - full) * 256u + t;
+        if (w == 0) return false;
         i = 32 * tiles_x + (int)(e % w);
         j = (int)(e / w);
         return j < sy;
     }
 };
-TileMap tile_map(int sx, int sy) {
-    TileMap m{sx, sy, sx / 32, 0, 0};
-    m.full = m.tiles_x * ((sy + 7) / 8);
-    m.edge = (int)(((long long)(sx - 32 * m.tiles_x) * sy + 255) / 256);
-    return m;
-}
 
-// Advection stages on one component (a = 0..2 faces, 3 cell scalar):
+// Advection stages, blockIdx.y a component (three faces, or one cell scalar):
 //   0 order 1: out = cubic(src @ trace(+1)) where the position is open
 //   1 MacCormack forward:  aux = open ? cubic(src @ trace(+1)) : src
 //   2 MacCormack backward: aux = open ? cubic(fwd @ trace(-1)) : fwd
 //   3 MacCormack correct:  out = clamp(fwd + (src - bwd)/2) where open
 // (one kernel per stage: a smaller body for the instruction cache).
-// Bound by issue (78% of the slots, 2100 instructions a face at two to three
-// substeps; DRAM 4%): order 1 on the 16.8M faces of one component of a 256^3 grid
-// takes 1.08 ms, 1.55 ms in the straightforward form.  Of that 0.1 ms is the
-// short form itself; the rest came with one copy of the trace's sample and of the
-// tricubic's plane pair in the code (a third of all issue slots had waited for
-// instructions), arguments read in place instead of from a local copy, and floor
-// as an addition.
-template <int stage, bool P2>
-__global__ void __launch_bounds__(256) k_advect(const __grid_constant__ VelField F, int a, TileMap map, const float *__restrict__ src,
-                                                const float *__restrict__ fwd, const float *__restrict__ bwd,
-                                                float *__restrict__ out, float dt, int max_substeps, int z0) {
-    int sx, sy, sz;
-    if (a < 3) comp_shape(F.g, a, sx, sy, sz);
-    else sx = F.g.nx, sy = F.g.ny, sz = F.g.nz;
-    const F3 o = comp_origin(F.g, a);
-    int i, j;
-    if (!map.at(i, j)) return;
-    const int k = z0 + (int)blockIdx.z;
-    const int f = i + sx * (j + sy * k);
+struct AdvectIO {
+    const float *src[3], *fwd[3], *bwd[3];
+    float *out[3];
+};
+// FORM: the straightforward form of the trace and the samples, or the short one
+enum { ADVECT_PLAIN, ADVECT_SHORT, ADVECT_SHORT_P2 };
+template <int FORM>
+__device__ __forceinline__ float advect_phi(const VelField &F, F3 p) {
+    if constexpr (FORM == ADVECT_PLAIN) return sample_phi(F, F.phi, p);
+    else return trace_phi<FORM == ADVECT_SHORT_P2>(F, p);
+}
+template <int FORM>
+__device__ __forceinline__ F3 advect_trace(const VelField &F, F3 pos, float dt, float dirn, int max_substeps, float phi) {
+    if constexpr (FORM == ADVECT_PLAIN) return back_trace_plain(F, pos, dt, dirn, max_substeps);
+    else return back_trace<FORM == ADVECT_SHORT_P2>(F, pos, dt, dirn, max_substeps, phi);
+}
+template <int FORM>
+__device__ __forceinline__ float advect_cubic(const VelField &F, int a, const float *d, int sx, int sy, int sz, F3 o, F3 p) {
+    if constexpr (FORM == ADVECT_PLAIN) return tricubic(d, sx, sy, sz, F.g, o, p);
+    else return trace_cubic<FORM == ADVECT_SHORT_P2>(F, a, d, sx, sy, sz, o, p);
+}
+template <int stage, int FORM>
+__device__ __forceinline__ void advect_at(const VelField &F, int a, const AdvectIO &io, int q, int sx, int sy, int sz, F3 o,
+                                          long long f, int i, int j, int k, float dt, int max_substeps) {
+    const float *src = io.src[q], *fwd = io.fwd[q], *bwd = io.bwd[q];
+    float *out = io.out[q];
     const F3 pos = index_pos(F.g, o, i, j, k);
-    const float phi = trace_phi<P2>(F, pos);
+    const float phi = advect_phi<FORM>(F, pos);
     const bool open = phi > 0.0f;
+    auto traced = [&](const float *d, float dirn) {
+        return advect_cubic<FORM>(F, a, d, sx, sy, sz, o, advect_trace<FORM>(F, pos, dt, dirn, max_substeps, phi));
+    };
     if constexpr (stage == 0) {
-        if (open) out[f] = trace_cubic<P2>(F, a, src, sx, sy, sz, o, back_trace<P2>(F, pos, dt, 1.0f, max_substeps, phi));
+        if (open) out[f] = traced(src, 1.0f);
     } else if constexpr (stage == 1) {
-        out[f] = open ? trace_cubic<P2>(F, a, src, sx, sy, sz, o, back_trace<P2>(F, pos, dt, 1.0f, max_substeps, phi)) : src[f];
+        out[f] = open ? traced(src, 1.0f) : src[f];
     } else if constexpr (stage == 2) {
-        out[f] = open ? trace_cubic<P2>(F, a, fwd, sx, sy, sz, o, back_trace<P2>(F, pos, dt, -1.0f, max_substeps, phi)) : fwd[f];
+        out[f] = open ? traced(fwd, -1.0f) : fwd[f];
     } else if (open) {
         // clampCorrection (stage 3): min/max over the 8 trilinear corners of the
         // traced point whose own positions are open
-        const F3 tr = back_trace<P2>(F, pos, dt, 1.0f, max_substeps, phi);
+        const F3 tr = advect_trace<FORM>(F, pos, dt, 1.0f, max_substeps, phi);
         const float fv = fwd[f];
         const float corr = fv + (src[f] - bwd[f]) * 0.5f;
         const float gx = gclamp((tr.x - o.x) / F.g.hx), gy = gclamp((tr.y - o.y) / F.g.hy),
@@ -216,18 +223,63 @@ __global__ void __launch_bounds__(256) k_advect(const __grid_constant__ VelField
         const int kc[2] = {iclamp(k0, 0, sz - 1), iclamp(k0 + 1, 0, sz - 1)};
         float mn = 1e30f, mx = -1e30f;
         bool have = false;
-#pragma unroll 1
-        for (int c = 0; c < 8; ++c) {
+        auto corner = [&](int c) {
             const int ni = ic[c & 1], nj = jc[(c >> 1) & 1], nk = kc[(c >> 2) & 1];
-            const bool valid = trace_phi<P2>(F, index_pos(F.g, o, ni, nj, nk)) > 0.0f;
-            const float val = src[ni + sx * (nj + sy * nk)];
+            const bool valid = advect_phi<FORM>(F, index_pos(F.g, o, ni, nj, nk)) > 0.0f;
+            const float val = src[ni + (long long)sx * (nj + (long long)sy * nk)];
             if (valid) {
                 mn = fminf(mn, val);
                 mx = fmaxf(mx, val);
                 have = true;
             }
+        };
+        if constexpr (FORM == ADVECT_PLAIN) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) corner(c);
+        } else {
+#pragma unroll 1
+            for (int c = 0; c < 8; ++c) corner(c);
         }
         out[f] = (have && corr >= mn && corr <= mx) ? corr : fv;
+    }
+}
+// The short form: bound by issue (78% of the slots, 2100 instructions a face at two to
+// three substeps; DRAM 4%): order 1 on the 16.8M faces of one component of a 256^3
+// grid takes 1.08 ms, 1.55 ms in the straightforward form.  Of that 0.1 ms is the
+// short form itself; the rest came with one copy of the trace's sample and of the
+// tricubic's plane pair in the code (a third of all issue slots had waited for
+// instructions), arguments read in place instead of from a local copy, and floor
+// as an addition.
+template <int stage, int FORM>
+__global__ void __launch_bounds__(256) k_advect(const __grid_constant__ VelField F, int a0, const __grid_constant__ AdvectIO io,
+                                                float dt, int max_substeps, int z0) {
+    const int a = a0 + (int)blockIdx.y, k = z0 + (int)blockIdx.z;
+    int sx, sy, sz, i, j;
+    if (a < 3) comp_shape(F.g, a, sx, sy, sz);
+    else sx = F.g.nx, sy = F.g.ny, sz = F.g.nz;
+    if (k >= sz || !TileMap(sx, sy).at(i, j)) return;
+    advect_at<stage, FORM>(F, a, io, blockIdx.y, sx, sy, sz, comp_origin(F.g, a), i + (long long)sx * (j + (long long)sy * k), i,
+                           j, k, dt, max_substeps);
+}
+// The straightforward form, runs of 256 faces, below ADVECT_SHORT_CELLS cells: there
+// most warps touch an end of the arrays, where the short form only adds to this one,
+// and a small grid is bound by one warp's latency, which the short form's loops
+// lengthen.  Order 1, all faces, this form and the short one: 33 x 43 x 49 32 and 41 us
+// (43 with a launch a component), 64^3 91 and 92, 65 x 54 x 203 230 and 250, 96^3 273
+// and 273, 128 x 96 x 96 363 and 331, 128^3 627 and 490, 200^3 2301 and 1659.
+constexpr long long ADVECT_SHORT_CELLS = 1LL << 20;
+template <int stage>
+__global__ void k_advect_plain(const __grid_constant__ VelField F, int a0, const __grid_constant__ AdvectIO io, float dt,
+                               int max_substeps) {
+    const int a = a0 + (int)blockIdx.y;
+    int sx, sy, sz, i, j, k;
+    if (a < 3) comp_shape(F.g, a, sx, sy, sz);
+    else sx = F.g.nx, sy = F.g.ny, sz = F.g.nz;
+    const long long n = (long long)sx * sy * sz;
+    const F3 o = comp_origin(F.g, a);
+    for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < n; f += (long long)gridDim.x * blockDim.x) {
+        unflatten(f, sx, sy, i, j, k);
+        advect_at<stage, ADVECT_PLAIN>(F, a, io, blockIdx.y, sx, sy, sz, o, f, i, j, k, dt, max_substeps);
     }
 }
 
@@ -525,30 +577,53 @@ extern "C" int ff_advect3_set_collider(ff_advect a, ff_field phi) {
     return FF_OK;
 }
 
-static int advect_component(ff_advect a, const VelField &F, int c, const float *src, float *out) {
+// components a0 .. a0 + na - 1, one launch a stage
+static int advect_components(ff_advect a, const VelField &F, int a0, int na, const float *const *src, float *const *out) {
     cudaStream_t s = a->ctx->stream;
-    int sx, sy, sz;
-    if (c < 3) comp_shape(a->g, c, sx, sy, sz);
-    else sx = a->g.nx, sy = a->g.ny, sz = a->g.nz;
-    const TileMap map = tile_map(sx, sy);
     const float dt = (float)a->desc.dt;
     const int ms = a->desc.max_substeps;
-    // a launch per stage and 65535 planes
-    auto run = [&](auto stage, const float *fwd, const float *bwd, float *o) {
+    const long long cells = (long long)a->g.nx * a->g.ny * a->g.nz;
+    long long n = 0;
+    int planes = 0, blocks = 0;
+    AdvectIO io{};
+    for (int q = 0; q < na; ++q) {
+        const int c = a0 + q;
+        int sx = a->g.nx, sy = a->g.ny, sz = a->g.nz;
+        if (c < 3) comp_shape(a->g, c, sx, sy, sz);
+        n = std::max(n, (long long)sx * sy * sz);
+        planes = std::max(planes, sz);
+        blocks = std::max(blocks, TileMap(sx, sy).blocks());
+        io.src[q] = src[q];
+    }
+    auto run = [&](auto stage, float *const *to) {
         constexpr int st = decltype(stage)::value;
-        const auto kernel = F.pow2 ? k_advect<st, true> : k_advect<st, false>;
-        for (int z0 = 0; z0 < sz; z0 += 65535)
-            kernel<<<dim3((unsigned)(map.full + map.edge), 1, (unsigned)std::min(65535, sz - z0)), 256, 0, s>>>(
-                F, c, map, src, fwd, bwd, o, dt, ms, z0);
+        for (int q = 0; q < na; ++q) {
+            io.fwd[q] = a->fwd[a0 + q];
+            io.bwd[q] = a->bwd[a0 + q];
+            io.out[q] = to[q];
+        }
+        if (cells < ADVECT_SHORT_CELLS) {
+            k_advect_plain<st><<<dim3((unsigned)launch_blocks(n), (unsigned)na), 256, 0, s>>>(F, a0, io, dt, ms);
+            return;
+        }
+        const auto kernel = F.pow2 ? k_advect<st, ADVECT_SHORT_P2> : k_advect<st, ADVECT_SHORT>;
+        for (int z0 = 0; z0 < planes; z0 += 65535)
+            kernel<<<dim3((unsigned)blocks, (unsigned)na, (unsigned)std::min(65535, planes - z0)), 256, 0, s>>>(F, a0, io, dt,
+                                                                                                              ms, z0);
     };
     if (a->desc.order == 1) {
-        run(std::integral_constant<int, 0>(), nullptr, nullptr, out);
+        run(std::integral_constant<int, 0>(), out);
         return post("advect");
     }
-    run(std::integral_constant<int, 1>(), nullptr, nullptr, a->fwd[c]);
-    run(std::integral_constant<int, 2>(), a->fwd[c], nullptr, a->bwd[c]);
-    run(std::integral_constant<int, 3>(), a->fwd[c], a->bwd[c], out);
+    run(std::integral_constant<int, 1>(), a->fwd + a0);
+    run(std::integral_constant<int, 2>(), a->bwd + a0);
+    run(std::integral_constant<int, 3>(), out);
     return post("advect (MacCormack)");
+}
+
+static bool overlap(ff_field a, ff_field b) {
+    const char *p = (const char *)a->d, *q = (const char *)b->d;
+    return p < q + b->bytes && q < p + a->bytes;
 }
 
 extern "C" int ff_advect3_faces(ff_advect a, ff_field vu, ff_field vv, ff_field vw, ff_field iu, ff_field iv,
@@ -565,7 +640,16 @@ extern "C" int ff_advect3_faces(ff_advect a, ff_field vu, ff_field vv, ff_field 
     cudaSetDevice(a->ctx->device);
     const VelField F = trace_field({a->g, (const float *)vu->d, (const float *)vv->d, (const float *)vw->d,
                                     a->phi ? (const float *)a->phi->d : nullptr});
-    for (int c = 0; c < 3; ++c) FF_TRY(advect_component(a, F, c, (const float *)in[c]->d, (float *)out[c]->d));
+    const float *src[3] = {(const float *)iu->d, (const float *)iv->d, (const float *)iw->d};
+    float *dst[3] = {(float *)ou->d, (float *)ov->d, (float *)ow->d};
+    // fields that overlap across components: one after the other, as they are used
+    bool apart = true;
+    for (int c = 0; c < 3; ++c)
+        for (int q = 0; q < 3; ++q)
+            if (q != c)
+                apart = apart && !overlap(out[c], in[q]) && !overlap(out[c], vel[q]) && !overlap(out[c], out[q]);
+    if (apart) return advect_components(a, F, 0, 3, src, dst);
+    for (int c = 0; c < 3; ++c) FF_TRY(advect_components(a, F, c, 1, src + c, dst + c));
     return FF_OK;
 }
 
@@ -579,7 +663,9 @@ extern "C" int ff_advect3_scalar(ff_advect a, ff_field vu, ff_field vv, ff_field
     cudaSetDevice(a->ctx->device);
     const VelField F = trace_field({a->g, (const float *)vu->d, (const float *)vv->d, (const float *)vw->d,
                                     a->phi ? (const float *)a->phi->d : nullptr});
-    return advect_component(a, F, 3, (const float *)s_in->d, (float *)s_out->d);
+    const float *src = (const float *)s_in->d;
+    float *dst = (float *)s_out->d;
+    return advect_components(a, F, 3, 1, &src, &dst);
 }
 
 extern "C" int ff_advect3_trace(ff_advect a, ff_field vu, ff_field vv, ff_field vw, ff_field p_in, ff_field p_out,

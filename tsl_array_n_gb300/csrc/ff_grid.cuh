@@ -295,12 +295,16 @@ __device__ __forceinline__ void lin_uv(const VelField &F, const Point6 &q, float
     s = add2(s, prod2(d(a3 + 1, b3 + 1), mul2(w11, fz), F.nzero));
     unpack2(s, u, v);
 }
+// Lanes that are together here take one path: the other's results are the same, and
+// both one after the other cost more than the straightforward form alone (which
+// showed on small grids, where most warps touch an end: one of 39 us took 63).
+__device__ __forceinline__ bool warp_any(bool p) { return __any_sync(__activemask(), p); }
 __device__ __noinline__ F3 sample_vel_ends(const VelField &F, F3 p) { return sample_vel(F, p); }
 __device__ __noinline__ float sample_phi_ends(const VelField &F, F3 p) { return sample_phi(F, F.phi, p); }
 template <bool P2>
 __device__ __forceinline__ F3 trace_vel(const VelField &F, F3 p) {
     Point6 q;
-    if (!point6<P2>(F, p, q)) return sample_vel_ends(F, p);
+    if (warp_any(!point6<P2>(F, p, q))) return sample_vel_ends(F, p);
     F3 r;
     lin_uv(F, q, r.x, r.y);
     r.z = lin1(F.w, F.g.nx, F.g.ny, F.g.nx * F.g.ny, q.x.i[1], q.y.i[1], q.z.i[0], q.x.f[1], q.y.f[1], q.z.f[0]);
@@ -314,7 +318,7 @@ __device__ __forceinline__ float trace_phi(const VelField &F, F3 p) {
     bool in = axis_at<P2>(F.ax[0], 1, p.x, i, fx);
     in &= axis_at<P2>(F.ax[1], 1, p.y, j, fy);
     in &= axis_at<P2>(F.ax[2], 1, p.z, k, fz);
-    if (!in) return sample_phi_ends(F, p);
+    if (warp_any(!in)) return sample_phi_ends(F, p);
     const G3 &g = F.g;
     return lin1(F.phi, g.nx, g.ny, g.nz == 1 ? 0 : g.nx * g.ny, i, j, k, fx, fy, fz);
 }
@@ -354,7 +358,7 @@ __device__ __forceinline__ float trace_cubic(const VelField &F, int a, const flo
     in &= axis_at<P2>(F.ax[2], a != 2, p.z, k, fz);
     // one plane: every z tap is that plane
     const int z0 = sz == 1 ? 0 : 1, dz = sz == 1 ? 0 : sx * sy;
-    if (!(in && i >= 1 && i <= sx - 3 && j >= 1 && j <= sy - 3 && k >= z0 && (sz == 1 || k <= sz - 3)))
+    if (warp_any(!(in && i >= 1 && i <= sx - 3 && j >= 1 && j <= sy - 3 && k >= z0 && (sz == 1 || k <= sz - 3))))
         return tricubic_ends(d, sx, sy, sz, F.g, o, p);
     const f32x2 fx2 = pack2(fx, fx), fy2 = pack2(fy, fy);
     const float *r = d + ((i - 1) + sx * ((j - 1) + sy * (k - z0)));
@@ -375,7 +379,36 @@ __device__ __forceinline__ float trace_cubic(const VelField &F, int a, const flo
 }
 
 // backTrace (advection_solver3.js:20-62): RK2 midpoint substeps of at most
-// one cell, stopping on the collider with a linear blend of the last step.
+// one cell, stopping on the collider with a linear blend of the last step.  The
+// straightforward form.
+__device__ inline F3 back_trace_plain(const VelField &F, F3 pos, float dt, float dirn, int max_substeps) {
+    const float h = fminf(F.g.hx, fminf(F.g.hy, F.g.hz));
+    F3 pt = pos;
+    float T = dt;
+    for (int s = 0; s < max_substeps; ++s) {
+        if (T <= 1e-6f) break;
+        const F3 v0 = sample_vel(F, pt);
+        const float len = sqrtf(v0.x * v0.x + v0.y * v0.y + v0.z * v0.z);
+        const float nsub = fmaxf(ceilf(len * T / h), 1.0f);
+        const float sdt = T / nsub;
+        const float hs = sdt * 0.5f;
+        const F3 mid{pt.x - v0.x * hs * dirn, pt.y - v0.y * hs * dirn, pt.z - v0.z * hs * dirn};
+        const F3 mv = sample_vel(F, mid);
+        const F3 nxt{pt.x - mv.x * sdt * dirn, pt.y - mv.y * sdt * dirn, pt.z - mv.z * sdt * dirn};
+        const float phi0 = sample_phi(F, F.phi, pt), phi1 = sample_phi(F, F.phi, nxt);
+        if (phi1 <= 0.0f) {
+            const float w = fabsf(phi1) / (fabsf(phi0) + fabsf(phi1));
+            const float wm = 1.0f - w;
+            pt = F3{pt.x * w + nxt.x * wm, pt.y * w + nxt.y * wm, pt.z * w + nxt.z * wm};
+            break;
+        }
+        T = T - sdt;
+        pt = nxt;
+    }
+    return pt;
+}
+
+// back_trace_plain in the short form.
 // phi0: the collider's value at pos, if the caller has it (else a NaN); a
 // substep's end is the next one's start, with its value.
 template <bool P2>
