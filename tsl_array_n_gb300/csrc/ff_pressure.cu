@@ -61,7 +61,7 @@ struct ff_pressure_s {
     int tail_l = -1;
     // level 0 is small enough for the whole solve in one cooperative launch
     bool resident_fits = false;
-    int cluster = 0;                // blocks of a cluster for the resident solve
+    int cluster = 0;                // blocks of a cluster (the solve and the coarsest sweeps on one)
     bool use_tail = true;
     unsigned *tail_bar = nullptr;   // its grid barrier: arrivals, generation, abort
     // learned warm start (borrowed network), its guess field, last choice
@@ -294,7 +294,7 @@ extern "C" int ff_pressure3_create(ff_ctx ctx, const ff_pressure_desc *desc, ff_
                             ffk::sweep_tma_ok(ps->lv[0].d) && ps->lv[0].buf && (L == 2 || ps->tail_l == 1) &&
                             (desc->mg_coarse_mode == FF_COARSE_DIRECT || ps->lv[L - 1].d.n() <= 16384);
     }
-    if (ps->resident_fits) ps->cluster = ffk::cluster_blocks();
+    ps->cluster = ffk::cluster_blocks();
     if ((ps->tail_l >= 0 || ps->resident_fits) &&
         (st = ff_dev_alloc((void **)&ps->tail_bar, 4 * sizeof(unsigned), s)))
         return bail(st);
@@ -694,6 +694,12 @@ static int vcycle(ff_pressure ps, int l, const PcgState *st) {
             return ffk::mg_coarse_direct(v, ps->G, ps->nG, xbf, bbf, st, ps->s());
         }
         long long n = v.d.n();
+        if (vb == 0 && ps->cluster > 0 && ps->use_tail) {
+            bool done = false;
+            FF_TRY(ffk::coarse_cluster(v, ps->dims, ps->desc.mg_coarsest, (float)ps->desc.mg_sor, st, ps->cluster, done,
+                                       ps->s()));
+            if (done) return FF_OK;
+        }
         if (n <= 16384) {
             if (l == 0) FF_TRY(zero_x(ps, 0));
             return ffk::mg_coarse_sweeps(v, ps->dims, ps->desc.mg_coarsest, (float)ps->desc.mg_sor, xbf,
@@ -768,8 +774,13 @@ static int vcycle_fused(ff_pressure ps, int l, PcgState *st, int rz_mode, float 
         if (ps->desc.mg_coarse_mode == FF_COARSE_DIRECT) {
             FF_TRY(ffk::mg_coarse_direct(v, ps->G, ps->nG, 0, 0, st, s));
         } else if (v.d.n() <= 16384) {
-            FF_CUDA(cudaMemsetAsync(v.x, 0, (size_t)v.d.n() * 4, s));
-            FF_TRY(ffk::mg_coarse_sweeps(v, ps->dims, ps->desc.mg_coarsest, sor, 0, 0, 0, st, s));
+            bool done = false;
+            if (ps->cluster > 0 && ps->use_tail)
+                FF_TRY(ffk::coarse_cluster(v, ps->dims, ps->desc.mg_coarsest, sor, st, ps->cluster, done, s));
+            if (!done) {
+                FF_CUDA(cudaMemsetAsync(v.x, 0, (size_t)v.d.n() * 4, s));
+                FF_TRY(ffk::mg_coarse_sweeps(v, ps->dims, ps->desc.mg_coarsest, sor, 0, 0, 0, st, s));
+            }
         } else {
             for (int it = 0; it < ps->desc.mg_coarsest; ++it) {
                 int nxt = cur < 0 ? 0 : 1 - cur;

@@ -67,7 +67,7 @@ struct VArgs {
     int coarse_sweeps;             // > 0: that many sweeps on the coarsest level instead of G b
     unsigned *bar;                 // grid barrier: arrivals, blocks done, abort
     int ro, cxo, cbo;              // shared memory: held levels' residual, the coarsest x and b
-    int cr, crx, cop, cow;         // cluster levels' residual and its x taps; the swept coarsest's diagonals and pair words
+    int cr, crx, cop, cow, cok;    // cluster levels' residual and its x taps; the swept coarsest's diagonals, pair words and couplings
     int p, xh, xl, rhs;            // k_pcg_cluster's search direction, iterate (lv[0]'s x layout) and right-hand side
     int floats;                    // shared memory in use
     DotOrder dot[3];               // of p.Ap, r.r and r.z
@@ -1200,8 +1200,9 @@ __device__ __noinline__ void c_prolong(int l) {
 // Sweeps of a coarsest level spread over the cluster, coarse_relax's
 // arithmetic.  A pair of neighbours of a row is a word: its first cell (14
 // bits), its row (10), (j + k) & 1, and for each cell whether its couplings are
-// the plain ones on all sides (then nothing else is loaded); a cell's diagonal
-// and its reciprocal are kept.
+// the plain ones on all sides (then nothing else is loaded); the diagonals, their
+// reciprocals and, where they fit, the couplings of the others are kept (through L2,
+// after a cluster barrier, they cost more than the rest of a pass).
 template <bool D3>
 __device__ __forceinline__ void coarse_couplings(const RLevel &C, int c, int i, int j, int k, float (&kf)[6], float &e) {
     const Dims d = C.g.d;
@@ -1238,6 +1239,11 @@ __device__ __noinline__ void c_coarse_build() {
             if (j < d.ny - 1) D -= kf[3];
             if (D3 && k < d.nz - 1) D -= kf[5];
             diag[e] = make_float2(D, 1.f / D);
+            if (SA.cok >= 0) {
+                float4 *q8 = reinterpret_cast<float4 *>(rsm + SA.cok + 8 * e);
+                q8[0] = make_float4(kf[0], kf[1], kf[2], kf[3]);
+                q8[1] = make_float4(kf[4], kf[5], E, 0.f);
+            }
             const bool plain = E == 0.f && kf[0] == C.g.h2x && kf[1] == C.g.h2x && kf[2] == C.g.h2y && kf[3] == C.g.h2y &&
                                (!D3 || (kf[4] == C.g.h2z && kf[5] == C.g.h2z));
             if (plain) w |= 1u << (25 + o);
@@ -1257,6 +1263,11 @@ __device__ __noinline__ void c_coarse() {
     const float2 *diag = reinterpret_cast<const float2 *>(rsm + SA.cop);
     float *x = rsm + C.cx;
     const float *b = rsm + C.cb;
+    // a plain cell's diagonal, summed as c_coarse_build sums it
+    float2 plain;
+    plain.x = -(0.f + C.g.h2x + C.g.h2y + C.g.h2z) - C.g.h2x - C.g.h2y;
+    if (D3) plain.x -= C.g.h2z;
+    plain.y = 1.f / plain.x;
     for (int e = threadIdx.x; e < nx * R.n; e += NT) x[e] = 0.f;
     cluster_sync();
     for (int pass = 0; pass < passes; ++pass) {
@@ -1273,11 +1284,18 @@ __device__ __noinline__ void c_coarse() {
             // (a row's end: any finite value, its coupling is 0)
             const float xm = x[i > 0 ? e - 1 : e], xp = x[i < nx - 1 ? e + 1 : e];
             float kf[6] = {C.g.h2x, C.g.h2x, C.g.h2y, C.g.h2y, C.g.h2z, C.g.h2z}, E = 0.f;
+            float2 D = plain;
             if (!(w >> (25 + o) & 1u)) {
-                const int q = R.q0 + lr, k = D3 ? tdiv(q, C.mny) : 0, j = q - k * d.ny;
-                coarse_couplings<D3>(C, R.q0 * nx + e, i, j, k, kf, E);
+                D = diag[e];
+                if (SA.cok >= 0) {
+                    const float4 *q8 = reinterpret_cast<const float4 *>(rsm + SA.cok + 8 * e);
+                    const float4 k0 = q8[0], k1 = q8[1];
+                    kf[0] = k0.x, kf[1] = k0.y, kf[2] = k0.z, kf[3] = k0.w, kf[4] = k1.x, kf[5] = k1.y, E = k1.z;
+                } else {
+                    const int q = R.q0 + lr, k = D3 ? tdiv(q, C.mny) : 0, j = q - k * d.ny;
+                    coarse_couplings<D3>(C, R.q0 * nx + e, i, j, k, kf, E);
+                }
             }
-            const float2 D = diag[e];
             float s = -E * xc;
             s += kf[0] * (xm - xc);
             s += kf[1] * (xp - xc);
@@ -1624,6 +1642,31 @@ __global__ void __launch_bounds__(NT, 1) k_vcycle_tail(const __grid_constant__ V
     if (blockIdx.x == 0) low_init<D3, false>();
     if (vcycle<D3, false>(passed, false, nullptr)) grid_done(SA.bar);
     else if (threadIdx.x == 0 && st) atomicOr(&st->err, 2);
+}
+
+// The sweeps of a coarsest level alone, from x = 0: its rows over the blocks of a
+// cluster (up to 2 NT cells: in one block), the operator in tables, x in shared memory
+// from the first pass to the last.  Bound by latency, a pass being a cluster barrier
+// and a remote round trip.  45 x 27 x 33 with 40 passes: 55 us, 90 with one launch a
+// pass (projection of 90 x 54 x 66: 7.03 -> 6.20 ms).
+template <bool D3>
+__global__ void __launch_bounds__(NT, 1) k_coarse_cluster(const __grid_constant__ VArgs a, const PcgState *st) {
+    if (st && st->stop) return;
+    load_args(a);
+    low_init<D3, true>();
+    const RLevel &C = SA.lv[0];
+    if (SA.ccoarse) {
+        const Rows R = rows_of(C);
+        const int n = C.g.d.nx * R.n, c0 = R.q0 * C.g.d.nx;
+        for (int e = threadIdx.x; e < n; e += NT) rsm[C.cb + e] = __ldg(C.b + c0 + e);
+        __syncthreads();
+        c_coarse<D3>();
+        for (int e = threadIdx.x; e < n; e += NT) C.x[c0 + e] = rsm[C.cx + e];
+    } else {
+        tier_copy<D3>(0, true);
+        coarse_sweeps<D3>();
+        tier_copy<D3>(0, false);
+    }
 }
 
 // -------------------------------------------------------------- PCG solve --
@@ -2234,6 +2277,7 @@ int place(VArgs &a, bool d3, bool solver) {
         const long long floats = 8LL * (l < a.held ? (long long)a.lv[l].rows * a.lv[l].g.d.nx : a.lv[l].g.d.n());
         a.lv[l].co = fits(floats) ? take(floats) : -1;
     }
+    a.cok = a.ccoarse && fits(8 * ccells) ? take(8 * ccells) : -1;
     a.floats = used;
     return 4 * used;
 }
@@ -2269,7 +2313,7 @@ VArgs make_args(const Level *lv, const SweepMaps *sm, int nl, int dims, int down
         t.mhx = magic(std::max(1, L.d.nx / 2));
         t.mnx = magic(L.d.nx);
         t.mny = magic(L.d.ny);
-        if (l < nl - 1) {
+        if (l < nl - 1 && sm) {
             t.cls = sm[l].cls_ptr;
             t.cpitch = sm[l].cls_pitch;
             t.gco = sm[l].gco;
@@ -2360,6 +2404,18 @@ int vcycle_tail(const Level *lv, const SweepMaps *sm, int nl, int dims, int down
     const bool alone = a.clu == 0 && coarse_sweeps > 0;
     return launch(dims == 3 ? (const void *)k_vcycle_tail<true> : (const void *)k_vcycle_tail<false>, alone ? 1 : sm_count, 1,
                   smem, s, args);
+}
+
+int coarse_cluster(const Level &L, int dims, int sweeps, float sor, const PcgState *st, int cluster, bool &done,
+                   cudaStream_t s) {
+    int smem = 0;
+    const int csize = L.d.n() <= 2 * NT ? 1 : cluster;
+    VArgs a = make_args(&L, nullptr, 1, dims, 0, 0, 0, sor, nullptr, 0, sweeps, nullptr, csize, false, 0, smem);
+    done = csize == 1 || a.ccoarse;
+    if (!done) return FF_OK;
+    void *args[] = {&a, &st};
+    return launch(dims == 3 ? (const void *)k_coarse_cluster<true> : (const void *)k_coarse_cluster<false>, csize, csize, smem,
+                  s, args);
 }
 
 int pcg_resident(const Level *lv, const SweepMaps *sm, int nl, int dims, int down, int up, int fin, float sor,
