@@ -52,6 +52,7 @@ __host__ __device__ inline int growth_first_check(int last_iters) {
 struct ff_ctx_s {
     int device = 0;
     int sm_count = 0;
+    int cluster_blocks = -1;   // blocks of a thread-block cluster the solvers use (0: none), once asked for
     cudaStream_t stream = nullptr;
     cudaEvent_t events[16] = {};
     // copy streams of the host-buffer entry points (created on first use):
@@ -250,7 +251,7 @@ size_t cls_row_pitch(const Dims &d);
 // launch and after a failed one; st may be null (no stop or error flags)
 int vcycle_tail(const Level *lv, const SweepMaps *sm, int nl, int dims, int down, int up, float sor,
                 const double *G, int nG, int coarse_sweeps, PcgState *st, unsigned *bar, int sm_count,
-                cudaStream_t s);
+                int cluster, cudaStream_t s);
 // a whole PCG solve (after k_state_init) in one launch, for
 // hierarchies of at most 12 levels with classes on all but the coarsest
 // and at least one sweep before and after the correction; levels' x and b as in

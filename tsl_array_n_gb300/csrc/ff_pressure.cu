@@ -294,7 +294,8 @@ extern "C" int ff_pressure3_create(ff_ctx ctx, const ff_pressure_desc *desc, ff_
                             ffk::sweep_tma_ok(ps->lv[0].d) && ps->lv[0].buf && (L == 2 || ps->tail_l == 1) &&
                             (desc->mg_coarse_mode == FF_COARSE_DIRECT || ps->lv[L - 1].d.n() <= 16384);
     }
-    ps->cluster = ffk::cluster_blocks();
+    if (ctx->cluster_blocks < 0) ctx->cluster_blocks = ffk::cluster_blocks();
+    ps->cluster = ctx->cluster_blocks;
     if ((ps->tail_l >= 0 || ps->resident_fits) &&
         (st = ff_dev_alloc((void **)&ps->tail_bar, 4 * sizeof(unsigned), s)))
         return bail(st);
@@ -766,7 +767,7 @@ static int vcycle_fused(ff_pressure ps, int l, PcgState *st, int rz_mode, float 
         // this level and every coarser one in one cooperative launch
         FF_TRY(ffk::vcycle_tail(&ps->lv[l], &ps->smaps[l], Ln - l, ps->dims, ps->desc.mg_down, ps->desc.mg_up, sor,
                                 direct ? ps->G : nullptr, direct ? ps->nG : 0, direct ? 0 : ps->desc.mg_coarsest, st,
-                                ps->tail_bar, ps->ctx->sm_count, s));
+                                ps->tail_bar, ps->ctx->sm_count, ps->cluster, s));
         *out = (float *)v.x;
         return FF_OK;
     }
