@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("shape,levels,coarse", [((128, 64, 64), 4, "sweeps"), ((136, 64, 64), 4, "sweeps"),
                                                  ((512, 512, 1), 5, "sweeps"), ((512, 544, 1), 5, "sweeps"),
                                                  ((256, 128, 40), 4, "sweeps"), ((96, 48, 48), 4, "direct"),
-                                                 ((64, 32, 4), 2, "sweeps"), ((256, 64, 64), 3, "direct")])
+                                                 ((64, 32, 4), 2, "sweeps"), ((256, 64, 64), 4, "direct")])
 def test_preconditioner(gpu, shape, levels, coarse):
     from tsl_array_n_gb300.tsl_array_n import Field
     s, grid, _ = solver_for(shape, levels, coarse, "mixed", 5)

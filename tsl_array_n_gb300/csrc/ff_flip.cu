@@ -1,12 +1,12 @@
 // 3D FLIP particle-grid transfer (fluxflow src/grid/grid_flip_solver3.js):
-// particle advection through the grid velocity, fixed-point P2G with int32
-// atomics, fluid marking and the reduced-pressure Dirichlet condition of
+// particle advection through the grid velocity, fixed-point P2G through
+// shared-memory windows, fluid marking and the reduced-pressure Dirichlet condition of
 // air cells, the variable-density beta faces and reduced gravity, G2P with
 // the FLIP/PIC blend, and the per-step orchestration (onAdvanceTimeStep).
 //
 // FP32 arithmetic rounds one operation at a time (-fmad=false), in the
 // reference's evaluation order; P2G accumulates round(v w S) and round(w S)
-// as int32 (wrapping like the reference's i32 atomics), so its result does
+// as integers (wrapping like the reference's i32 atomics), so its result does
 // not depend on the order particles arrive in.  Host-side seeding
 // (computeFlipBoxSeed3, mulberry32) is computed in doubles as JavaScript
 // does (-ffp-contract=off on the host compiler).

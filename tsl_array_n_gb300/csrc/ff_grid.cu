@@ -9,8 +9,9 @@
 // and every expression keeps the reference's evaluation order.  That makes
 // the results reproducible operation for operation on any IEEE FP32 machine.
 //
-// All kernels are HBM/L2-bound gathers (a tricubic sample reads 64 taps of
-// one component, mostly L1/L2 hits); one thread per face or cell.
+// Advection is bound by issue (a tricubic sample reads 64 taps of one component,
+// mostly L1/L2 hits), the constraint by the bytes of the faces that its stages can
+// change, which lists keep; one thread per face or cell, or four for a pass over all.
 #include "ff_grid.cuh"
 #include <algorithm>
 #include <cmath>

@@ -2,9 +2,9 @@
 // (fluxflow src/grid/grid_pressure_solver3.js:66-574) and of the GPU-resident
 // PCG it drives (src/linalg/linalg.js:782-2469).
 //
-// A solve is two CUDA graphs: the setup sequence (linalg.js:1627-1637) and a
-// conditional WHILE node whose body is one PCG iteration (linalg.js:1404-1436
-// order).  The loop stops itself on the device (convergence, a guard, or the
+// A small solve is one launch (ff_resident.cu; see resident()).  Any other is two
+// CUDA graphs: the setup sequence (linalg.js:1627-1637) and a conditional WHILE
+// node whose body is one PCG iteration (linalg.js:1404-1436 order).  The loop stops itself on the device (convergence, a guard, or the
 // iteration cap), so the host waits once per solve instead of once per chunk
 // (linalg.js:1817-1911).
 #include "ff_internal.h"
@@ -63,7 +63,7 @@ struct ff_pressure_s {
     bool resident_fits = false;
     int cluster = 0;                // blocks of a cluster (the solve and the coarsest sweeps on one)
     bool use_tail = true;
-    unsigned *tail_bar = nullptr;   // its grid barrier: arrivals, generation, abort
+    unsigned *tail_bar = nullptr;   // the grid barrier: arrivals, blocks done, abort
     // learned warm start (borrowed network), its guess field, last choice
     ff_unet net = nullptr;
     ff_field guess = nullptr;
@@ -281,7 +281,8 @@ extern "C" int ff_pressure3_create(ff_ctx ctx, const ff_pressure_desc *desc, ff_
         }
         // the coarse V-cycle in one launch: from the first level of at most
         // 64^3 cells (below level 0) whose levels down to the last but one
-        // all have nx % 4 == 0 (class bytes per x-quad) and a residual buffer
+        // all have nx % 4 == 0 (as the level kernels of the fused V-cycle need) and a
+        // residual buffer
         for (int l = 1; l < L - 1 && ps->tail_l < 0; ++l) {
             if (ps->lv[l].d.n() > (1LL << 18)) continue;
             bool ok = true;

@@ -5,14 +5,14 @@
 //
 // Activations are stored channels-last (z, y, x, c) in BF16; convolutions
 // are implicit GEMMs (M = voxels, K = 27 taps x Cin, N = Cout) with BF16
-// operands and FP32 accumulation on tcgen05 (accumulators in TMEM):
-// forward, input-gradient and weight-gradient convolutions; pre-activations
+// operands and FP32 accumulation, forward and input-gradient convolutions on
+// tcgen05 (accumulators in TMEM), weight gradients on mma.sync; pre-activations
 // are kept in FP32 for the backward pass only (inference stores none);
 // master weights, gradients and the Adam moments are FP32, with a BF16 copy
 // of the weights for the GEMMs.  Forward and input-gradient convolutions run
 // in k_conv3_zm (a z-march over TMA-staged planes); the input-gradient one
 // takes the taps flipped and the weight matrix transposed; weight gradients
-// accumulate per-tap [Cin x Cout] tiles over voxel chunks with FP32 atomics.
+// (k_conv3_wgrad) march columns of voxels with the taps' sums in registers.
 #include "ff_internal.h"
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
