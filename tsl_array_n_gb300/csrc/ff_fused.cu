@@ -296,6 +296,9 @@ struct TqArgs {
     const float4 *coef;
     const uint8_t *bricks;
     const float4 *gco;             // class-3 upper couplings and 1 / diagonal
+    const float4 *rk;              // couplings and 1 / diagonal by pairs (SweepMaps)
+    const float2 *rinv;
+    long long quads;
     const int *order;              // work item of each block (tile column + z-chunk)
     int gx, gy;                    // tiles along x and y
     float sor, rdreg_sor, omsor;   // sor, sor / dreg, 1 - sor
@@ -381,6 +384,43 @@ __device__ __forceinline__ float relax_any(const Geo &g, const TqArgs &a, unsign
     return __fmaf_rn(bval - s, rd, a.omsor * vc);
 }
 
+// relax_any on the two cells of a pair (parity P of a quad), the PAIRS form of the
+// sweep.  Their couplings come as planes, 16 bytes a lane: per cell from coef and gco
+// a load of a warp touches 16 lines, and L1 lines bound the sweeps of a solve whose
+// cells are of class 3 throughout (256 x 128 x 128 with variable density: 55 -> 45 us a
+// sweep, 60 -> 52 with r.z).  Levels with few such cells keep the other form, which
+// needs fewer registers (256^3 sphere: 58 us, 62 in this form).
+struct PairK {
+    float4 x, y, z;
+    float2 inv;
+};
+__device__ __forceinline__ PairK pair_couplings(const TqArgs &a, bool any3, long long quad, int P) {
+    PairK k{};
+    if (any3) {
+        k.x = __ldg(a.rk + P * a.quads + quad);
+        k.y = __ldg(a.rk + (2 + P) * a.quads + quad);
+        k.z = __ldg(a.rk + (4 + P) * a.quads + quad);
+        k.inv = __ldg(a.rinv + P * a.quads + quad);
+    }
+    return k;
+}
+__device__ __forceinline__ float relax_with(const Geo &g, const TqArgs &a, unsigned cls, float kx, float ux, float ky,
+                                            float uy, float kz, float uz, float inv, float vc, float xm, float xp,
+                                            float ym, float yp, float zm, float zp, float bval, float rd) {
+    const bool gen = cls == 3u, plain = !(cls & 1u);
+    kx = gen ? kx : (plain ? g.h2x : 0.f), ux = gen ? ux : (plain ? g.h2x : 0.f);
+    ky = gen ? ky : (plain ? g.h2y : 0.f), uy = gen ? uy : (plain ? g.h2y : 0.f);
+    kz = gen ? kz : (plain ? g.h2z : 0.f), uz = gen ? uz : (plain ? g.h2z : 0.f);
+    rd = gen ? a.sor * inv : (plain ? rd : -a.sor);
+    float s = kx * xm;
+    s = __fmaf_rn(ux, xp, s);
+    s = __fmaf_rn(ky, ym, s);
+    s = __fmaf_rn(uy, yp, s);
+    s = __fmaf_rn(kz, zm, s);
+    s = __fmaf_rn(uz, zp, s);
+    return __fmaf_rn(bval - s, rd, a.omsor * vc);
+}
+
 // Scales (sor over the diagonal) of a quad's plain cells on one plane:
 // cells 0, 1-2 and 3 differ only in the x faces.
 struct QuadScale {
@@ -391,7 +431,7 @@ struct QuadScale {
 // registers: s is the x-neighbour outside the quad (cell -1 for P = 0, cell
 // 4 for P = 1), ym/yp/zm/zp the neighbouring quads, bq the right-hand side,
 // cq the class byte.
-template <int P>
+template <int P, bool PAIRS>
 __device__ __forceinline__ void relax_pair(const Geo &g, const TqArgs &a, float4 &q, float s, const float4 &ym,
                                            const float4 &yp, const float4 &zm, const float4 &zp, const float4 &bq,
                                            unsigned cq, const QuadScale &e, int gi, int gj, int k) {
@@ -407,8 +447,17 @@ __device__ __forceinline__ void relax_pair(const Geo &g, const TqArgs &a, float4
         n1 = relax_plain(g, a.omsor, v1, l1, r1, ym1, yp1, zm1, zp1, b1, rb);
     } else {
         const long long c = gi + P + g.sy * gj + g.sz * k;
-        n0 = relax_any(g, a, (cq >> (2 * P)) & 3u, c, v0, l0, r0, ym0, yp0, zm0, zp0, b0, ra);
-        n1 = relax_any(g, a, (cq >> (2 * P + 4)) & 3u, c + 2, v1, l1, r1, ym1, yp1, zm1, zp1, b1, rb);
+        const unsigned ca = (cq >> (2 * P)) & 3u, cb = (cq >> (2 * P + 4)) & 3u;
+        if (PAIRS) {
+            const PairK q2 = pair_couplings(a, ca == 3u || cb == 3u, c >> 2, P);
+            n0 = relax_with(g, a, ca, q2.x.x, q2.x.z, q2.y.x, q2.y.z, q2.z.x, q2.z.z, q2.inv.x, v0, l0, r0, ym0, yp0, zm0,
+                            zp0, b0, ra);
+            n1 = relax_with(g, a, cb, q2.x.y, q2.x.w, q2.y.y, q2.y.w, q2.z.y, q2.z.w, q2.inv.y, v1, l1, r1, ym1, yp1, zm1,
+                            zp1, b1, rb);
+        } else {
+            n0 = relax_any(g, a, ca, c, v0, l0, r0, ym0, yp0, zm0, zp0, b0, ra);
+            n1 = relax_any(g, a, cb, c + 2, v1, l1, r1, ym1, yp1, zm1, zp1, b1, rb);
+        }
     }
     if (P) {
         q.y = n0;
@@ -422,6 +471,7 @@ __device__ __forceinline__ void relax_pair(const Geo &g, const TqArgs &a, float4
 // relax_pair with the colour offset P chosen at run time (selects instead of
 // a branch): the two rows of the halo ring, whose colours differ, share one
 // warp without diverging.
+template <bool PAIRS>
 __device__ __forceinline__ void relax_pair_rt(const Geo &g, const TqArgs &a, float4 &q, float s, const float4 &ym,
                                               const float4 &yp, const float4 &zm, const float4 &zp, const float4 &bq,
                                               unsigned cq, const QuadScale &e, int gi, int gj, int k, int P) {
@@ -438,8 +488,17 @@ __device__ __forceinline__ void relax_pair_rt(const Geo &g, const TqArgs &a, flo
         n1 = relax_plain(g, a.omsor, v1, l1, r1, ym1, yp1, zm1, zp1, b1, rb);
     } else {
         const long long c = gi + P + g.sy * gj + g.sz * k;
-        n0 = relax_any(g, a, (cq >> (2 * P)) & 3u, c, v0, l0, r0, ym0, yp0, zm0, zp0, b0, ra);
-        n1 = relax_any(g, a, (cq >> (2 * P + 4)) & 3u, c + 2, v1, l1, r1, ym1, yp1, zm1, zp1, b1, rb);
+        const unsigned ca = (cq >> (2 * P)) & 3u, cb = (cq >> (2 * P + 4)) & 3u;
+        if (PAIRS) {
+            const PairK q2 = pair_couplings(a, ca == 3u || cb == 3u, c >> 2, P);
+            n0 = relax_with(g, a, ca, q2.x.x, q2.x.z, q2.y.x, q2.y.z, q2.z.x, q2.z.z, q2.inv.x, v0, l0, r0, ym0, yp0, zm0,
+                            zp0, b0, ra);
+            n1 = relax_with(g, a, cb, q2.x.y, q2.x.w, q2.y.y, q2.y.w, q2.z.y, q2.z.w, q2.inv.y, v1, l1, r1, ym1, yp1, zm1,
+                            zp1, b1, rb);
+        } else {
+            n0 = relax_any(g, a, ca, c, v0, l0, r0, ym0, yp0, zm0, zp0, b0, ra);
+            n1 = relax_any(g, a, cb, c + 2, v1, l1, r1, ym1, yp1, zm1, zp1, b1, rb);
+        }
     }
     q.x = p1 ? q.x : n0;
     q.y = p1 ? n0 : q.y;
@@ -458,6 +517,7 @@ __device__ __forceinline__ float first_scale(const TqArgs &a, unsigned cls, long
     if (cls == 3u) return a.sor * __ldg(&a.gco[c].w);
     return rd;
 }
+template <bool PAIRS>
 __device__ __forceinline__ void relax_pair_first(const Geo &g, const TqArgs &a, float4 &q, const float4 &bq,
                                                  unsigned cq, const QuadScale &e, int gi, int gj, int k, int P) {
     const bool p1 = P != 0;
@@ -465,8 +525,16 @@ __device__ __forceinline__ void relax_pair_first(const Geo &g, const TqArgs &a, 
     float r0 = p1 ? e.r12 : e.r0, r1 = p1 ? e.r3 : e.r12;
     if (cq & (0x11u << (2 * P))) {
         const long long c = gi + P + g.sy * gj + g.sz * k;
-        r0 = first_scale(a, (cq >> (2 * P)) & 3u, c, r0);
-        r1 = first_scale(a, (cq >> (2 * P + 4)) & 3u, c + 2, r1);
+        const unsigned ca = (cq >> (2 * P)) & 3u, cb = (cq >> (2 * P + 4)) & 3u;
+        if (PAIRS) {
+            float2 inv = make_float2(0.f, 0.f);
+            if (ca == 3u || cb == 3u) inv = __ldg(a.rinv + P * a.quads + (c >> 2));
+            r0 = ca == 3u ? a.sor * inv.x : (ca == 1u ? -a.sor : r0);
+            r1 = cb == 3u ? a.sor * inv.y : (cb == 1u ? -a.sor : r1);
+        } else {
+            r0 = first_scale(a, ca, c, r0);
+            r1 = first_scale(a, cb, c + 2, r1);
+        }
     }
     const float z = a.omsor * 0.f;
     const float n0 = __fmaf_rn(b0, r0, z), n1 = __fmaf_rn(b1, r1, z);
@@ -481,7 +549,23 @@ __device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefe
 // any cell of class 3 among the four 2-bit fields of a class byte
 __device__ __forceinline__ bool any_general(unsigned c) { return (c & (c >> 1) & 0x55u) != 0; }
 
-template <bool FIRST, bool RZ>
+// A row of a tile has 16 quads: two lines of each of the six planes and one of each
+// parity's inverses.  Where a quad of the row has a class-3 cell (`general`, all lanes
+// of the warp ask together) the row's lanes take one line each.  quad: the lane's;
+// right: whether the row's second half lies in the domain.
+__device__ __forceinline__ void prefetch_pairs(const TqArgs &a, bool general, long long quad, int lane16, int lane,
+                                               bool right) {
+    const unsigned m = __ballot_sync(0xffffffffu, general);
+    if (!(m >> (lane & 16) & 0xffffu)) return;
+    const long long row = quad - lane16;
+    if (lane16 < 12) {
+        if (right || !(lane16 & 1)) prefetch_l1(a.rk + (lane16 >> 1) * a.quads + row + 8 * (lane16 & 1));
+    } else if (lane16 < 14) {
+        prefetch_l1(a.rinv + (lane16 - 12) * a.quads + row);
+    }
+}
+
+template <bool FIRST, bool RZ, bool PAIRS>
 __global__ void __launch_bounds__(tq::NT, 4)
     k_sweep_tma(TqArgs a, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap bmap,
                 const __grid_constant__ CUtensorMap cmap) {
@@ -618,7 +702,10 @@ __global__ void __launch_bounds__(tq::NT, 4)
             // coefficient lines of this quad's class-3 cells on plane m+3 go
             // to L1 ahead of their first use in step m+1
             const int kp = m + 3;
-            if (quad_in && any_general(c3) && kp < g.d.nz) {
+            if (PAIRS) {
+                prefetch_pairs(a, quad_in && any_general(c3) && kp < g.d.nz, (qoff + g.sz * kp) >> 2, qx, lane,
+                               i0 + TX / 2 < g.d.nx);
+            } else if (quad_in && any_general(c3) && kp < g.d.nz) {
                 const long long off = qoff + g.sz * kp;
                 prefetch_l1(a.coef + off);
                 prefetch_l1(a.gco + off);
@@ -630,7 +717,7 @@ __global__ void __launch_bounds__(tq::NT, 4)
                 if (FIRST) {
                     const QuadScale e = scale_at(ka);
                     const unsigned c2 = (cpipe >> 16) & 0xffu;
-                    if (quad_in) relax_pair_first(g, a, q2, bb2, c2, e, gi, gj, ka, (ca ^ gj ^ ka) & 1);
+                    if (quad_in) relax_pair_first<PAIRS>(g, a, q2, bb2, c2, e, gi, gj, ka, (ca ^ gj ^ ka) & 1);
                 } else {
                     const float4 ym = lds4(X2 + o - RW), yp = lds4(X2 + o + RW);
                     const QuadScale e = scale_at(ka);
@@ -638,11 +725,11 @@ __global__ void __launch_bounds__(tq::NT, 4)
                     if ((ca ^ gj ^ ka) & 1) {
                         float s = __shfl_down_sync(FULL, q2.x, 1);
                         if (qx == QX - 1) s = X2[o + 4];
-                        if (quad_in) relax_pair<1>(g, a, q2, s, ym, yp, q1, q3, bb2, c2, e, gi, gj, ka);
+                        if (quad_in) relax_pair<1, PAIRS>(g, a, q2, s, ym, yp, q1, q3, bb2, c2, e, gi, gj, ka);
                     } else {
                         float s = __shfl_up_sync(FULL, q2.w, 1);
                         if (qx == 0) s = X2[o - 1];
-                        if (quad_in) relax_pair<0>(g, a, q2, s, ym, yp, q1, q3, bb2, c2, e, gi, gj, ka);
+                        if (quad_in) relax_pair<0, PAIRS>(g, a, q2, s, ym, yp, q1, q3, bb2, c2, e, gi, gj, ka);
                     }
                 }
                 if (quad_in) *reinterpret_cast<float4 *>(X2 + o) = q2;
@@ -656,11 +743,11 @@ __global__ void __launch_bounds__(tq::NT, 4)
                 if ((cb ^ gj ^ m) & 1) {
                     float s = __shfl_down_sync(FULL, q0.x, 1);
                     if (qx == QX - 1) s = X0[o + 4];
-                    if (quad_in) relax_pair<1>(g, a, q0, s, ym, yp, qm1, q1, bb0, c0, e, gi, gj, m);
+                    if (quad_in) relax_pair<1, PAIRS>(g, a, q0, s, ym, yp, qm1, q1, bb0, c0, e, gi, gj, m);
                 } else {
                     float s = __shfl_up_sync(FULL, q0.w, 1);
                     if (qx == 0) s = X0[o - 1];
-                    if (quad_in) relax_pair<0>(g, a, q0, s, ym, yp, qm1, q1, bb0, c0, e, gi, gj, m);
+                    if (quad_in) relax_pair<0, PAIRS>(g, a, q0, s, ym, yp, qm1, q1, bb0, c0, e, gi, gj, m);
                 }
                 if (quad_in) {
                     *reinterpret_cast<float4 *>(a.x_out + qoff + g.sz * m) = q0;
@@ -690,7 +777,10 @@ __global__ void __launch_bounds__(tq::NT, 4)
                 const int rco = (rlrow + 1) * CW + 16 + rl;
                 if (m == mstart) rcls = cs[rco];
                 const unsigned rnext = C3[rco];
-                if (rquad_in && any_general(rnext) && kp < g.d.nz) {
+                if (PAIRS) {
+                    prefetch_pairs(a, rquad_in && any_general(rnext) && kp < g.d.nz, (rgi + g.sy * rgj + g.sz * kp) >> 2,
+                                   rl, lane, i0 + TX / 2 < g.d.nx);
+                } else if (rquad_in && any_general(rnext) && kp < g.d.nz) {
                     const long long off = rgi + g.sy * rgj + g.sz * kp;
                     prefetch_l1(a.coef + off);
                     prefetch_l1(a.gco + off);
@@ -705,7 +795,7 @@ __global__ void __launch_bounds__(tq::NT, 4)
                         re.r0 = rdt[(rgi == 0) + 3 * rmy + mz];
                         re.r12 = rdt[3 * rmy + mz];
                         re.r3 = rdt[(rgi + 3 == g.d.nx - 1) + 3 * rmy + mz];
-                        relax_pair_first(g, a, rq, rbq, rcls, re, rgi, rgj, ka, (ca ^ rgj ^ ka) & 1);
+                        relax_pair_first<PAIRS>(g, a, rq, rbq, rcls, re, rgi, rgj, ka, (ca ^ rgj ^ ka) & 1);
                         *reinterpret_cast<float4 *>(X2 + ro4) = rq;
                     }
                 } else if (ka >= 0 && ka <= k1 && ka < g.d.nz) {
@@ -723,7 +813,7 @@ __global__ void __launch_bounds__(tq::NT, 4)
                         re.r12 = rdt[3 * rmy + mz];
                         re.r3 = rdt[(rgi + 3 == g.d.nx - 1) + 3 * rmy + mz];
                         const int P = (ca ^ rgj ^ ka) & 1;
-                        relax_pair_rt(g, a, rq, P ? sd : su, rym, ryp, rzm, rzp, rbq, rcls, re, rgi, rgj, ka, P);
+                        relax_pair_rt<PAIRS>(g, a, rq, P ? sd : su, rym, ryp, rzm, rzp, rbq, rcls, re, rgi, rgj, ka, P);
                         *reinterpret_cast<float4 *>(X2 + ro4) = rq;
                     }
                 }
@@ -2079,7 +2169,8 @@ __global__ void __launch_bounds__(256) k_prolong4(Dims fd, Dims cd, int dims, co
 __global__ void k_coef_classes(Geo g, int dims, const float *__restrict__ wu, const float *__restrict__ wv,
                                const float *__restrict__ ww, const uint8_t *__restrict__ mask, float hx2, float hy2,
                                float hz2, float4 *__restrict__ coef, uint2 *__restrict__ coef16,
-                               uint8_t *__restrict__ cls, int pitch, float4 *__restrict__ gco) {
+                               uint8_t *__restrict__ cls, int pitch, float4 *__restrict__ gco, float4 *__restrict__ rk,
+                               float2 *__restrict__ rinv) {
     // one thread per cell (coalesced coefficient stores); the four lanes of
     // an x-quad (blockDim.x is a multiple of 32) merge their classes into the
     // quad's byte with shuffles, cells past the row's end as class 0
@@ -2125,7 +2216,20 @@ __global__ void k_coef_classes(Geo g, int dims, const float *__restrict__ wu, co
     }
     if (cl == 3u) {
         const float diag = -(e + kx + ux + ky + uy + kz + uz);
-        gco[c] = make_float4(ux, uy, uz, 1.f / diag);
+        const float inv = 1.f / diag;
+        gco[c] = make_float4(ux, uy, uz, inv);
+        if (rk) {
+            const long long quads = (long long)(d.nx >> 2) * d.ny * d.nz, q = c >> 2;
+            const int P = i & 1, h = (i >> 1) & 1;
+            const float lo[3] = {kx, ky, kz}, hi[3] = {ux, uy, uz};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                float *t = reinterpret_cast<float *>(rk + (2 * a + P) * quads + q);
+                t[h] = lo[a];
+                t[2 + h] = hi[a];
+            }
+            reinterpret_cast<float *>(rinv + P * quads + q)[h] = inv;
+        }
     }
     if ((i & 3) == 0) cls[(i >> 2) + (long long)pitch * (j + (long long)d.ny * k)] = (uint8_t)byte;
 }
@@ -2497,7 +2601,7 @@ int coef_classes(const Level &L, const SweepMaps &m, uint8_t *bricks, int dims, 
     dim3 grid((L.d.nx + bx - 1) / bx, (L.d.ny + by - 1) / by, L.d.nz);
     k_coef_classes<<<grid, dim3(bx, by), 0, s>>>(g, dims, L.w[0], L.w[1], L.w[2], L.mask, L.h2inv[0], L.h2inv[1],
                                                   L.h2inv[2], L.coef, want16 ? L.coef16 : nullptr, m.cls_ptr,
-                                                  m.cls_pitch, m.gco);
+                                                  m.cls_pitch, m.gco, m.rk, m.rinv);
     FF_TRY(post("coef_classes"));
     if (bricks) {
         dim3 bg(g.bnx, g.bny, (L.d.nz + BZ - 1) / BZ);
@@ -2539,6 +2643,9 @@ int sweep_tma(const Level &L, const SweepMaps &m, const uint8_t *bricks, int in,
     a.rdreg_sor = sor / a.g.dreg;
     a.omsor = 1.f - sor;
     a.gco = m.gco;
+    a.rk = m.rk;
+    a.rinv = m.rinv;
+    a.quads = L.d.n() / 4;
     a.order = m.order;
     a.colour_a = colour_a;
     a.zc = sweep_planes(L.d, sm_count, rz_mode != 0);
@@ -2551,13 +2658,14 @@ int sweep_tma(const Level &L, const SweepMaps &m, const uint8_t *bricks, int in,
     a.gy = (L.d.ny + tq::TY - 1) / tq::TY;
     dim3 grid(a.gx * a.gy * ((L.d.nz + a.zc - 1) / a.zc));
     const CUtensorMap &xm = m.x[in < 0 ? out : in];
-    const bool rz = rz_mode != 0;
+    const bool rz = rz_mode != 0, pairs = m.rk != nullptr;
+    auto go = [&](auto kernel) { return launch_pdl(kernel, grid, dim3(tq::NT), tq::SMEM, s, a, xm, m.b, m.cls); };
     if (in < 0) {
-        if (rz) FF_CUDA(launch_pdl(k_sweep_tma<true, true>, grid, dim3(tq::NT), tq::SMEM, s, a, xm, m.b, m.cls));
-        else FF_CUDA(launch_pdl(k_sweep_tma<true, false>, grid, dim3(tq::NT), tq::SMEM, s, a, xm, m.b, m.cls));
+        if (rz) FF_CUDA(pairs ? go(k_sweep_tma<true, true, true>) : go(k_sweep_tma<true, true, false>));
+        else FF_CUDA(pairs ? go(k_sweep_tma<true, false, true>) : go(k_sweep_tma<true, false, false>));
     } else {
-        if (rz) FF_CUDA(launch_pdl(k_sweep_tma<false, true>, grid, dim3(tq::NT), tq::SMEM, s, a, xm, m.b, m.cls));
-        else FF_CUDA(launch_pdl(k_sweep_tma<false, false>, grid, dim3(tq::NT), tq::SMEM, s, a, xm, m.b, m.cls));
+        if (rz) FF_CUDA(pairs ? go(k_sweep_tma<false, true, true>) : go(k_sweep_tma<false, true, false>));
+        else FF_CUDA(pairs ? go(k_sweep_tma<false, false, true>) : go(k_sweep_tma<false, false, false>));
     }
     return post("sweep_tma");
 }
@@ -2629,10 +2737,14 @@ int fused_configure() {
     FF_CUDA(cudaFuncSetAttribute(k_sweep<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sweep_smem()));
     FF_CUDA(cudaFuncSetAttribute(k_sweep<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sweep_smem()));
     FF_CUDA(cudaFuncSetAttribute(k_sweep<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sweep_smem()));
-    FF_CUDA(cudaFuncSetAttribute(k_sweep_tma<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tq::SMEM));
-    FF_CUDA(cudaFuncSetAttribute(k_sweep_tma<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tq::SMEM));
-    FF_CUDA(cudaFuncSetAttribute(k_sweep_tma<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tq::SMEM));
-    FF_CUDA(cudaFuncSetAttribute(k_sweep_tma<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tq::SMEM));
+    FF_CUDA(cudaFuncSetAttribute(k_sweep_tma<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tq::SMEM));
+    FF_CUDA(cudaFuncSetAttribute(k_sweep_tma<true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tq::SMEM));
+    FF_CUDA(cudaFuncSetAttribute(k_sweep_tma<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tq::SMEM));
+    FF_CUDA(cudaFuncSetAttribute(k_sweep_tma<true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tq::SMEM));
+    FF_CUDA(cudaFuncSetAttribute(k_sweep_tma<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tq::SMEM));
+    FF_CUDA(cudaFuncSetAttribute(k_sweep_tma<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tq::SMEM));
+    FF_CUDA(cudaFuncSetAttribute(k_sweep_tma<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tq::SMEM));
+    FF_CUDA(cudaFuncSetAttribute(k_sweep_tma<false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tq::SMEM));
     FF_CUDA(cudaFuncSetAttribute(k_res_restrict, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rr_smem()));
     FF_CUDA(cudaFuncSetAttribute(k_p_pap, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p_pap_smem()));
     FF_CUDA(cudaFuncSetAttribute(k_p_pap_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tcg::PAP_SMEM));

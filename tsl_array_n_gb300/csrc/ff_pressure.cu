@@ -328,6 +328,8 @@ extern "C" int ff_pressure3_destroy(ff_pressure ps) {
         for (size_t l = 0; l < ps->lv.size(); ++l) {
             ff_dev_free(ps->smaps[l].cls_ptr);
             ff_dev_free(ps->smaps[l].gco);
+            ff_dev_free(ps->smaps[l].rk);
+            ff_dev_free(ps->smaps[l].rinv);
             ff_dev_free(ps->smaps[l].order);
             ff_dev_free(ps->smaps[l].order_pap);
             ff_dev_free(ps->smaps[l].order_xr);
@@ -550,6 +552,21 @@ static int input_hash(ff_pressure ps, unsigned long long *out) {
     return FF_OK;
 }
 
+// Face weights make cells of class 3 everywhere: their levels' sweeps read the
+// couplings as planes, kept from the first time that there are such weights.
+static int alloc_pair_planes(ff_pressure ps, bool *fresh) {
+    for (size_t l = 0; ps->smaps && l < ps->lv.size(); ++l) {
+        SweepMaps &m = ps->smaps[l];
+        if (!m.ok || m.rk) continue;
+        const size_t quads = (size_t)ps->lv[l].d.n() / 4;
+        if (!*fresh) destroy_graphs(ps);
+        *fresh = true;
+        FF_TRY(ff_dev_alloc((void **)&m.rinv, quads * 2 * sizeof(float2), ps->s()));
+        FF_TRY(ff_dev_alloc((void **)&m.rk, quads * 6 * sizeof(float4), ps->s()));
+    }
+    return FF_OK;
+}
+
 static int prepare(ff_pressure ps, ff_field u, ff_field v, ff_field w) {
     cudaStream_t s = ps->s();
     const Dims &d = ps->d;
@@ -559,7 +576,9 @@ static int prepare(ff_pressure ps, ff_field u, ff_field v, ff_field w) {
     // the operator's inputs unchanged since the last prepare: only b is new
     unsigned long long h = 0;
     FF_TRY(input_hash(ps, &h));
-    const bool reuse = ps->prepared && h == ps->input_hash;
+    bool planes = false;
+    if (fw[0]) FF_TRY(alloc_pair_planes(ps, &planes));
+    const bool reuse = ps->prepared && h == ps->input_hash && !planes;
     // updateDirichletFields (grid_pressure_solver3.js:171-206)
     ps->has_mask = ps->active || cw[0];
     // a zero mask is the same operator as no mask, so level 0 always reads
