@@ -11,6 +11,7 @@
 // (computeFlipBoxSeed3, mulberry32) is computed in doubles as JavaScript
 // does (-ffp-contract=off on the host compiler).
 #include "ff_grid.cuh"
+#include "ff_window.h"
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -102,7 +103,6 @@ __device__ __forceinline__ unsigned long long p2g_pack(int num, int den) {
 // them the window adds (2.4 bank passes each), half the global adds of the
 // eighth outside the windows, one lane each.
 constexpr int P2G_NT = 512, P2G_MAX_ROUNDS = 8;
-constexpr int P2G_CAP = 3096;   // window faces per component: 258 x 4 x 3, two rows of 256 cells
 
 // the value of rank r among the 32 lanes' values
 __device__ __forceinline__ int warp_rank_value(int v, int r) {
@@ -127,25 +127,14 @@ __global__ void __launch_bounds__(P2G_NT, 3) k_flip_scatter(G3 g, long long n, i
         const long long p = base + (long long)threadIdx.x * (count - 1) / 31;
         const float org[3] = {g.ox, g.oy, g.oz}, hh[3] = {g.hx, g.hy, g.hz};
         const int nn[3] = {g.nx, g.ny, g.nz};
-        int lo[3], w[3];
+        int q20[3], q80[3], lo[3], w[3];
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
             const int c = iclamp((int)floorf(gclamp((pos[3 * p + b] - org[b]) / hh[b])), 0, nn[b] - 1);
-            const int q20 = warp_rank_value(c, 6), q80 = warp_rank_value(c, 25), ext = (q80 - q20 + 2) / 3;
-            lo[b] = max(q20 - ext, 0);
-            w[b] = min(q80 + ext, nn[b] - 1) - lo[b] + 1;
+            q20[b] = warp_rank_value(c, 6);
+            q80[b] = warp_rank_value(c, 25);
         }
-        // faces from one below the first cell to one above the last
-        while ((w[0] + 2) * (w[1] + 2) * (w[2] + 2) > P2G_CAP) {
-            const int b = w[0] >= w[1] ? (w[0] >= w[2] ? 0 : 2) : (w[1] >= w[2] ? 1 : 2);
-            const int cut = max(1, w[b] / 16);
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-                if (q == b) {
-                    lo[q] += cut / 2;
-                    w[q] -= cut;
-                }
-        }
+        p2g_window(q20, q80, nn, lo, w);
         if (threadIdx.x < 3) {
             wlo[threadIdx.x] = (threadIdx.x == 0 ? lo[0] : (threadIdx.x == 1 ? lo[1] : lo[2])) - 1;
             wn[threadIdx.x] = (threadIdx.x == 0 ? w[0] : (threadIdx.x == 1 ? w[1] : w[2])) + 2;
