@@ -715,7 +715,7 @@ static int vcycle(ff_pressure ps, int l, const PcgState *st) {
             return ffk::mg_coarse_direct(v, ps->G, ps->nG, xbf, bbf, st, ps->s());
         }
         long long n = v.d.n();
-        if (vb == 0 && ps->cluster > 0 && ps->use_tail) {
+        if (vb == 0 && ps->cluster > 0 && ps->use_tail && ps->desc.mg_coarsest > 0) {
             bool done = false;
             FF_TRY(ffk::coarse_cluster(v, ps->dims, ps->desc.mg_coarsest, (float)ps->desc.mg_sor, st, ps->cluster, done,
                                        ps->s()));
@@ -796,7 +796,7 @@ static int vcycle_fused(ff_pressure ps, int l, PcgState *st, int rz_mode, float 
             FF_TRY(ffk::mg_coarse_direct(v, ps->G, ps->nG, 0, 0, st, s));
         } else if (v.d.n() <= 16384) {
             bool done = false;
-            if (ps->cluster > 0 && ps->use_tail)
+            if (ps->cluster > 0 && ps->use_tail && ps->desc.mg_coarsest > 0)
                 FF_TRY(ffk::coarse_cluster(v, ps->dims, ps->desc.mg_coarsest, sor, st, ps->cluster, done, s));
             if (!done) {
                 FF_CUDA(cudaMemsetAsync(v.x, 0, (size_t)v.d.n() * 4, s));
