@@ -16,6 +16,9 @@
 
 namespace {
 int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
+// blocks of the whole-array sums beside the solve (the start's norm, a guess's
+// residual): one partial sum each, whatever the array's size
+constexpr int SUM_BLOCKS = 256;
 }
 
 struct ff_pressure_s {
@@ -308,8 +311,8 @@ extern "C" int ff_pressure3_create(ff_ctx ctx, const ff_pressure_desc *desc, ff_
         m.cls_pitch = (int)ffk::cls_row_pitch(ps->lv[l].d);
     }
     // (one launch keeps the sums of p.Ap, r.r with b.b, and r.z apart)
-    if ((st = ff_dev_alloc((void **)&ps->partials, (size_t)blocks * (ps->resident_fits ? 4 : 2) * sizeof(double), s)))
-        return bail(st);
+    const size_t partials = std::max((size_t)blocks * (ps->resident_fits ? 4 : 2), (size_t)SUM_BLOCKS);
+    if ((st = ff_dev_alloc((void **)&ps->partials, partials * sizeof(double), s))) return bail(st);
     if (ps->smaps && ps->smaps[0].ok &&
         (st = ffk::cg_tma_maps(ps->lv[0], (const float *)ps->z, ps->x2[0], ps->p0, ps->p1, ps->xh0(), ps->x_lo0,
                                ps->x_hi1, ps->x_lo1, (const float *)ps->bfield->d, ps->ds(), ps->cgm)))
@@ -1119,7 +1122,7 @@ static int residual_sq(ff_pressure ps, const float *x, float *ax, double *out) {
     cudaStream_t s = ps->s();
     const long long n = ps->d.n();
     FF_TRY(ffk::laplacian_apply(ps->d, ps->lv[0].coef, x, ax, s));
-    const int nb = 256;
+    const int nb = SUM_BLOCKS;
     k_res_sumsq<<<nb, 256, 0, s>>>(n, (const float *)ps->bfield->d, ax, ps->partials);
     FF_CUDA(cudaGetLastError());
     std::vector<double> hp(nb);
@@ -1135,7 +1138,7 @@ static int residual_sq(ff_pressure ps, const float *x, float *ax, double *out) {
 // linalg.js:884-905)
 static int start_norm(ff_pressure ps) {
     cudaStream_t s = ps->s();
-    const int nb = 256;
+    const int nb = SUM_BLOCKS;
     k_iterate_sumsq<<<nb, 256, 0, s>>>(ps->d.n(), ps->xh0(), ps->x_lo0, ps->partials);
     FF_CUDA(cudaGetLastError());
     std::vector<double> hp(nb);
