@@ -34,11 +34,16 @@ int ff_dev_alloc(void **p, size_t bytes, cudaStream_t s) {
     cudaError_t e = cudaMalloc(p, padded);
     if (e != cudaSuccess) {
         *p = nullptr;
+        (void)cudaGetLastError();   // (reported here, not by the next launch's check)
         return ff_set_error(e == cudaErrorMemoryAllocation ? FF_E_NOMEM : FF_E_CUDA,
                             "cudaMalloc(%zu): %s", padded, cudaGetErrorString(e));
     }
     e = cudaMemsetAsync(*p, 0, padded, s);
-    if (e != cudaSuccess) return ff_set_error(FF_E_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        ff_dev_free(*p);
+        *p = nullptr;
+        return ff_set_error(FF_E_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
+    }
     return FF_OK;
 }
 

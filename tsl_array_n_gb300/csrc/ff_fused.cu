@@ -2601,7 +2601,7 @@ int coef_classes(const Level &L, const SweepMaps &m, uint8_t *bricks, int dims, 
     dim3 grid((L.d.nx + bx - 1) / bx, (L.d.ny + by - 1) / by, L.d.nz);
     k_coef_classes<<<grid, dim3(bx, by), 0, s>>>(g, dims, L.w[0], L.w[1], L.w[2], L.mask, L.h2inv[0], L.h2inv[1],
                                                   L.h2inv[2], L.coef, want16 ? L.coef16 : nullptr, m.cls_ptr,
-                                                  m.cls_pitch, m.gco, m.rk, m.rinv);
+                                                  m.cls_pitch, m.gco, m.planes ? m.rk : nullptr, m.rinv);
     FF_TRY(post("coef_classes"));
     if (bricks) {
         dim3 bg(g.bnx, g.bny, (L.d.nz + BZ - 1) / BZ);
@@ -2658,7 +2658,7 @@ int sweep_tma(const Level &L, const SweepMaps &m, const uint8_t *bricks, int in,
     a.gy = (L.d.ny + tq::TY - 1) / tq::TY;
     dim3 grid(a.gx * a.gy * ((L.d.nz + a.zc - 1) / a.zc));
     const CUtensorMap &xm = m.x[in < 0 ? out : in];
-    const bool rz = rz_mode != 0, pairs = m.rk != nullptr;
+    const bool rz = rz_mode != 0, pairs = m.planes;
     auto go = [&](auto kernel) { return launch_pdl(kernel, grid, dim3(tq::NT), tq::SMEM, s, a, xm, m.b, m.cls); };
     if (in < 0) {
         if (rz) FF_CUDA(pairs ? go(k_sweep_tma<true, true, true>) : go(k_sweep_tma<true, true, false>));

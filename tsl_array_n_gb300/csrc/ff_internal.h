@@ -140,12 +140,14 @@ struct SweepMaps {
     // per cell of class 3: couplings across the upper x, y, z faces and the
     // reciprocal of the diagonal (other cells' entries are not written)
     float4 *gco = nullptr;
-    // with face weights (else null): the same couplings as the sweep's colour passes
-    // read them (class-3 cells' entries only): of the two cells of an x-quad with one parity P of i, (lower x of
-    // both, upper x of both), y and z likewise, 1 / diagonal of both; entry
-    // (axis * 2 + P) * quads + quad, and P * quads + quad of rinv
+    // the same couplings as the sweep's colour passes read them with face weights
+    // (class-3 cells' entries only): of the two cells of an x-quad with one parity P of
+    // i, (lower x of both, upper x of both), y and z likewise, 1 / diagonal of both;
+    // entry (axis * 2 + P) * quads + quad, and P * quads + quad of rinv.  Null until they
+    // are first used; planes: written with the coefficients and read by the sweeps
     float4 *rk = nullptr;
     float2 *rinv = nullptr;
+    bool planes = false;
     // work order of the sweep's blocks (tile columns x z-chunks, those with
     // non-plain cells first)
     int *order = nullptr;

@@ -8,6 +8,7 @@
 // iteration cap), so the host waits once per solve instead of once per chunk
 // (linalg.js:1817-1911).
 #include "ff_internal.h"
+#include "ff_pairalloc.h"
 #include <nvtx3/nvToolsExt.h>
 #include <algorithm>
 #include <cmath>
@@ -67,6 +68,7 @@ struct ff_pressure_s {
     int cluster = 0;                // blocks of a cluster (the solve and the coarsest sweeps on one)
     bool use_tail = true;
     unsigned *tail_bar = nullptr;   // the grid barrier: arrivals, blocks done, abort
+    bool planes_tried = false;      // room for the coupling planes was asked for (pair_planes)
     // learned warm start (borrowed network), its guess field, last choice
     ff_unet net = nullptr;
     ff_field guess = nullptr;
@@ -457,6 +459,29 @@ extern "C" int ff_pressure3_fields(ff_pressure ps, ff_field *pressure, ff_field 
     return FF_OK;
 }
 
+// the level-0 CG kernels run in the TMA layout when the sweep does
+static bool cg_tma(const ff_pressure ps) { return ps->use_tma && ps->cgm.ok && ps->smaps && ps->smaps[0].ok; }
+
+// The whole solve in one launch: a multigrid-preconditioned solve with a
+// small level 0, with none of the settings that ask for the separate
+// kernels, whose results it gives bit for bit (a rounding of its own would, in a
+// slowly converging solve, now and then end it an iteration earlier or later).
+// Measured against the graph of separate launches (whole projection): 48 x 24 x 24
+// 1.32 -> 0.45 ms, 2D 128^2 3.73 -> 1.25, 1024 x 256 channel step 16.2 -> 9.6.  The
+// line lies where the two meet: 96^3 3.32 -> 3.10 ms (10.9 -> 9.3 with variable
+// density), 1024 x 768 19.7 -> 18.3, 1024^2 25.3 -> 23.6, 128 x 96 x 96 (1.2M cells)
+// 6.69 against 6.67.
+static bool one_launch(const ff_pressure ps) {
+    return ps->resident_fits && ps->use_graph && cg_tma(ps) && ps->use_tail &&
+           ps->desc.preconditioner == FF_PRE_MULTIGRID && ps->desc.mg_down > 0 && ps->desc.mg_final > 0 &&
+           (ps->desc.mg_coarse_mode == FF_COARSE_DIRECT || ps->desc.mg_coarsest > 0);
+}
+// (a direct coarsest solve needs its factorisation, which a prepare with another
+// preconditioner does not make)
+static bool resident(const ff_pressure ps) {
+    return one_launch(ps) && (ps->desc.mg_coarse_mode != FF_COARSE_DIRECT || ps->G != nullptr);
+}
+
 // --------------------------------------------------------------- prepare --
 static const float *fptr(ff_field f) { return f ? (const float *)f->d : nullptr; }
 
@@ -555,19 +580,31 @@ static int input_hash(ff_pressure ps, unsigned long long *out) {
     return FF_OK;
 }
 
-// Face weights make cells of class 3 everywhere: their levels' sweeps read the
-// couplings as planes, kept from the first time that there are such weights.
-static int alloc_pair_planes(ff_pressure ps, bool *fresh) {
-    for (size_t l = 0; ps->smaps && l < ps->lv.size(); ++l) {
+// Face weights make cells of class 3 everywhere, and the sweeps of separate launches
+// then read the couplings as planes: those of a solve that is not one launch, with
+// multigrid on the TMA sweeps.  The planes come with the first such prepare, stay for
+// as long as there are face weights, and are out of use without them (a solver with few
+// class-3 cells is faster per cell).  A level whose planes find no memory keeps the form
+// per cell, the same results.  changed: some level goes over to the other form.
+static void pair_planes(ff_pressure ps, bool *changed) {
+    *changed = false;
+    if (!ps->smaps) return;
+    const bool sweeps = ps->use_tma && ps->desc.preconditioner == FF_PRE_MULTIGRID && !one_launch(ps);
+    if (!ps->fw[0]) ps->planes_tried = false;
+    for (size_t l = 0; l < ps->lv.size(); ++l) {
         SweepMaps &m = ps->smaps[l];
-        if (!m.ok || m.rk) continue;
-        const size_t quads = (size_t)ps->lv[l].d.n() / 4;
-        if (!*fresh) destroy_graphs(ps);
-        *fresh = true;
-        FF_TRY(ff_dev_alloc((void **)&m.rinv, quads * 2 * sizeof(float2), ps->s()));
-        FF_TRY(ff_dev_alloc((void **)&m.rk, quads * 6 * sizeof(float4), ps->s()));
+        if (!m.ok) continue;
+        if (ps->fw[0] && sweeps && !m.rk && !ps->planes_tried) {
+            const size_t quads = (size_t)ps->lv[l].d.n() / 4;
+            alloc_both((void **)&m.rk, quads * 6 * sizeof(float4), (void **)&m.rinv, quads * 2 * sizeof(float2),
+                       [&](void **p, size_t bytes) { return ff_dev_alloc(p, bytes, ps->s()); }, ff_dev_free);
+        }
+        const bool use = ps->fw[0] && m.rk && (sweeps || m.planes);
+        *changed = *changed || use != m.planes;
+        m.planes = use;
     }
-    return FF_OK;
+    if (ps->fw[0] && sweeps) ps->planes_tried = true;
+    if (*changed) destroy_graphs(ps);
 }
 
 static int prepare(ff_pressure ps, ff_field u, ff_field v, ff_field w) {
@@ -580,8 +617,9 @@ static int prepare(ff_pressure ps, ff_field u, ff_field v, ff_field w) {
     unsigned long long h = 0;
     FF_TRY(input_hash(ps, &h));
     bool planes = false;
-    if (fw[0]) FF_TRY(alloc_pair_planes(ps, &planes));
+    pair_planes(ps, &planes);
     const bool reuse = ps->prepared && h == ps->input_hash && !planes;
+    if (!reuse) ps->prepared = false;   // (until the last level is built)
     // updateDirichletFields (grid_pressure_solver3.js:171-206)
     ps->has_mask = ps->active || cw[0];
     // a zero mask is the same operator as no mask, so level 0 always reads
@@ -892,9 +930,6 @@ static int reset_tail_bar(ff_pressure ps) {
     return FF_OK;
 }
 
-// the level-0 CG kernels run in the TMA layout when the sweep does
-static bool cg_tma(const ff_pressure ps) { return ps->use_tma && ps->cgm.ok && ps->smaps && ps->smaps[0].ok; }
-
 static int enqueue_setup(ff_pressure ps) {
     const Dims &d = ps->d;
     cudaStream_t s = ps->s();
@@ -983,21 +1018,6 @@ static int build_graphs(ff_pressure ps) {
     FF_CUDA(e);
     FF_CUDA(cudaGraphInstantiate(&ps->loop_exec, lg, 0));
     return FF_OK;
-}
-
-// The whole solve in one launch: a multigrid-preconditioned solve with a
-// small level 0, with none of the settings that ask for the separate
-// kernels, whose results it gives bit for bit (a rounding of its own would, in a
-// slowly converging solve, now and then end it an iteration earlier or later).
-// Measured against the graph of separate launches (whole projection): 48 x 24 x 24
-// 1.32 -> 0.45 ms, 2D 128^2 3.73 -> 1.25, 1024 x 256 channel step 16.2 -> 9.6.  The
-// line lies where the two meet: 96^3 3.32 -> 3.10 ms (10.9 -> 9.3 with variable
-// density), 1024 x 768 19.7 -> 18.3, 1024^2 25.3 -> 23.6, 128 x 96 x 96 (1.2M cells)
-// 6.69 against 6.67.
-static bool resident(const ff_pressure ps) {
-    return ps->resident_fits && ps->use_graph && cg_tma(ps) && ps->use_tail &&
-           ps->desc.preconditioner == FF_PRE_MULTIGRID && ps->desc.mg_down > 0 && ps->desc.mg_final > 0 &&
-           (ps->desc.mg_coarse_mode == FF_COARSE_DIRECT ? ps->G != nullptr : ps->desc.mg_coarsest > 0);
 }
 
 static int run_solve(ff_pressure ps) {
