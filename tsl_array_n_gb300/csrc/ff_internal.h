@@ -269,10 +269,10 @@ int vcycle_tail(const Level *lv, const SweepMaps *sm, int nl, int dims, int down
 // cluster: blocks of one cluster that the device can run (cluster_blocks()), 0: none
 constexpr long long PCG_RESIDENT_CELLS = 1LL << 20;
 int cluster_blocks();
-// the sweeps of a coarsest FP32 level from x = 0 (mg_relax's arithmetic) in one launch on a
-// cluster; done: false and nothing launched where the level does not fit one
-int coarse_cluster(const Level &L, int dims, int sweeps, float sor, const PcgState *st, int cluster, bool &done,
-                   cudaStream_t s);
+// the sweeps (one or more) of a coarsest FP32 level from x = 0 (mg_relax's arithmetic)
+// in one launch on a cluster, where the level fits one
+bool coarse_cluster_fits(const Level &L, int dims, int sweeps, int cluster);
+int coarse_cluster(const Level &L, int dims, int sweeps, float sor, const PcgState *st, int cluster, cudaStream_t s);
 int pcg_resident(const Level *lv, const SweepMaps *sm, int nl, int dims, int down, int up, int fin, float sor,
                  const double *G, int nG, int coarse_sweeps, const float *b, float *p0, float *p1, float *xh0, float *xl0,
                  float *xh1, float *xl1, int ds, PcgState *st, double *partials, unsigned *bar, int sm_count,

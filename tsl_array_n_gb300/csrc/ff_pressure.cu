@@ -743,6 +743,12 @@ static int zero_x(ff_pressure ps, int l) {
     return FF_OK;
 }
 
+// the coarsest level's sweeps in one launch on a cluster (FP32 storage)
+static bool coarsest_on_cluster(const ff_pressure ps) {
+    return !ps->vbf() && ps->cluster > 0 && ps->use_tail && ps->desc.mg_coarsest > 0 &&
+           ffk::coarse_cluster_fits(ps->lv.back(), ps->dims, ps->desc.mg_coarsest, ps->cluster);
+}
+
 // vCycle (multigrid.js:1609-1642); x of `l` is zero on entry.  Storage:
 // level-0 x (z) and b (r) are FP32; coarse x, b and every residual buffer
 // take the V-cycle storage type.
@@ -756,12 +762,8 @@ static int vcycle(ff_pressure ps, int l, const PcgState *st) {
             return ffk::mg_coarse_direct(v, ps->G, ps->nG, xbf, bbf, st, ps->s());
         }
         long long n = v.d.n();
-        if (vb == 0 && ps->cluster > 0 && ps->use_tail && ps->desc.mg_coarsest > 0) {
-            bool done = false;
-            FF_TRY(ffk::coarse_cluster(v, ps->dims, ps->desc.mg_coarsest, (float)ps->desc.mg_sor, st, ps->cluster, done,
-                                       ps->s()));
-            if (done) return FF_OK;
-        }
+        if (coarsest_on_cluster(ps))
+            return ffk::coarse_cluster(v, ps->dims, ps->desc.mg_coarsest, (float)ps->desc.mg_sor, st, ps->cluster, ps->s());
         if (n <= 16384) {
             if (l == 0) FF_TRY(zero_x(ps, 0));
             return ffk::mg_coarse_sweeps(v, ps->dims, ps->desc.mg_coarsest, (float)ps->desc.mg_sor, xbf,
@@ -789,6 +791,14 @@ static int vcycle(ff_pressure ps, int l, const PcgState *st) {
     return relax_level(ps, l, l > 0 ? ps->desc.mg_up : ps->desc.mg_final, true, nf, st);
 }
 
+// whether level l and every coarser one run in one launch
+static bool tail_from(const ff_pressure ps, int l) {
+    return l == ps->tail_l && ps->use_tail && l > 0 && ps->tail_bar &&
+           (ps->desc.mg_coarse_mode == FF_COARSE_DIRECT ? ps->G != nullptr : ps->desc.mg_coarsest > 0);
+}
+// whether level l's sweeps (and with a residual buffer its restriction) are the TMA ones
+static bool level_tma(const ff_pressure ps, int l) { return ps->use_tma && ps->smaps && ps->smaps[l].ok; }
+
 // The FP32 V-cycle on fused sweeps.  Every sweep is out of place, so each
 // level alternates between its two x buffers; the sequence is static, so
 // where each level's result lands is known when the work is enqueued.
@@ -802,7 +812,7 @@ static int level_sweep(ff_pressure ps, int l, PcgState *st, float *const bufs[2]
                        int rz_mode) {
     Level &v = ps->lv[l];
     const float sor = (float)ps->desc.mg_sor;
-    if (ps->use_tma && ps->smaps && ps->smaps[l].ok) {
+    if (level_tma(ps, l)) {
         // descriptors index the buffers as {level x, second buffer}
         const int in = cur < 0 ? -1 : (bufs[cur] == ps->smaps[l].xp[0] ? 0 : 1);
         const int out = in == 0 ? 1 : 0;
@@ -823,8 +833,7 @@ static int vcycle_fused(ff_pressure ps, int l, PcgState *st, int rz_mode, float 
     int cur = -1;   // -1: x is identically zero
     *rz_done = false;
     const bool direct = ps->desc.mg_coarse_mode == FF_COARSE_DIRECT;
-    if (l == ps->tail_l && ps->use_tail && l > 0 && ps->tail_bar &&
-        (direct ? ps->G != nullptr : ps->desc.mg_coarsest > 0)) {
+    if (tail_from(ps, l)) {
         // this level and every coarser one in one cooperative launch
         FF_TRY(ffk::vcycle_tail(&ps->lv[l], &ps->smaps[l], Ln - l, ps->dims, ps->desc.mg_down, ps->desc.mg_up, sor,
                                 direct ? ps->G : nullptr, direct ? ps->nG : 0, direct ? 0 : ps->desc.mg_coarsest, st,
@@ -836,10 +845,9 @@ static int vcycle_fused(ff_pressure ps, int l, PcgState *st, int rz_mode, float 
         if (ps->desc.mg_coarse_mode == FF_COARSE_DIRECT) {
             FF_TRY(ffk::mg_coarse_direct(v, ps->G, ps->nG, 0, 0, st, s));
         } else if (v.d.n() <= 16384) {
-            bool done = false;
-            if (ps->cluster > 0 && ps->use_tail && ps->desc.mg_coarsest > 0)
-                FF_TRY(ffk::coarse_cluster(v, ps->dims, ps->desc.mg_coarsest, sor, st, ps->cluster, done, s));
-            if (!done) {
+            if (coarsest_on_cluster(ps)) {
+                FF_TRY(ffk::coarse_cluster(v, ps->dims, ps->desc.mg_coarsest, sor, st, ps->cluster, s));
+            } else {
                 FF_CUDA(cudaMemsetAsync(v.x, 0, (size_t)v.d.n() * 4, s));
                 FF_TRY(ffk::mg_coarse_sweeps(v, ps->dims, ps->desc.mg_coarsest, sor, 0, 0, 0, st, s));
             }
@@ -867,7 +875,7 @@ static int vcycle_fused(ff_pressure ps, int l, PcgState *st, int rz_mode, float 
     }
     // residual and restriction into the coarse b, fused (the fine residual
     // never reaches memory)
-    if (ps->use_tma && ps->smaps && ps->smaps[l].ok && v.buf)
+    if (level_tma(ps, l) && v.buf)
         FF_TRY(ffk::res_restrict2(v, ps->smaps[l], bufs[cur], (float *)v.buf, c, ps->dims, st, s));
     else
         FF_TRY(ffk::res_restrict(v, ps->bricks[l], bufs[cur], c, ps->dims, st, ps->ctx->sm_count, s));
@@ -1292,21 +1300,24 @@ extern "C" int ff_pressure3_project_host(ff_pressure ps, ff_field u_in, ff_field
     return FF_OK;
 }
 
-// kernel launches of one V-cycle, as vcycle() below enqueues them
+// kernel launches of one V-cycle, as vcycle() or vcycle_fused() enqueues them
 static int vcycle_launches(ff_pressure ps) {
-    const int Ln = (int)ps->lv.size();
+    const int Ln = (int)ps->lv.size(), colours = ps->fused ? 1 : 2;   // launches a sweep
     int n = 0;
     for (int l = 0; l < Ln - 1; ++l) {
-        n += 2 * ps->desc.mg_down + 3 + 2 * (l > 0 ? ps->desc.mg_up : ps->desc.mg_final);
+        if (ps->fused && tail_from(ps, l)) return n + 1;
+        const int transfers = !ps->fused || (level_tma(ps, l) && ps->lv[l].buf) ? 3 : 2;
+        n += transfers + colours * (ps->desc.mg_down + (l > 0 ? ps->desc.mg_up : ps->desc.mg_final));
     }
-    const Level &c = ps->lv[Ln - 1];
-    if (ps->desc.mg_coarse_mode == FF_COARSE_DIRECT || c.d.n() <= 16384) n += 1;
-    else n += 2 * ps->desc.mg_coarsest;
-    return n;
+    const bool one = ps->desc.mg_coarse_mode == FF_COARSE_DIRECT || ps->lv[Ln - 1].d.n() <= 16384 ||
+                     (!ps->fused && coarsest_on_cluster(ps));
+    return n + (one ? 1 : colours * ps->desc.mg_coarsest);
 }
 
+// the preconditioner's launches, and that of r.z where the V-cycle's last sweep has not formed it
 static int precond_launches(ff_pressure ps) {
-    return ps->desc.preconditioner == FF_PRE_MULTIGRID ? vcycle_launches(ps) : 1;
+    if (ps->desc.preconditioner != FF_PRE_MULTIGRID) return 2;
+    return vcycle_launches(ps) + (ps->fused && ps->lv.size() > 1 && ps->desc.mg_final > 0 ? 0 : 1);
 }
 
 // prepare(): Dirichlet fields, system weights, build, per-level coarsening
@@ -1361,11 +1372,13 @@ static int read_diag(ff_pressure ps, ff_diag *diag, int extra_launches) {
             diag->floor_threshold = thr;
             diag->tolerance_below_floor = thr < fl ? 1 : 0;
         }
-        // setup: state init, residual, preconditioner, r.z; then each loop
-        // body the device ran: p/pAp, x/residual, preconditioner, r.z, control
-        int per_iter = 4 + precond_launches(ps);
-        diag->kernel_launches = resident(ps) ? extra_launches + 2
-                                             : extra_launches + 3 + precond_launches(ps) + h.launched * per_iter;
+        // setup: state init, residual, preconditioner with r.z; then each loop
+        // body the device ran: p/pAp, x/residual, preconditioner with r.z, control
+        diag->kernel_launches = extra_launches + 2;
+        if (!resident(ps)) {
+            const int m = precond_launches(ps);
+            diag->kernel_launches += m + h.launched * (3 + m);
+        }
     }
     return FF_OK;
 }

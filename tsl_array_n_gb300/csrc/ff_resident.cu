@@ -2466,13 +2466,21 @@ int vcycle_tail(const Level *lv, const SweepMaps *sm, int nl, int dims, int down
                   smem, s, args);
 }
 
-int coarse_cluster(const Level &L, int dims, int sweeps, float sor, const PcgState *st, int cluster, bool &done,
-                   cudaStream_t s) {
+// (up to 2 NT cells: one block)
+static int coarse_blocks(const Level &L, int cluster) { return L.d.n() <= 2 * NT ? 1 : cluster; }
+
+bool coarse_cluster_fits(const Level &L, int dims, int sweeps, int cluster) {
     int smem = 0;
-    const int csize = L.d.n() <= 2 * NT ? 1 : cluster;
+    const int csize = coarse_blocks(L, cluster);
+    return csize == 1 ||
+           make_args(&L, nullptr, 1, dims, 0, 0, 0, 1.f, nullptr, 0, sweeps, nullptr, csize, false, 0, smem).ccoarse;
+}
+
+int coarse_cluster(const Level &L, int dims, int sweeps, float sor, const PcgState *st, int cluster, cudaStream_t s) {
+    int smem = 0;
+    const int csize = coarse_blocks(L, cluster);
     VArgs a = make_args(&L, nullptr, 1, dims, 0, 0, 0, sor, nullptr, 0, sweeps, nullptr, csize, false, 0, smem);
-    done = csize == 1 || a.ccoarse;
-    if (!done) return FF_OK;
+    FF_CHECK(sweeps > 0 && (csize == 1 || a.ccoarse), FF_E_STATE, "coarsest sweeps: the level does not fit a cluster");
     void *args[] = {&a, &st};
     return launch(dims == 3 ? (const void *)k_coarse_cluster<true> : (const void *)k_coarse_cluster<false>, csize, csize, smem,
                   s, args);
