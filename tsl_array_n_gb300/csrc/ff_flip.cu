@@ -38,13 +38,14 @@ __device__ __forceinline__ long long cell_of(const G3 &g, const float *p) {
 // particles of a one-cell-thick grid standing in for a 2D one stay on their
 // plane (the trace leaves z alone there anyway, except for the rounding of
 // the collider-crossing blend)
-template <bool P2>
-__global__ void k_flip_advect(const __grid_constant__ VelField F, long long n, float *__restrict__ pos, float dt, int max_substeps, F3 mn,
-                              F3 mx, float push_thresh, float push_shift, int keep_z) {
+template <int FORM>
+__global__ void __launch_bounds__(256, 4) k_flip_advect(const __grid_constant__ VelField F, long long n, float *__restrict__ pos,
+                                                        float dt, int max_substeps, F3 mn, F3 mx, float push_thresh,
+                                                        float push_shift, int keep_z) {
     const F3 oc = comp_origin(F.g, 3);
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const F3 prev{pos[3 * p], pos[3 * p + 1], pos[3 * p + 2]};
-        const F3 tr = back_trace<P2>(F, prev, dt, -1.0f, max_substeps, NAN);
+        const F3 tr = trace_back<FORM>(F, prev, dt, -1.0f, max_substeps, NAN);
         const bool bad = nonfinite(tr.x) || nonfinite(tr.y) || nonfinite(tr.z);
         F3 q{fminf(fmaxf(bad ? prev.x : tr.x, mn.x), mx.x), fminf(fmaxf(bad ? prev.y : tr.y, mn.y), mx.y),
              fminf(fmaxf(bad ? prev.z : tr.z, mn.z), mx.z)};
@@ -905,6 +906,14 @@ int post(const char *what) {
     return FF_OK;
 }
 
+void flip_advect(const VelField &F, long long n, float *pos, float dt, int max_substeps, F3 mn, F3 mx, float push_thresh,
+                 float push_shift, int keep_z, cudaStream_t s) {
+    const int form = point_form(F, n);
+    const auto kernel = form == FORM_PLAIN ? k_flip_advect<FORM_PLAIN>
+                        : form == FORM_SHORT ? k_flip_advect<FORM_SHORT> : k_flip_advect<FORM_SHORT_P2>;
+    kernel<<<blocks_for(n), 256, 0, s>>>(F, n, pos, dt, max_substeps, mn, mx, push_thresh, push_shift, keep_z);
+}
+
 Comps3 comps3(const G3 &g, float *const d[3], int ncomp) {
     Comps3 C{};
     for (int a = 0; a < ncomp; ++a) {
@@ -1287,8 +1296,8 @@ extern "C" int ff_flip3_stage(ff_flip f, int stage) {
                      (float)(d.resolution[2] * d.grid_spacing[2])};
         const F3 mn{g.ox + 1e-4f, g.oy + 1e-4f, g.oz + 1e-4f};
         const F3 mx{(g.ox + ext.x) - 1e-4f, (g.oy + ext.y) - 1e-4f, (g.oz + ext.z) - 1e-4f};
-        (F.pow2 ? k_flip_advect<true> : k_flip_advect<false>)<<<blocks_for(n), 256, 0, s>>>(F, n, pos, (float)d.dt, d.max_substeps, mn, mx,
-                                                    (float)d.collider_push_thresh, (float)d.collider_push_shift, 0);
+        flip_advect(F, n, pos, (float)d.dt, d.max_substeps, mn, mx, (float)d.collider_push_thresh,
+                    (float)d.collider_push_shift, 0, s);
         return post("advectParticles");
     }
     case FF_FLIP_P2G:
@@ -1900,9 +1909,8 @@ extern "C" int ff_twophase2_stage(ff_twophase t, int stage) {
         const F3 mx{(g.ox + (float)(d.resolution[0] * d.grid_spacing[0])) - 1e-4f,
                     (g.oy + (float)(d.resolution[1] * d.grid_spacing[1])) - 1e-4f,
                     three ? (g.oz + (float)(d.resolution[2] * d.grid_spacing[2])) - 1e-4f : (g.oz + g.hz) - 1e-4f};
-        (F.pow2 ? k_flip_advect<true> : k_flip_advect<false>)<<<blocks_for(n), 256, 0, s>>>(F, n, pos, (float)d.dt, d.max_substeps, mn, mx,
-                                                    (float)d.collider_push_thresh, (float)d.collider_push_shift,
-                                                    three ? 0 : 1);
+        flip_advect(F, n, pos, (float)d.dt, d.max_substeps, mn, mx, (float)d.collider_push_thresh,
+                    (float)d.collider_push_shift, three ? 0 : 1, s);
         return post("advectParticles");
     }
     case FF_TP_DENSITY:

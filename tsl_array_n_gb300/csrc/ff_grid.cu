@@ -176,22 +176,15 @@ struct AdvectIO {
     const float *src[3], *fwd[3], *bwd[3];
     float *out[3];
 };
-// FORM: the straightforward form of the trace and the samples, or the short one
-enum { ADVECT_PLAIN, ADVECT_SHORT, ADVECT_SHORT_P2 };
 template <int FORM>
 __device__ __forceinline__ float advect_phi(const VelField &F, F3 p) {
-    if constexpr (FORM == ADVECT_PLAIN) return sample_phi(F, F.phi, p);
-    else return trace_phi<FORM == ADVECT_SHORT_P2>(F, p);
-}
-template <int FORM>
-__device__ __forceinline__ F3 advect_trace(const VelField &F, F3 pos, float dt, float dirn, int max_substeps, float phi) {
-    if constexpr (FORM == ADVECT_PLAIN) return back_trace_plain(F, pos, dt, dirn, max_substeps);
-    else return back_trace<FORM == ADVECT_SHORT_P2>(F, pos, dt, dirn, max_substeps, phi);
+    if constexpr (FORM == FORM_PLAIN) return sample_phi(F, F.phi, p);
+    else return trace_phi<FORM == FORM_SHORT_P2>(F, p);
 }
 template <int FORM>
 __device__ __forceinline__ float advect_cubic(const VelField &F, int a, const float *d, int sx, int sy, int sz, F3 o, F3 p) {
-    if constexpr (FORM == ADVECT_PLAIN) return tricubic(d, sx, sy, sz, F.g, o, p);
-    else return trace_cubic<FORM == ADVECT_SHORT_P2>(F, a, d, sx, sy, sz, o, p);
+    if constexpr (FORM == FORM_PLAIN) return tricubic(d, sx, sy, sz, F.g, o, p);
+    else return trace_cubic<FORM == FORM_SHORT_P2>(F, a, d, sx, sy, sz, o, p);
 }
 template <int stage, int FORM>
 __device__ __forceinline__ void advect_at(const VelField &F, int a, const AdvectIO &io, int q, int sx, int sy, int sz, F3 o,
@@ -202,7 +195,7 @@ __device__ __forceinline__ void advect_at(const VelField &F, int a, const Advect
     const float phi = advect_phi<FORM>(F, pos);
     const bool open = phi > 0.0f;
     auto traced = [&](const float *d, float dirn) {
-        return advect_cubic<FORM>(F, a, d, sx, sy, sz, o, advect_trace<FORM>(F, pos, dt, dirn, max_substeps, phi));
+        return advect_cubic<FORM>(F, a, d, sx, sy, sz, o, trace_back<FORM>(F, pos, dt, dirn, max_substeps, phi));
     };
     if constexpr (stage == 0) {
         if (open) out[f] = traced(src, 1.0f);
@@ -213,7 +206,7 @@ __device__ __forceinline__ void advect_at(const VelField &F, int a, const Advect
     } else if (open) {
         // clampCorrection (stage 3): min/max over the 8 trilinear corners of the
         // traced point whose own positions are open
-        const F3 tr = advect_trace<FORM>(F, pos, dt, 1.0f, max_substeps, phi);
+        const F3 tr = trace_back<FORM>(F, pos, dt, 1.0f, max_substeps, phi);
         const float fv = fwd[f];
         const float corr = fv + (src[f] - bwd[f]) * 0.5f;
         const float gx = gclamp((tr.x - o.x) / F.g.hx), gy = gclamp((tr.y - o.y) / F.g.hy),
@@ -234,7 +227,7 @@ __device__ __forceinline__ void advect_at(const VelField &F, int a, const Advect
                 have = true;
             }
         };
-        if constexpr (FORM == ADVECT_PLAIN) {
+        if constexpr (FORM == FORM_PLAIN) {
 #pragma unroll
             for (int c = 0; c < 8; ++c) corner(c);
         } else {
@@ -262,15 +255,29 @@ __global__ void __launch_bounds__(256) k_advect(const __grid_constant__ VelField
     advect_at<stage, FORM>(F, a, io, blockIdx.y, sx, sy, sz, comp_origin(F.g, a), i + (long long)sx * (j + (long long)sy * k), i,
                            j, k, dt, max_substeps);
 }
-// The straightforward form, runs of 256 faces, below ADVECT_SHORT_CELLS cells: there
-// most warps touch an end of the arrays, where the short form only adds to this one,
-// and a small grid is bound by one warp's latency, which the short form's loops
-// lengthen.  Order 1, all faces, this form and the short one: 33 x 43 x 49 32 and 41 us
-// (43 with a launch a component), 64^3 91 and 92, 65 x 54 x 203 230 and 250, 96^3 273
-// and 273, 128 x 96 x 96 363 and 331, 128^3 627 and 490, 200^3 2301 and 1659.
-constexpr long long ADVECT_SHORT_CELLS = 1LL << 20;
+// The straightforward form, runs of 256 faces, where the short one does not pay.  64
+// registers, as a small grid is bound by one warp's latency (48, the compiler's choice:
+// 32^3 with a collider 13.2 us, 12.1 so).  In the short form a warp that touches an end of
+// the arrays takes the straightforward sample there, so its gain goes with the share of
+// the warps (32 faces of a row) that touch none, and a spacing that is no power of two
+// costs it the corrected quotients.  Straightforward over short, all faces and a scalar,
+// both orders, 0.3 and 1.6 cells a step, with and without a collider (least and most):
+//   power of two:  112^3 (share 0.41) 1.03-1.23, 128^3 1.03-1.23, 256 x 256 x 16 1.08-1.21,
+//                  160^3 1.12-1.32, 256^3 1.24-1.56; 64 x 1024 x 64 (share 0) 0.93-1.09,
+//                  512 x 512 x 4 (0.22) 0.97-1.14, 2048 x 1024 x 2 (0) 0.87-1.08
+//   any spacing:   112^3 0.92-1.02, 144^3 (0.53) 0.99-1.14, 256 x 256 x 16 (0.60, 1.05M
+//                  cells) 0.96-1.10, 160^3 (0.58) 1.00-1.14, 200^3 1.10-1.29, 256^3 1.14-1.39;
+//                  64 x 1024 x 64 0.81-0.93, 2048 x 1024 x 2 0.79-0.90
+// and below a million cells it was slower throughout (33 x 43 x 49 41 us against 32).
+int advect_form(const VelField &F) {
+    const double nx = F.g.nx, ny = F.g.ny, nz = F.g.nz;
+    const double share = std::max(0.0, nx - 64) / nx * std::max(0.0, ny - 3) / ny * std::max(0.0, nz - 3) / nz;
+    const double cells = nx * ny * nz;
+    if (F.pow2) return cells >= 1 << 20 && share >= 0.4 ? FORM_SHORT_P2 : FORM_PLAIN;
+    return cells >= 1 << 21 && share >= 0.55 ? FORM_SHORT : FORM_PLAIN;
+}
 template <int stage>
-__global__ void k_advect_plain(const __grid_constant__ VelField F, int a0, const __grid_constant__ AdvectIO io, float dt,
+__global__ void __launch_bounds__(256, 4) k_advect_plain(const __grid_constant__ VelField F, int a0, const __grid_constant__ AdvectIO io, float dt,
                                int max_substeps) {
     const int a = a0 + (int)blockIdx.y;
     int sx, sy, sz, i, j, k;
@@ -280,16 +287,16 @@ __global__ void k_advect_plain(const __grid_constant__ VelField F, int a0, const
     const F3 o = comp_origin(F.g, a);
     for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < n; f += (long long)gridDim.x * blockDim.x) {
         unflatten(f, sx, sy, i, j, k);
-        advect_at<stage, ADVECT_PLAIN>(F, a, io, blockIdx.y, sx, sy, sz, o, f, i, j, k, dt, max_substeps);
+        advect_at<stage, FORM_PLAIN>(F, a, io, blockIdx.y, sx, sy, sz, o, f, i, j, k, dt, max_substeps);
     }
 }
 
 // trace(start, direction) of a list of points (float3 per point)
-template <bool P2>
-__global__ void k_trace(const __grid_constant__ VelField F, long long n, const float *__restrict__ pin, float *__restrict__ pout, float dt,
-                        float dirn, int max_substeps) {
+template <int FORM>
+__global__ void __launch_bounds__(256, 4) k_trace(const __grid_constant__ VelField F, long long n, const float *__restrict__ pin,
+                                                  float *__restrict__ pout, float dt, float dirn, int max_substeps) {
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const F3 r = back_trace<P2>(F, F3{pin[3 * q], pin[3 * q + 1], pin[3 * q + 2]}, dt, dirn, max_substeps, NAN);
+        const F3 r = trace_back<FORM>(F, F3{pin[3 * q], pin[3 * q + 1], pin[3 * q + 2]}, dt, dirn, max_substeps, NAN);
         pout[3 * q] = r.x;
         pout[3 * q + 1] = r.y;
         pout[3 * q + 2] = r.z;
@@ -582,8 +589,7 @@ extern "C" int ff_advect3_set_collider(ff_advect a, ff_field phi) {
 static int advect_components(ff_advect a, const VelField &F, int a0, int na, const float *const *src, float *const *out) {
     cudaStream_t s = a->ctx->stream;
     const float dt = (float)a->desc.dt;
-    const int ms = a->desc.max_substeps;
-    const long long cells = (long long)a->g.nx * a->g.ny * a->g.nz;
+    const int ms = a->desc.max_substeps, form = advect_form(F);
     long long n = 0;
     int planes = 0, blocks = 0;
     AdvectIO io{};
@@ -603,11 +609,11 @@ static int advect_components(ff_advect a, const VelField &F, int a0, int na, con
             io.bwd[q] = a->bwd[a0 + q];
             io.out[q] = to[q];
         }
-        if (cells < ADVECT_SHORT_CELLS) {
+        if (form == FORM_PLAIN) {
             k_advect_plain<st><<<dim3((unsigned)launch_blocks(n), (unsigned)na), 256, 0, s>>>(F, a0, io, dt, ms);
             return;
         }
-        const auto kernel = F.pow2 ? k_advect<st, ADVECT_SHORT_P2> : k_advect<st, ADVECT_SHORT>;
+        const auto kernel = form == FORM_SHORT_P2 ? k_advect<st, FORM_SHORT_P2> : k_advect<st, FORM_SHORT>;
         for (int z0 = 0; z0 < planes; z0 += 65535)
             kernel<<<dim3((unsigned)blocks, (unsigned)na, (unsigned)std::min(65535, planes - z0)), 256, 0, s>>>(F, a0, io, dt,
                                                                                                               ms, z0);
@@ -683,8 +689,10 @@ extern "C" int ff_advect3_trace(ff_advect a, ff_field vu, ff_field vv, ff_field 
                                     a->phi ? (const float *)a->phi->d : nullptr});
     const long long n = p_in->count;
     if (n == 0) return FF_OK;
-    (F.pow2 ? k_trace<true> : k_trace<false>)<<<launch_blocks(n), 256, 0, a->ctx->stream>>>(F, n, (const float *)p_in->d, (float *)p_out->d,
-                                                          (float)a->desc.dt, (float)direction, a->desc.max_substeps);
+    const int form = point_form(F, n);
+    const auto kernel = form == FORM_PLAIN ? k_trace<FORM_PLAIN> : form == FORM_SHORT ? k_trace<FORM_SHORT> : k_trace<FORM_SHORT_P2>;
+    kernel<<<launch_blocks(n), 256, 0, a->ctx->stream>>>(F, n, (const float *)p_in->d, (float *)p_out->d,
+                                                         (float)a->desc.dt, (float)direction, a->desc.max_substeps);
     return post("trace");
 }
 

@@ -135,10 +135,9 @@ inline VelField trace_field(VelField F) {
     for (int a = 0; a < 3; ++a) {
         int e;
         F.pow2 = F.pow2 && frexpf(h[a], &e) == 0.5f;
-        // (split() takes coordinates below 2^22; a grid one cell thick has one
-        // centre plane, both of its taps)
+        // (split() takes coordinates below 2^22)
         const int end = std::min(n[a], 1 << 22);
-        F.ax[a] = TraceAxis{h[a], 1.0f / h[a], {o[a], o[a] + h[a] * 0.5f}, {end, a == 2 && n[a] == 1 ? 1 : end - 1}};
+        F.ax[a] = TraceAxis{h[a], 1.0f / h[a], {o[a], o[a] + h[a] * 0.5f}, {end, end - 1}};
     }
     return F;
 }
@@ -160,6 +159,7 @@ __device__ __forceinline__ float sample_phi(const VelField &F, const float *phi,
 }
 
 // ---- samples away from the array ends -----------------------------------
+// (of grids of two planes and more: see advect_form and point_form)
 // The trace and the tricubic sample are bound by issue and by instruction
 // fetch (about 2300 instructions a face in the straightforward form), so where
 // no tap needs clamping they run in a shorter form of the same operations: the
@@ -256,11 +256,10 @@ __device__ __forceinline__ bool point6(const VelField &F, F3 p, Point6 &q) {
     }
     return in;
 }
-// trilinear() at index (i, j, k) with all taps inside, planes dz apart (0 for
-// the centre plane of a grid one cell thick)
-__device__ __forceinline__ float lin1(const float *__restrict__ d, int sx, int sy, int dz, int i, int j, int k, float fx,
-                                      float fy, float fz) {
-    const float *r0 = d + (i + sx * (j + sy * k)), *r1 = r0 + sx, *r2 = r0 + dz, *r3 = r2 + sx;
+// trilinear() at index (i, j, k) with all taps inside
+__device__ __forceinline__ float lin1(const float *__restrict__ d, int sx, int sy, int i, int j, int k, float fx, float fy,
+                                      float fz) {
+    const float *r0 = d + (i + sx * (j + sy * k)), *r1 = r0 + sx, *r2 = r0 + sx * sy, *r3 = r2 + sx;
     const float ux = 1.0f - fx, uy = 1.0f - fy, uz = 1.0f - fz;
     const float w00 = ux * uy, w10 = fx * uy, w01 = ux * fy, w11 = fx * fy;
     float s = __ldg(r0) * (w00 * uz);
@@ -277,9 +276,8 @@ __device__ __forceinline__ void lin_uv(const VelField &F, const Point6 &q, float
     const int nx = F.g.nx, ny = F.g.ny;
     const float *a0 = F.u + (q.x.i[0] + (nx + 1) * (q.y.i[1] + ny * q.z.i[1]));
     const float *b0 = F.v + (q.x.i[1] + nx * (q.y.i[0] + (ny + 1) * q.z.i[1]));
-    const bool flat = F.g.nz == 1;
-    const float *a1 = a0 + (nx + 1), *a2 = a0 + (flat ? 0 : (nx + 1) * ny), *a3 = a2 + (nx + 1);
-    const float *b1 = b0 + nx, *b2 = b0 + (flat ? 0 : nx * (ny + 1)), *b3 = b2 + nx;
+    const float *a1 = a0 + (nx + 1), *a2 = a0 + (nx + 1) * ny, *a3 = a2 + (nx + 1);
+    const float *b1 = b0 + nx, *b2 = b0 + nx * (ny + 1), *b3 = b2 + nx;
     const f32x2 one = pack2(1.0f, 1.0f);
     const f32x2 fx = pack2(q.x.f[0], q.x.f[1]), fy = pack2(q.y.f[1], q.y.f[0]), fz = pack2(q.z.f[1], q.z.f[1]);
     const f32x2 ux = sub2(one, fx), uy = sub2(one, fy), uz = sub2(one, fz);
@@ -307,7 +305,7 @@ __device__ __forceinline__ F3 trace_vel(const VelField &F, F3 p) {
     if (warp_any(!point6<P2>(F, p, q))) return sample_vel_ends(F, p);
     F3 r;
     lin_uv(F, q, r.x, r.y);
-    r.z = lin1(F.w, F.g.nx, F.g.ny, F.g.nx * F.g.ny, q.x.i[1], q.y.i[1], q.z.i[0], q.x.f[1], q.y.f[1], q.z.f[0]);
+    r.z = lin1(F.w, F.g.nx, F.g.ny, q.x.i[1], q.y.i[1], q.z.i[0], q.x.f[1], q.y.f[1], q.z.f[0]);
     return r;
 }
 template <bool P2>
@@ -319,8 +317,7 @@ __device__ __forceinline__ float trace_phi(const VelField &F, F3 p) {
     in &= axis_at<P2>(F.ax[1], 1, p.y, j, fy);
     in &= axis_at<P2>(F.ax[2], 1, p.z, k, fz);
     if (warp_any(!in)) return sample_phi_ends(F, p);
-    const G3 &g = F.g;
-    return lin1(F.phi, g.nx, g.ny, g.nz == 1 ? 0 : g.nx * g.ny, i, j, k, fx, fy, fz);
+    return lin1(F.phi, F.g.nx, F.g.ny, i, j, k, fx, fy, fz);
 }
 
 // mono_cubic on two rows of taps at once
@@ -356,12 +353,11 @@ __device__ __forceinline__ float trace_cubic(const VelField &F, int a, const flo
     bool in = axis_at<P2>(F.ax[0], a != 0, p.x, i, fx);
     in &= axis_at<P2>(F.ax[1], a != 1, p.y, j, fy);
     in &= axis_at<P2>(F.ax[2], a != 2, p.z, k, fz);
-    // one plane: every z tap is that plane
-    const int z0 = sz == 1 ? 0 : 1, dz = sz == 1 ? 0 : sx * sy;
-    if (warp_any(!(in && i >= 1 && i <= sx - 3 && j >= 1 && j <= sy - 3 && k >= z0 && (sz == 1 || k <= sz - 3))))
+    const int dz = sx * sy;
+    if (warp_any(!(in && i >= 1 && i <= sx - 3 && j >= 1 && j <= sy - 3 && k >= 1 && k <= sz - 3)))
         return tricubic_ends(d, sx, sy, sz, F.g, o, p);
     const f32x2 fx2 = pack2(fx, fx), fy2 = pack2(fy, fy);
-    const float *r = d + ((i - 1) + sx * ((j - 1) + sy * (k - z0)));
+    const float *r = d + ((i - 1) + sx * ((j - 1) + sy * (k - 1)));
     float z[4];
 #pragma unroll 1
     for (int c = 0; c < 2; ++c) {
@@ -395,8 +391,9 @@ __device__ inline F3 back_trace_plain(const VelField &F, F3 pos, float dt, float
         const F3 mid{pt.x - v0.x * hs * dirn, pt.y - v0.y * hs * dirn, pt.z - v0.z * hs * dirn};
         const F3 mv = sample_vel(F, mid);
         const F3 nxt{pt.x - mv.x * sdt * dirn, pt.y - mv.y * sdt * dirn, pt.z - mv.z * sdt * dirn};
-        const float phi0 = sample_phi(F, F.phi, pt), phi1 = sample_phi(F, F.phi, nxt);
+        const float phi1 = sample_phi(F, F.phi, nxt);
         if (phi1 <= 0.0f) {
+            const float phi0 = sample_phi(F, F.phi, pt);   // (here: few paths end at the collider)
             const float w = fabsf(phi1) / (fabsf(phi0) + fabsf(phi1));
             const float wm = 1.0f - w;
             pt = F3{pt.x * w + nxt.x * wm, pt.y * w + nxt.y * wm, pt.z * w + nxt.z * wm};
@@ -451,6 +448,27 @@ __device__ __forceinline__ F3 back_trace(const VelField &F, F3 pos, float dt, fl
         pt = nxt;
     }
     return pt;
+}
+
+// the forms of the trace and the samples: the straightforward one, and the short one
+// for any spacing and for powers of two
+enum { FORM_PLAIN, FORM_SHORT, FORM_SHORT_P2 };
+template <int FORM>
+__device__ __forceinline__ F3 trace_back(const VelField &F, F3 pos, float dt, float dirn, int max_substeps, float phi0) {
+    if constexpr (FORM == FORM_PLAIN) return back_trace_plain(F, pos, dt, dirn, max_substeps);
+    else return back_trace<FORM == FORM_SHORT_P2>(F, pos, dt, dirn, max_substeps, phi0);
+}
+
+// The form for a list of n points.  A point takes a trace and no tricubic sample, and
+// lanes of one warp can have points anywhere: the short form pays for lists that keep
+// the GPU full, in cell order from about a million points (128^3, straightforward over
+// short: 1M points 0.91-1.03, 2M 1.00-1.18, 8M 1.25-1.36), in random
+// order from about eight (4M 0.95-0.98, 8M 1.00); in a grid one cell thick it never does
+// (1024 x 256, a million points: 0.62-0.69).
+constexpr long long POINTS_SHORT = 1LL << 23;
+inline int point_form(const VelField &F, long long n) {
+    if (F.g.nz == 1 || n < POINTS_SHORT) return FORM_PLAIN;
+    return F.pow2 ? FORM_SHORT_P2 : FORM_SHORT;
 }
 
 // (i, j, k) of a flat index; below 2^31 in 32-bit unsigned arithmetic (a
