@@ -96,17 +96,19 @@ __device__ __forceinline__ unsigned long long p2g_pack(int num, int den) {
 // run touches fit in shared memory, where an int32 add costs a bank access and
 // not a trip to L2.  The window comes from 32 samples of the run: per axis the
 // 20% to 80% quantiles of the cells, widened to the whole range of an even
-// spread and cut to the capacity around its middle.  Particles outside it
+// spread and cut to the capacity around its middle (p2g_window).  Particles outside it
 // (moved by resampling, spray) add to the global sums; the window's nonzero
-// sums follow once per block.  Measured at 13.4M particles, 8 a cell, an eighth
+// sums follow once per block.  A run too spread for a window adds to the global sums
+// throughout: lists in random order, whole P2G 40^3 with one particle a cell 56 us with
+// windows, 31 without, 64^3 with eight 217 and 161.  Measured at 13.4M particles, 8 a cell, an eighth
 // of them out of order: 0.65 ms against 1.59 ms for 48 global int32 adds a
 // particle.  Now bound by the LSU data path (83% of its wavefronts): half of
 // them the window adds (2.4 bank passes each), half the global adds of the
 // eighth outside the windows, one lane each.
 constexpr int P2G_NT = 512, P2G_MAX_ROUNDS = 8;
 
-// the value of rank r among the 32 lanes' values
-__device__ __forceinline__ int warp_rank_value(int v, int r) {
+// this lane's rank among the 32 lanes' values
+__device__ __forceinline__ int warp_rank(int v) {
     int rank = 0;
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -114,6 +116,9 @@ __device__ __forceinline__ int warp_rank_value(int v, int r) {
         const int x = __shfl_sync(0xffffffffu, v, o);
         rank += x < v || (x == v && o < lane);
     }
+    return rank;
+}
+__device__ __forceinline__ int value_of_rank(int v, int rank, int r) {
     return __shfl_sync(0xffffffffu, v, __ffs(__ballot_sync(0xffffffffu, rank == r)) - 1);
 }
 
@@ -132,13 +137,15 @@ __global__ void __launch_bounds__(P2G_NT, 3) k_flip_scatter(G3 g, long long n, i
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
             const int c = iclamp((int)floorf(gclamp((pos[3 * p + b] - org[b]) / hh[b])), 0, nn[b] - 1);
-            q20[b] = warp_rank_value(c, 6);
-            q80[b] = warp_rank_value(c, 25);
+            const int rank = warp_rank(c);
+            q20[b] = value_of_rank(c, rank, 6);
+            q80[b] = value_of_rank(c, rank, 25);
         }
-        p2g_window(q20, q80, nn, lo, w);
+        p2g_window(q20, q80, nn, count, lo, w);
         if (threadIdx.x < 3) {
+            const int extent = threadIdx.x == 0 ? w[0] : (threadIdx.x == 1 ? w[1] : w[2]);
             wlo[threadIdx.x] = (threadIdx.x == 0 ? lo[0] : (threadIdx.x == 1 ? lo[1] : lo[2])) - 1;
-            wn[threadIdx.x] = (threadIdx.x == 0 ? w[0] : (threadIdx.x == 1 ? w[1] : w[2])) + 2;
+            wn[threadIdx.x] = extent > 0 ? extent + 2 : 0;
         }
     }
     __syncthreads();
