@@ -1948,8 +1948,8 @@ __global__ void __launch_bounds__(256, 4) k_resid_rx(Geo g, const float *__restr
     if (2 * qx + 1 >= cnx - 1) rh = r3;                     // fine 2I+2 clamps to 2I+1 at the end
     else if (lane == 31) rh = resid_scalar(g, x, b, coef, crow, row, rym, ryp, rzm, rzp, i0 + 4, j, k);
     float2 out;
-    out.x = 0.125f * rl + 0.375f * r0 + 0.375f * r1 + 0.125f * r2;
-    out.y = 0.125f * r1 + 0.375f * r2 + 0.375f * r3 + 0.125f * rh;
+    out.x = x_taps(true, rl, r0, r1, r2);
+    out.y = x_taps(false, r1, r2, r3, rh);
     *reinterpret_cast<float2 *>(rx + (long long)cnx * (j + (long long)g.d.ny * k) + 2 * qx) = out;
 }
 
@@ -2004,8 +2004,8 @@ __global__ void __launch_bounds__(256, 5) k_resid_rx_rows(Geo g, const float *__
     const float rh = qx == nq - 1 ? r3 : s_r0[t + 1];
     if (!valid) return;
     float2 out;
-    out.x = 0.125f * rl + 0.375f * r0 + 0.375f * r1 + 0.125f * r2;
-    out.y = 0.125f * r1 + 0.375f * r2 + 0.375f * r3 + 0.125f * rh;
+    out.x = x_taps(true, rl, r0, r1, r2);
+    out.y = x_taps(false, r1, r2, r3, rh);
     *reinterpret_cast<float2 *>(rx + (long long)cnx * (j + (long long)g.d.ny * k) + 2 * qx) = out;
 }
 
@@ -2132,10 +2132,10 @@ __global__ void __launch_bounds__(256) k_prolong4(Dims fd, Dims cd, int dims, co
                 const float *row = coarse + (long long)cd.nx * (jj[b] + (long long)cd.ny * kk[g]);
                 const float w = wj[b] * wk[g];
                 const float v0 = __ldg(row + c0), v1 = __ldg(row + c1), v2 = __ldg(row + c2), v3 = __ldg(row + c3);
-                a0 += (0.25f * v0 + 0.75f * v1) * w;
-                a1 += (0.75f * v1 + 0.25f * v2) * w;
-                a2 += (0.25f * v1 + 0.75f * v2) * w;
-                a3 += (0.75f * v2 + 0.25f * v3) * w;
+                a0 = __fmaf_rn(two_taps(0.25f, v0, 0.75f, v1), w, a0);
+                a1 = __fmaf_rn(two_taps(0.75f, v1, 0.25f, v2), w, a1);
+                a2 = __fmaf_rn(two_taps(0.25f, v1, 0.75f, v2), w, a2);
+                a3 = __fmaf_rn(two_taps(0.75f, v2, 0.25f, v3), w, a3);
             }
         a[p][0] = a0;
         a[p][1] = a1;

@@ -32,14 +32,14 @@ __device__ __forceinline__ float op_and_diag(const Dims &d, int i, int j, int k,
                                              XF X, float &D) {
     const long long sy = d.nx, sz = (long long)d.nx * d.ny;
     float4 kc = ldcoef<C16>(c32, c16, c);
-    float s = -kc.w * xc;
+    float s = __fmul_rn(-kc.w, xc);
     D = -(kc.w + kc.x + kc.y + kc.z);
-    if (i > 0) s += kc.x * (X(c - 1) - xc);
-    if (i < d.nx - 1) { float k1 = ldkx<C16>(c32, c16, c + 1); s += k1 * (X(c + 1) - xc); D -= k1; }
-    if (j > 0) s += kc.y * (X(c - sy) - xc);
-    if (j < d.ny - 1) { float k1 = ldky<C16>(c32, c16, c + sy); s += k1 * (X(c + sy) - xc); D -= k1; }
-    if (k > 0) s += kc.z * (X(c - sz) - xc);
-    if (k < d.nz - 1) { float k1 = ldkz<C16>(c32, c16, c + sz); s += k1 * (X(c + sz) - xc); D -= k1; }
+    if (i > 0) s = __fmaf_rn(kc.x, X(c - 1) - xc, s);
+    if (i < d.nx - 1) { float k1 = ldkx<C16>(c32, c16, c + 1); s = __fmaf_rn(k1, X(c + 1) - xc, s); D -= k1; }
+    if (j > 0) s = __fmaf_rn(kc.y, X(c - sy) - xc, s);
+    if (j < d.ny - 1) { float k1 = ldky<C16>(c32, c16, c + sy); s = __fmaf_rn(k1, X(c + sy) - xc, s); D -= k1; }
+    if (k > 0) s = __fmaf_rn(kc.z, X(c - sz) - xc, s);
+    if (k < d.nz - 1) { float k1 = ldkz<C16>(c32, c16, c + sz); s = __fmaf_rn(k1, X(c + sz) - xc, s); D -= k1; }
     return s;
 }
 

@@ -14,8 +14,8 @@
 //  - levels of up to HELD_CELLS cells, and the coarsest level's sweeps, run in
 //    block 0 with their arrays in shared memory: a phase there costs a block
 //    barrier and a shared-memory round trip.
-// Per cell the arithmetic is that of the level kernels in ff_fused.cu, bit for bit:
-// the
+// Per cell the arithmetic is that of the level kernels in ff_fused.cu, bit for bit
+// (sums of two products are rounded as ff_stencil.cuh writes them out): the
 // sweep's relaxation by class, the residual by class followed by the x, y and
 // z taps of the restriction, k_coarse_direct's row products, k_prolong4's
 // correction; the CG phases are k_update_p_pap's and k_update_x_residual's.
@@ -326,14 +326,8 @@ __device__ __noinline__ void g_residual(int l, bool xzero) {
     }
 }
 
-// x taps of the restriction from level 0 as k_resid_rx's roundings are (of an even
-// and of an odd coarse cell)
-__device__ __forceinline__ float x_taps(int odd, float r0, float r1, float r2, float r3) {
-    const float s = odd ? __fmaf_rn(0.125f, r0, __fmul_rn(0.375f, r1)) : __fmaf_rn(0.375f, r1, 0.125f * r0);
-    return __fmaf_rn(0.125f, r3, __fmaf_rn(0.375f, r2, s));
-}
 // the 1/8, 3/8, 3/8, 1/8 taps per axis on the fine residual around coarse
-// cell (I, J, K); level0: with x_taps
+// cell (I, J, K); level0: F is the solver's level 0, whose x taps k_resid_rx rounds
 template <bool D3, class LD>
 __device__ __forceinline__ float restrict_cell(const Dims &fd, const Dims &cd, int I, int J, int K, LD ldr,
                                                bool level0 = false) {
@@ -352,7 +346,7 @@ __device__ __forceinline__ float restrict_cell(const Dims &fd, const Dims &cd, i
         for (int p = 0; p < 4; ++p) {
             const int row = fd.nx * (jy[p] + fd.ny * kz[q]);
             const float r0 = ldr(row + ix[0]), r1 = ldr(row + ix[1]), r2 = ldr(row + ix[2]), r3 = ldr(row + ix[3]);
-            const float rx = level0 ? x_taps(I & 1, r0, r1, r2, r3) : 0.125f * r0 + 0.375f * r1 + 0.375f * r2 + 0.125f * r3;
+            const float rx = x_taps(level0 && !(I & 1), r0, r1, r2, r3);
             part += rx * w4[p];
         }
         s += part * wz;
@@ -395,7 +389,7 @@ __device__ __forceinline__ float prolong_cell(const Dims &cd, int i, int j, int 
 #pragma unroll
         for (int q = 0; q < (D3 ? 2 : 1); ++q) {
             const float w = wj[b] * wk[q];
-            acc += (wi[0] * ldx(ii[0], jj[b], kk[q]) + wi[1] * ldx(ii[1], jj[b], kk[q])) * w;
+            acc = __fmaf_rn(two_taps(wi[0], ldx(ii[0], jj[b], kk[q]), wi[1], ldx(ii[1], jj[b], kk[q])), w, acc);
         }
     return acc;
 }
@@ -446,14 +440,14 @@ __device__ __noinline__ void g_coarse_colour(int col) {
         if (((i + j + k) & 1) != col) continue;
         const float xc = __ldcg(x + c);
         const float4 kc = __ldg(C.coef + c);
-        float s = -kc.w * xc;
+        float s = __fmul_rn(-kc.w, xc);
         float D = -(kc.w + kc.x + kc.y + kc.z);
-        if (i > 0) s += kc.x * (__ldcg(x + c - 1) - xc);
-        if (i < d.nx - 1) { const float k1 = __ldg(&C.coef[c + 1].x); s += k1 * (__ldcg(x + c + 1) - xc); D -= k1; }
-        if (j > 0) s += kc.y * (__ldcg(x + c - sy) - xc);
-        if (j < d.ny - 1) { const float k1 = __ldg(&C.coef[c + sy].y); s += k1 * (__ldcg(x + c + sy) - xc); D -= k1; }
-        if (k > 0) s += kc.z * (__ldcg(x + c - sz) - xc);
-        if (k < d.nz - 1) { const float k1 = __ldg(&C.coef[c + sz].z); s += k1 * (__ldcg(x + c + sz) - xc); D -= k1; }
+        if (i > 0) s = __fmaf_rn(kc.x, __ldcg(x + c - 1) - xc, s);
+        if (i < d.nx - 1) { const float k1 = __ldg(&C.coef[c + 1].x); s = __fmaf_rn(k1, __ldcg(x + c + 1) - xc, s); D -= k1; }
+        if (j > 0) s = __fmaf_rn(kc.y, __ldcg(x + c - sy) - xc, s);
+        if (j < d.ny - 1) { const float k1 = __ldg(&C.coef[c + sy].y); s = __fmaf_rn(k1, __ldcg(x + c + sy) - xc, s); D -= k1; }
+        if (k > 0) s = __fmaf_rn(kc.z, __ldcg(x + c - sz) - xc, s);
+        if (k < d.nz - 1) { const float k1 = __ldg(&C.coef[c + sz].z); s = __fmaf_rn(k1, __ldcg(x + c + sz) - xc, s); D -= k1; }
         x[c] = xc + ((__ldcg(C.b + c) - s) / D) * sor;
     }
 }
@@ -697,9 +691,9 @@ __device__ __forceinline__ CoarseCell<D3> coarse_cell(const RLevel &C, const flo
 template <bool D3>
 __device__ __forceinline__ void coarse_relax(const CoarseCell<D3> &q, float *x, float sor) {
     const float xc = x[q.c];
-    float s = -q.e * xc;
+    float s = __fmul_rn(-q.e, xc);
 #pragma unroll
-    for (int f = 0; f < (D3 ? 6 : 4); ++f) s += q.k[f] * (x[q.n[f]] - xc);
+    for (int f = 0; f < (D3 ? 6 : 4); ++f) s = __fmaf_rn(q.k[f], x[q.n[f]] - xc, s);
     x[q.c] = xc + quotient(q.b - s, q.D, q.r) * sor;
 }
 template <bool D3>
@@ -1085,8 +1079,7 @@ __device__ __noinline__ void c_residual(int l, bool xzero) {
         int ix[4];
         rtap4(t - lr * hx, hx, ix);
         const float *row = r + lr * nx;
-        rsm[SA.crx + t] = l == 0 && SA.pairs ? x_taps((t - lr * hx) & 1, row[ix[0]], row[ix[1]], row[ix[2]], row[ix[3]])
-                                 : 0.125f * row[ix[0]] + 0.375f * row[ix[1]] + 0.375f * row[ix[2]] + 0.125f * row[ix[3]];
+        rsm[SA.crx + t] = x_taps(l == 0 && SA.pairs && !((t - lr * hx) & 1), row[ix[0]], row[ix[1]], row[ix[2]], row[ix[3]]);
     }
 }
 
@@ -1211,8 +1204,8 @@ __device__ __noinline__ void c_prolong(int l) {
 #pragma unroll
             for (int z = 0; z < (D3 ? 2 : 1); ++z) {
                 const float wt = wj[b] * wk[z];
-                s0 += (wa[0] * v[b][z][0] + wa[1] * v[b][z][1]) * wt;
-                s1 += (wb[0] * v[b][z][1] + wb[1] * v[b][z][2]) * wt;
+                s0 = __fmaf_rn(two_taps(wa[0], v[b][z][0], wa[1], v[b][z][1]), wt, s0);
+                s1 = __fmaf_rn(two_taps(wb[0], v[b][z][1], wb[1], v[b][z][2]), wt, s1);
             }
         if ((q.cls & 3u) != 1u) x[q.e] += s0;
         if (q.cls >> 2 != 1u) x[q.e + 1] += s1;
@@ -1318,14 +1311,14 @@ __device__ __noinline__ void c_coarse() {
                     coarse_couplings<D3>(C, R.q0 * nx + e, i, j, k, kf, E);
                 }
             }
-            float s = -E * xc;
-            s += kf[0] * (xm - xc);
-            s += kf[1] * (xp - xc);
-            s += kf[2] * (ym - xc);
-            s += kf[3] * (yp - xc);
+            float s = __fmul_rn(-E, xc);
+            s = __fmaf_rn(kf[0], xm - xc, s);
+            s = __fmaf_rn(kf[1], xp - xc, s);
+            s = __fmaf_rn(kf[2], ym - xc, s);
+            s = __fmaf_rn(kf[3], yp - xc, s);
             if (D3) {
-                s += kf[4] * (zm - xc);
-                s += kf[5] * (zp - xc);
+                s = __fmaf_rn(kf[4], zm - xc, s);
+                s = __fmaf_rn(kf[5], zp - xc, s);
             }
             x[e] = xc + quotient(b[e] - s, D.x, D.y) * sor;
         }

@@ -49,14 +49,13 @@ __device__ __forceinline__ Coef coef_at(const Geo &g, const float4 *coef, bool r
 // staged neighbour values are zero-filled (finite).
 __device__ __forceinline__ float apply_q(const Coef &q, float vc, float xm, float xp, float ym, float yp,
                                          float zm, float zp) {
-    float s = -q.e * vc;
-    s += q.kx * (xm - vc);
-    s += q.ux * (xp - vc);
-    s += q.ky * (ym - vc);
-    s += q.uy * (yp - vc);
-    s += q.kz * (zm - vc);
-    s += q.uz * (zp - vc);
-    return s;
+    float s = __fmul_rn(-q.e, vc);
+    s = __fmaf_rn(q.kx, xm - vc, s);
+    s = __fmaf_rn(q.ux, xp - vc, s);
+    s = __fmaf_rn(q.ky, ym - vc, s);
+    s = __fmaf_rn(q.uy, yp - vc, s);
+    s = __fmaf_rn(q.kz, zm - vc, s);
+    return __fmaf_rn(q.uz, zp - vc, s);
 }
 __device__ __forceinline__ float diag_q(const Coef &q) {
     return -(q.e + q.kx + q.ux + q.ky + q.uy + q.kz + q.uz);
@@ -106,6 +105,21 @@ __device__ __forceinline__ void ptaps2(int f, int nc, int *idx, float *w) {
         idx[0] = ci; w[0] = 0.75f;
         idx[1] = ci < nc - 1 ? ci + 1 : ci; w[1] = 0.25f;
     }
+}
+
+// The sums of products below are shared by the launch-per-pass kernels and the one-launch
+// ones, whose results are equal bit for bit: which product is rounded before it enters a
+// fused multiply-add is written out, not left to the compiler (it chose by what else a
+// product is used for, differently for the two cells of a thread).
+// x taps of the restriction; first: the first product is the rounded one (even coarse
+// cells of level 0), else the second
+__device__ __forceinline__ float x_taps(bool first, float r0, float r1, float r2, float r3) {
+    const float s = first ? __fmaf_rn(0.375f, r1, __fmul_rn(0.125f, r0)) : __fmaf_rn(0.125f, r0, __fmul_rn(0.375f, r1));
+    return __fmaf_rn(0.125f, r3, __fmaf_rn(0.375f, r2, s));
+}
+// the two x taps of the prolongation
+__device__ __forceinline__ float two_taps(float wa, float a, float wb, float b) {
+    return __fmaf_rn(wa, a, __fmul_rn(wb, b));
 }
 
 // compensated (TwoSum) FP32 accumulation, folded into FP64 once
