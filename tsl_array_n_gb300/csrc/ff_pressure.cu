@@ -92,6 +92,7 @@ struct ff_pressure_s {
     // coarsest direct solve
     double *G = nullptr;
     int nG = 0;
+    bool factored = false;          // G is of the operator last prepared
     std::vector<float4> coarse_key;
 
     // graphs
@@ -618,7 +619,8 @@ static int prepare(ff_pressure ps, ff_field u, ff_field v, ff_field w) {
     FF_TRY(input_hash(ps, &h));
     bool planes = false;
     pair_planes(ps, &planes);
-    const bool reuse = ps->prepared && h == ps->input_hash && !planes;
+    const bool direct = ps->desc.preconditioner == FF_PRE_MULTIGRID && ps->desc.mg_coarse_mode == FF_COARSE_DIRECT;
+    const bool reuse = ps->prepared && h == ps->input_hash && !planes && (!direct || ps->factored);
     if (!reuse) ps->prepared = false;   // (until the last level is built)
     // updateDirichletFields (grid_pressure_solver3.js:171-206)
     ps->has_mask = ps->active || cw[0];
@@ -693,8 +695,9 @@ static int prepare(ff_pressure ps, ff_field u, ff_field v, ff_field w) {
     ps->prepared = true;
     ps->input_hash = h;
     ++ps->rebuilds;
+    ps->factored = false;
     // FP64 direct coarsest solve: refactor when the coarsest operator changed
-    if (ps->desc.preconditioner == FF_PRE_MULTIGRID && ps->desc.mg_coarse_mode == FF_COARSE_DIRECT) {
+    if (direct) {
         Level &c = ps->lv[Ln - 1];
         int nc = (int)c.d.n();
         std::vector<float4> key(nc);
@@ -711,6 +714,7 @@ static int prepare(ff_pressure ps, ff_field u, ff_field v, ff_field w) {
             ps->nG = nc;
             ps->coarse_key.swap(key);
         }
+        ps->factored = true;
     }
     return FF_OK;
 }
