@@ -10,12 +10,16 @@
 
 // ---------------------------------------------------------------- errors --
 int ff_set_error(int code, const char *fmt, ...);
+// (an error is reported here and cleared: the check after the next launch, maybe of
+// another call, must not report it again)
 #define FF_CUDA(call)                                                            \
     do {                                                                         \
         cudaError_t _e = (call);                                                 \
-        if (_e != cudaSuccess)                                                   \
+        if (_e != cudaSuccess) {                                                 \
+            (void)cudaGetLastError();                                            \
             return ff_set_error(FF_E_CUDA, "%s:%d %s: %s", __FILE__, __LINE__,   \
                                 #call, cudaGetErrorString(_e));                  \
+        }                                                                        \
     } while (0)
 #define FF_CHECK(cond, code, ...)                                                \
     do {                                                                         \

@@ -1005,7 +1005,11 @@ static int build_graphs(ff_pressure ps) {
     int st = enqueue_setup(ps);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(s, &g);
-    if (st != FF_OK) { if (g) cudaGraphDestroy(g); return st; }
+    if (st != FF_OK) {
+        if (g) cudaGraphDestroy(g);
+        (void)cudaGetLastError();   // (of the capture that st ended)
+        return st;
+    }
     FF_CUDA(e);
     ps->setup_graph = g;
     FF_CUDA(cudaGraphInstantiate(&ps->setup_exec, g, 0));
@@ -1026,7 +1030,10 @@ static int build_graphs(ff_pressure ps) {
     FF_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     st = enqueue_iteration(ps, (unsigned long long)h, 1);
     e = cudaStreamEndCapture(s, &body);
-    FF_TRY(st);
+    if (st != FF_OK) {
+        (void)cudaGetLastError();
+        return st;
+    }
     FF_CUDA(e);
     FF_CUDA(cudaGraphInstantiate(&ps->loop_exec, lg, 0));
     return FF_OK;
