@@ -175,7 +175,9 @@ int ff_pressure3_project_host(ff_pressure ps, ff_field u_in, ff_field v_in, ff_f
 /* Runtime settings object (:135): key names as in the reference
  * ("tolerance", "maxIterations", "relativeTolerance", "checkBadCells",
  * "preconditioner", "sorFactor", "reportNoiseFloor"), plus "useGraph",
- * "useTma" and "coarseTail" for this implementation's paths. */
+ * "useTma", "coarseTail" and "clusterBlocks" (blocks of the thread-block
+ * cluster that small solves and coarse levels use: 16, 8, or 0 for none) for
+ * this implementation's paths. */
 int ff_pressure3_set(ff_pressure ps, const char *key, double value);
 /* project(inGrid, outGrid)() (:339-556).  u_out may equal u_in.  The
  * pressure field persists between calls and is the warm start.           */

@@ -440,6 +440,13 @@ extern "C" int ff_pressure3_set(ff_pressure ps, const char *key, double value) {
     else if (k == "useGraph") { ps->use_graph = value != 0; }
     else if (k == "useTma") { ps->use_tma = value != 0; destroy_graphs(ps); }
     else if (k == "coarseTail") { ps->use_tail = value != 0; destroy_graphs(ps); }
+    else if (k == "clusterBlocks") {
+        const int c = (int)value;
+        FF_CHECK(c == 0 || ((c == 8 || c == 16) && c <= ps->ctx->cluster_blocks), FF_E_ARG,
+                 "clusterBlocks: %d (0, 8 or 16, at most the %d the device runs)", c, ps->ctx->cluster_blocks);
+        ps->cluster = c;
+        destroy_graphs(ps);
+    }
     else if (k == "preconditioner") {
         FF_CHECK(value >= 0 && value <= 2, FF_E_ARG, "unknown preconditioner %g", value);
         ps->desc.preconditioner = (int)value;
