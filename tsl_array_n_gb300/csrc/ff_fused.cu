@@ -2172,12 +2172,12 @@ __global__ void k_coef_classes(Geo g, int dims, const float *__restrict__ wu, co
                                uint8_t *__restrict__ cls, int pitch, float4 *__restrict__ gco, float4 *__restrict__ rk,
                                float2 *__restrict__ rinv) {
     // one thread per cell (coalesced coefficient stores); the four lanes of
-    // an x-quad (blockDim.x is a multiple of 32) merge their classes into the
-    // quad's byte with shuffles, cells past the row's end as class 0
+    // an x-quad (nx % 4 == 0, blockDim.x a multiple of 32) merge their
+    // classes into the quad's byte with shuffles
     const Dims d = g.d;
     const int ir = blockIdx.x * blockDim.x + threadIdx.x;
     const int jr = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    const bool in = ir < d.nx && jr < d.ny;
+    const bool in = ir < d.nx && jr < d.ny;   // whole quads are in or out
     const int i = in ? ir : 0, j = in ? jr : 0;
     auto W = [](const float *w, long long f) { return w ? w[f] : 1.f; };
     auto P = [&](long long n) { return mask ? mask[n] != 0 : false; };
@@ -2205,7 +2205,7 @@ __global__ void k_coef_classes(Geo g, int dims, const float *__restrict__ wu, co
     const bool pinned = e == 1.f && kx == 0.f && ky == 0.f && kz == 0.f && ux == 0.f && uy == 0.f && uz == 0.f;
     const bool inner = i > 0 && i < d.nx - 1 && j > 0 && j < d.ny - 1 && k > 0 && k < d.nz - 1;
     const unsigned cl = plain ? (inner ? 0u : 2u) : (pinned ? 1u : 3u);
-    unsigned byte = in ? cl << (2 * (ir & 3)) : 0u;
+    unsigned byte = cl << (2 * (ir & 3));
     byte |= __shfl_xor_sync(0xffffffffu, byte, 1);
     byte |= __shfl_xor_sync(0xffffffffu, byte, 2);
     if (!in) return;
@@ -2549,7 +2549,7 @@ static int encode_planes(CUtensorMap *m, const float *base, const Dims &d, int r
     return FF_OK;
 }
 
-static int cls_pitch(const Dims &d) { return (((d.nx + 3) / 4 + 15) / 16) * 16; }
+static int cls_pitch(const Dims &d) { return ((d.nx / 4 + 15) / 16) * 16; }
 
 size_t sweep_tma_cls_bytes(const Dims &d) { return (size_t)cls_pitch(d) * d.ny * d.nz; }
 

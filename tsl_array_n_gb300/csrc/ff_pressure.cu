@@ -259,8 +259,8 @@ extern "C" int ff_pressure3_create(ff_ctx ctx, const ff_pressure_desc *desc, ff_
                        div_up(g.ny, 256 / (g.nx >= 128 ? 128 : g.nx >= 64 ? 64 : 32)) * g.nz;
     blocks = std::max(blocks, (long long)div_up(n, 1024));
     blocks = std::max(blocks, (long long)ffk::fused_blocks(ps->d, ctx->sm_count));
-    if (ps->fused) ps->smaps = new SweepMaps[L];
     if (ps->fused) {
+        ps->smaps = new SweepMaps[L];
         for (int l = 0; l < L; ++l) {
             Level &v = ps->lv[l];
             if (l == L - 1 || !ffk::sweep_tma_ok(v.d)) continue;
