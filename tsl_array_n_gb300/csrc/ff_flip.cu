@@ -96,15 +96,15 @@ __device__ __forceinline__ unsigned long long p2g_pack(int num, int den) {
 // run touches fit in shared memory, where an int32 add costs a bank access and
 // not a trip to L2.  The window comes from 32 samples of the run: per axis the
 // 20% to 80% quantiles of the cells, widened to the whole range of an even
-// spread and cut to the capacity around its middle (p2g_window).  Particles outside it
-// (moved by resampling, spray) add to the global sums; the window's nonzero
-// sums follow once per block.  A run too spread for a window adds to the global sums
-// throughout: lists in random order, whole P2G 40^3 with one particle a cell 56 us with
-// windows, 31 without, 64^3 with eight 217 and 161.  Measured at 13.4M particles, 8 a cell, an eighth
-// of them out of order: 0.65 ms against 1.59 ms for 48 global int32 adds a
-// particle.  Now bound by the LSU data path (83% of its wavefronts): half of
-// them the window adds (2.4 bank passes each), half the global adds of the
-// eighth outside the windows, one lane each.
+// spread and cut to the capacity around its middle (p2g_window).  Particles
+// outside it (moved by resampling, spray) add to the global sums; the window's
+// nonzero sums follow once per block.  A run too spread for a window adds to
+// the global sums throughout: lists in random order, whole P2G at 40^3 with one
+// particle a cell 56 us with windows, 31 without, 64^3 with eight 217 and 161.
+// Measured at 13.4M particles, 8 a cell, an eighth of them out of order: 0.65 ms
+// against 1.59 ms for 48 global int32 adds a particle.  Now bound by the LSU data
+// path (83% of its wavefronts): half of them the window adds (2.4 bank passes
+// each), half the global adds of the eighth outside the windows, one lane each.
 constexpr int P2G_NT = 512, P2G_MAX_ROUNDS = 8;
 
 // this lane's rank among the 32 lanes' values
